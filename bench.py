@@ -347,6 +347,64 @@ def measure_norms(r: Ranks, cuda, rows_total, steps, warmup, peaks):
             "per_kernel_ms": dict(zip(names, per)), "roofline": block, "launches": 3 * steps}
 
 
+class CApiHost:
+    """The e2e loop's calls over the mhlo_* C API, for a build without the PJRT plugin (which is layered on the same API)."""
+
+    def __init__(self):
+        from metalhlo_b200 import capi
+
+        self.capi, self.client = capi, capi.Client()
+        self.done_type = ctypes.CFUNCTYPE(None, ctypes.c_void_p)
+        self.to_host_async = capi.lib.mhlo_b200_buffer_to_host_async
+        self.to_host_async.restype = ctypes.c_int
+        self.to_host_async.argtypes = [ctypes.c_void_p, ctypes.c_void_p, ctypes.c_size_t, self.done_type, ctypes.c_void_p]
+
+    def buffer(self, array):
+        return self._wrap(self.client.buffer(array))
+
+    def buffer_from_pointer(self, ptr, dtype, shape):
+        import numpy as np
+
+        n = int(np.prod(shape))
+        view = np.frombuffer((ctypes.c_byte * (n * np.dtype(dtype).itemsize)).from_address(ptr), dtype=dtype, count=n).reshape(shape)
+        return self.buffer(view)
+
+    def compile(self, text):
+        host, exe = self, self.client.compile(text, opt_level=3)
+
+        class Loaded:
+            def execute(self, args):
+                return [host._wrap(b) for b in exe.execute(args)]
+
+        return Loaded()
+
+    def _wrap(self, buffer):
+        def start(ptr, nbytes):
+            landed = threading.Event()
+            done = self.done_type(lambda _user: landed.set())
+            self.capi._check(self.to_host_async(buffer._h, ptr, nbytes, done, None))
+
+            def wait(keep=done):
+                landed.wait()
+
+            return wait
+
+        buffer.to_host_pointer_start = start
+        buffer.to_host_pointer = lambda ptr, nbytes: self.capi._check(self.capi.lib.mhlo_buffer_to_host(buffer._h, ptr, nbytes))
+        return buffer
+
+
+def e2e_host():
+    """(host, description of the calls): the PJRT plugin where it is built, the C API underneath it otherwise."""
+    plugin = os.path.join(ROOT, "metalhlo_b200", "lib", "pjrt_plugin_metalhlo_b200.so")
+    if os.path.exists(plugin):
+        from metalhlo_b200 import pjrt
+
+        return pjrt.Host(), "GetPjrtApi: BufferFromHostBuffer(token ids, pinned) -> LoadedExecutable_Execute -> Buffer_ToHostBuffer(fp16 logits, pinned)"
+    return CApiHost(), ("C API (the PJRT plugin is not built here): mhlo_buffer_create(token ids, pinned) -> mhlo_execute -> "
+                        "mhlo_b200_buffer_to_host_async(fp16 logits, pinned)")
+
+
 def measure_gpt2(r: Ranks, args, peaks):
     """Device-resident and end-to-end (PJRT, host buffers) throughput of the GPT-2 forward pass, batch split over the ranks
     by the compiler."""
@@ -401,12 +459,10 @@ def measure_gpt2(r: Ranks, args, peaks):
 
     # ---- end to end through the PJRT plugin (GetPjrtApi) with host buffers. The plugin's client reads the shard from the
     # environment, as a launcher would set it per process; the parameters become device buffers once.
-    from metalhlo_b200 import pjrt
-
     os.environ["METALHLO_SHARD_COUNT"], os.environ["METALHLO_SHARD_INDEX"] = str(r.world), str(r.rank)
     os.environ["METALHLO_DEVICE"] = str(r.local)
     os.environ["METALHLO_OPT_LEVEL"] = "O3"  # the plugin compiles at O2 unless told otherwise, like the reference's (PJRTExecutable.swift:1755-1766)
-    host = pjrt.Host()
+    host, e2e_path = e2e_host()
     pexe = host.compile(text)
     param_bufs = [host.buffer(a) for a in host_inputs[1:]]
     ids_pinned = torch.from_numpy(ids_shard).pin_memory()
@@ -474,7 +530,7 @@ def measure_gpt2(r: Ranks, args, peaks):
                                  f"with the masked half counted the figure would be {FLOP_PER_TOKEN_FULL_ATTENTION} FLOP per token"),
         "e2e": {"value": tokens / (e2e_ms * 1e-3), "unit": "tokens/s", "h2d_bytes_per_step": BATCH * SEQ * 4, "d2h_bytes_per_step": BATCH * SEQ * VOCAB * 2,
                 "ms_per_step": e2e_ms, "steps": e2e_steps, "launches_per_step": launches,
-                "path": "GetPjrtApi: BufferFromHostBuffer(token ids, pinned) -> LoadedExecutable_Execute -> Buffer_ToHostBuffer(fp16 logits, pinned); parameters resident; "
+                "path": e2e_path + "; parameters resident; "
                         "the transfer's event is awaited after the next step's Execute, so the logits of step i travel while step i + 1 computes",
                 "one_step_at_a_time": {"value": tokens / (e2e_serial_ms * 1e-3), "ms_per_step": e2e_serial_ms,
                                        "note": "the same calls with every transfer awaited before the next step starts"},

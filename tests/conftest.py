@@ -16,7 +16,20 @@ def pytest_configure(config):
     config.addinivalue_line("markers", "gpu: needs a CUDA device (run with -m gpu on a B200)")
 
 
+def plugin_cannot_be_built():
+    """True where there is neither a built PJRT plugin nor the OpenXLA header it is compiled against."""
+    from __graft_entry__ import _pjrt_include
+
+    plugin = os.path.join(ROOT, "metalhlo_b200", "lib", "pjrt_plugin_metalhlo_b200.so")
+    return not os.path.exists(plugin) and _pjrt_include() is None
+
+
 def pytest_collection_modifyitems(config, items):
+    if plugin_cannot_be_built():
+        no_plugin = pytest.mark.skip(reason="pjrt_c_api.h is not available here, so the PJRT plugin is not built")
+        for item in items:
+            if "pjrt" in item.nodeid or item.name.startswith("test_plugin_"):
+                item.add_marker(no_plugin)
     try:
         import torch
 

@@ -1,420 +1,18 @@
-// Generic tensor kernels over strided views: the elementwise-program interpreter (every unary / binary /
-// compare / select / clamp / convert / iota op, data movement expressed as a strided copy, and fused
-// elementwise chains), reductions, gather, dynamic slicing and the any-layout dot product. They are the
-// non-specialised side of the hot path; the specialised side (row kernels, tensor-core GEMM, attention) lives
-// in its own files.
+// Generic tensor kernels over strided views: reductions, gather, dynamic slicing, batched dtype conversion and the
+// any-layout dot product. They are the non-specialised side of the hot path; the specialised side (row kernels,
+// tensor-core GEMM, attention) and the elementwise programs live in their own files.
 #include <cfloat>
 
 #include <mutex>
 
 #include "common.cuh"
+#include "element_access.cuh"
 
+#include <algorithm>
 #include <type_traits>
 
 namespace mhlo {
 namespace {
-
-// ---- loads / stores in a compute domain ----------------------------------------------------------------------
-
-template <typename C>
-__device__ __forceinline__ C load_as(const void* base, int dtype, int64_t off) {
-    switch (dtype) {
-        case MHLO_DT_F32: return static_cast<C>(static_cast<const float*>(base)[off]);
-        case MHLO_DT_F16: return static_cast<C>(__half2float(static_cast<const __half*>(base)[off]));
-        case MHLO_DT_BF16: return static_cast<C>(__bfloat162float(static_cast<const __nv_bfloat16*>(base)[off]));
-        case MHLO_DT_F64: return static_cast<C>(static_cast<const double*>(base)[off]);
-        case MHLO_DT_I1: return static_cast<C>(static_cast<const uint8_t*>(base)[off] != 0);
-        case MHLO_DT_I8: return static_cast<C>(static_cast<const int8_t*>(base)[off]);
-        case MHLO_DT_UI8: return static_cast<C>(static_cast<const uint8_t*>(base)[off]);
-        case MHLO_DT_I16: return static_cast<C>(static_cast<const int16_t*>(base)[off]);
-        case MHLO_DT_UI16: return static_cast<C>(static_cast<const uint16_t*>(base)[off]);
-        case MHLO_DT_I32: return static_cast<C>(static_cast<const int32_t*>(base)[off]);
-        case MHLO_DT_UI32: return static_cast<C>(static_cast<const uint32_t*>(base)[off]);
-        case MHLO_DT_I64: return static_cast<C>(static_cast<const int64_t*>(base)[off]);
-        default: {  // UI64
-            const uint64_t v = static_cast<const uint64_t*>(base)[off];
-            if constexpr (sizeof(C) == 8 && !std::is_floating_point<C>::value) return static_cast<C>(v);
-            return static_cast<C>(v);
-        }
-    }
-}
-
-// float -> integer follows a C cast (toward zero) that saturates at the ends of the result type and maps NaN to 0, for the
-// types narrower than the 64 bits CUDA converts through as well; integer -> narrower integer keeps the low bits.
-template <typename C>
-__device__ __forceinline__ int64_t to_integer(C v, int64_t lo, int64_t hi) {
-    int64_t i = static_cast<int64_t>(v);
-    if constexpr (std::is_floating_point<C>::value) i = i < lo ? lo : (i > hi ? hi : i);
-    return i;
-}
-
-template <typename C>
-__device__ __forceinline__ void store_as(void* base, int dtype, int64_t off, C v) {
-    if constexpr (std::is_floating_point<C>::value) {
-        // NaN -> 0 for every integer type (the hardware conversion gives 0 or the type's minimum depending on the widths)
-        if (v != v && dtype != MHLO_DT_F32 && dtype != MHLO_DT_F16 && dtype != MHLO_DT_BF16 && dtype != MHLO_DT_F64 && dtype != MHLO_DT_I1) v = C(0);
-    }
-    switch (dtype) {
-        case MHLO_DT_F32: static_cast<float*>(base)[off] = static_cast<float>(v); break;
-        case MHLO_DT_F16: static_cast<__half*>(base)[off] = __float2half_rn(static_cast<float>(v)); break;
-        case MHLO_DT_BF16: static_cast<__nv_bfloat16*>(base)[off] = __float2bfloat16_rn(static_cast<float>(v)); break;
-        case MHLO_DT_F64: static_cast<double*>(base)[off] = static_cast<double>(v); break;
-        case MHLO_DT_I1: static_cast<uint8_t*>(base)[off] = v != C(0) ? 1 : 0; break;
-        case MHLO_DT_I8: static_cast<int8_t*>(base)[off] = static_cast<int8_t>(to_integer(v, -128, 127)); break;
-        case MHLO_DT_UI8: static_cast<uint8_t*>(base)[off] = static_cast<uint8_t>(to_integer(v, 0, 255)); break;
-        case MHLO_DT_I16: static_cast<int16_t*>(base)[off] = static_cast<int16_t>(to_integer(v, -32768, 32767)); break;
-        case MHLO_DT_UI16: static_cast<uint16_t*>(base)[off] = static_cast<uint16_t>(to_integer(v, 0, 65535)); break;
-        case MHLO_DT_I32: static_cast<int32_t*>(base)[off] = static_cast<int32_t>(v); break;
-        case MHLO_DT_UI32: static_cast<uint32_t*>(base)[off] = static_cast<uint32_t>(to_integer(v, 0, 4294967295LL)); break;
-        case MHLO_DT_I64: static_cast<int64_t*>(base)[off] = static_cast<int64_t>(v); break;
-        default:
-            if constexpr (std::is_floating_point<C>::value) static_cast<uint64_t*>(base)[off] = static_cast<uint64_t>(v);  // saturates; negative and NaN -> 0
-            else static_cast<uint64_t*>(base)[off] = static_cast<uint64_t>(static_cast<int64_t>(v));
-            break;
-    }
-}
-
-// ---- elementwise program ---------------------------------------------------------------------------------------
-
-struct EwParams {
-    mhlo_cuda_view in[MHLO_CUDA_EW_MAX_INPUTS];
-    mhlo_cuda_ew_inst prog[MHLO_CUDA_EW_MAX_INSTS];
-    int64_t out_shape[MHLO_CUDA_MAX_RANK];
-    int64_t n;
-    void* out;
-    int32_t n_inputs, n_insts, rank, out_dtype;
-    int32_t contiguous_mask;  // bit k: input k is dense row-major over the output shape (offset = linear index)
-    int32_t unsigned_mode;    // integer domain: treat values as uint64 for div/rem/shift/compare/min/max
-    int32_t bool_mode;        // integer domain: NOT is logical (i1)
-    int32_t int_bits;         // integer domain: width of the operand type (shifts, popcnt, clz)
-    int32_t out_strided;      // store through out_stride instead of the linear index
-    int64_t out_stride[MHLO_CUDA_MAX_RANK];
-};
-
-// stablehlo.reduce_precision on the bits of a float (8 / 23) or a double (11 / 52): round the mantissa to nearest even at
-// `mant` bits, then clamp the exponent range to `expo` bits (overflow -> infinity, underflow -> signed zero).
-template <typename U, int kExpBits, int kMantBits>
-__device__ __forceinline__ U reduce_precision_bits(U bits, int expo, int mant) {
-    const U one = 1;
-    const U exp_mask = ((one << kExpBits) - 1) << kMantBits, mant_mask = (one << kMantBits) - 1, sign = bits & (one << (kExpBits + kMantBits));
-    const bool is_nan = (bits & exp_mask) == exp_mask && (bits & mant_mask) != 0;
-    if (is_nan) return mant > 0 ? bits : (sign | exp_mask);  // a format without mantissa bits has no NaN: it becomes infinity
-    if (mant < kMantBits) {
-        const U last = one << (kMantBits - mant);
-        const U bias = (last >> 1) - 1 + ((bits & last) >> (kMantBits - mant));
-        bits = (bits + bias) & ~(last - 1);
-    }
-    if (expo < kExpBits) {
-        const long long full_bias = (1ll << (kExpBits - 1)) - 1, reduced_bias = (1ll << (expo - 1)) - 1;
-        const U max_exp = static_cast<U>(full_bias + reduced_bias) << kMantBits, min_exp = static_cast<U>(full_bias - reduced_bias) << kMantBits;
-        const U e = bits & exp_mask;
-        if (e > max_exp) bits = sign | exp_mask;
-        else if (e <= min_exp) bits = sign;
-    }
-    return bits;
-}
-__device__ __forceinline__ float reduce_precision_value(float a, int expo, int mant) {
-    return __uint_as_float(reduce_precision_bits<uint32_t, 8, 23>(__float_as_uint(a), expo, mant));
-}
-__device__ __forceinline__ double reduce_precision_value(double a, int expo, int mant) {
-    return __longlong_as_double(static_cast<long long>(reduce_precision_bits<unsigned long long, 11, 52>(static_cast<unsigned long long>(__double_as_longlong(a)), expo, mant)));
-}
-
-template <typename C>
-__device__ __forceinline__ C ew_float_op(int op, C a, C b, C c, double imm) {
-    switch (op) {
-        case MHLO_EW_COPY: return a;
-        case MHLO_EW_IMM: return static_cast<C>(imm);
-        case MHLO_EW_ADD: return a + b;
-        case MHLO_EW_SUB: return a - b;
-        case MHLO_EW_MUL: return a * b;
-        case MHLO_EW_DIV: return a / b;
-        case MHLO_EW_REM: return fmod(a, b);
-        case MHLO_EW_MAX: return (a != a || b != b) ? C(NAN) : (a > b ? a : b);
-        case MHLO_EW_MIN: return (a != a || b != b) ? C(NAN) : (a < b ? a : b);
-        case MHLO_EW_POW: return pow(a, b);
-        case MHLO_EW_ATAN2: return atan2(a, b);
-        case MHLO_EW_AND: return C(a != C(0) && b != C(0));
-        case MHLO_EW_OR: return C(a != C(0) || b != C(0));
-        case MHLO_EW_XOR: return C((a != C(0)) != (b != C(0)));
-        case MHLO_EW_NEG: return -a;
-        case MHLO_EW_ABS: return fabs(a);
-        case MHLO_EW_EXP: return exp(a);
-        case MHLO_EW_EXPM1: return expm1(a);
-        case MHLO_EW_LOG: return log(a);
-        case MHLO_EW_LOG1P: return log1p(a);
-        case MHLO_EW_SQRT: return sqrt(a);
-        case MHLO_EW_RSQRT: return C(1) / sqrt(a);
-        case MHLO_EW_CBRT: return cbrt(a);
-        case MHLO_EW_TANH: return tanh(a);
-        case MHLO_EW_LOGISTIC: return C(1) / (C(1) + exp(-a));
-        case MHLO_EW_SIN: return sin(a);
-        case MHLO_EW_COS: return cos(a);
-        case MHLO_EW_TAN: return tan(a);
-        case MHLO_EW_FLOOR: return floor(a);
-        case MHLO_EW_CEIL: return ceil(a);
-        case MHLO_EW_ROUND_AFZ: return round(a);
-        case MHLO_EW_ROUND_EVEN: return rint(a);
-        case MHLO_EW_SIGN: return a != a ? a : C((a > C(0)) - (a < C(0)));
-        case MHLO_EW_NOT: return C(a == C(0));
-        case MHLO_EW_IS_FINITE: return C(isfinite(a) ? 1 : 0);
-        case MHLO_EW_CMP_EQ: return C(a == b);
-        case MHLO_EW_CMP_NE: return C(a != b);
-        case MHLO_EW_CMP_LT: return C(a < b);
-        case MHLO_EW_CMP_LE: return C(a <= b);
-        case MHLO_EW_CMP_GT: return C(a > b);
-        case MHLO_EW_CMP_GE: return C(a >= b);
-        case MHLO_EW_SELECT: return a != C(0) ? b : c;
-        case MHLO_EW_CLAMP: {  // minimum(maximum(operand, min), max), each of which hands a NaN on
-            if (a != a || b != b || c != c) return C(NAN);
-            C lo = b < a ? a : b;
-            return lo > c ? c : lo;
-        }
-        case MHLO_EW_GELU_TANH: {
-            const C inner = C(0.7978845608028654) * (a + C(0.044715) * a * a * a);
-            return C(0.5) * a * (C(1) + tanh(inner));
-        }
-        case MHLO_EW_GELU_ERF: return C(0.5) * a * (C(1) + erf(a * C(0.70710678118654752440)));
-        case MHLO_EW_SILU: return a / (C(1) + exp(-a));
-        case MHLO_EW_RELU: return a > C(0) ? a : (a != a ? a : C(0));
-        case MHLO_EW_ROUND_TO: {
-            const int dt = static_cast<int>(imm);
-            if (dt == MHLO_DT_F16) return C(__half2float(__float2half_rn(static_cast<float>(a))));
-            if (dt == MHLO_DT_BF16) return C(__bfloat162float(__float2bfloat16_rn(static_cast<float>(a))));
-            if (dt == MHLO_DT_F32) return C(static_cast<float>(a));
-            return a;
-        }
-        case MHLO_EW_ERF: return erf(a);
-        case MHLO_EW_REDUCE_PRECISION: return reduce_precision_value(a, static_cast<int>(imm) / 64, static_cast<int>(imm) % 64);
-        default: return a;
-    }
-}
-
-__device__ __forceinline__ int64_t ew_int_op(int op, int64_t a, int64_t b, int64_t c, double imm, bool uns, bool boolean,
-                                             int bits) {
-    const uint64_t ua = static_cast<uint64_t>(a), ub = static_cast<uint64_t>(b);
-    const uint64_t wmask = bits >= 64 ? ~0ull : ((1ull << bits) - 1);  // operand width: shifts and bit counts are per type
-    switch (op) {
-        case MHLO_EW_COPY: return a;
-        case MHLO_EW_IMM: return static_cast<int64_t>(imm);
-        case MHLO_EW_ADD: return static_cast<int64_t>(ua + ub);
-        case MHLO_EW_SUB: return static_cast<int64_t>(ua - ub);
-        case MHLO_EW_MUL: return static_cast<int64_t>(ua * ub);
-        case MHLO_EW_DIV: return b == 0 ? -1 : (uns ? static_cast<int64_t>(ua / ub) : (b == -1 ? static_cast<int64_t>(0 - ua) : a / b));
-        case MHLO_EW_REM: return b == 0 ? a : (uns ? static_cast<int64_t>(ua % ub) : (b == -1 ? 0 : a % b));
-        case MHLO_EW_MAX: return uns ? static_cast<int64_t>(ua > ub ? ua : ub) : (a > b ? a : b);
-        case MHLO_EW_MIN: return uns ? static_cast<int64_t>(ua < ub ? ua : ub) : (a < b ? a : b);
-        case MHLO_EW_POW: {
-            if (b < 0 && !uns) return a == 1 ? 1 : (a == -1 ? ((b & 1) ? -1 : 1) : 0);
-            uint64_t r = 1, base = ua, e = ub;
-            while (e) { if (e & 1) r *= base; base *= base; e >>= 1; }
-            return static_cast<int64_t>(r);
-        }
-        case MHLO_EW_AND: return a & b;
-        case MHLO_EW_OR: return a | b;
-        case MHLO_EW_XOR: return a ^ b;
-        case MHLO_EW_SHL: return ub >= static_cast<uint64_t>(bits) ? 0 : static_cast<int64_t>(ua << ub);
-        case MHLO_EW_SHR_A: return ub >= static_cast<uint64_t>(bits) ? (a < 0 ? -1 : 0) : (a >> ub);
-        case MHLO_EW_SHR_L: return ub >= static_cast<uint64_t>(bits) ? 0 : static_cast<int64_t>((ua & wmask) >> ub);
-        case MHLO_EW_NEG: return static_cast<int64_t>(0 - ua);
-        case MHLO_EW_ABS: return a < 0 ? static_cast<int64_t>(0 - ua) : a;
-        case MHLO_EW_SIGN: return (a > 0) - (a < 0);
-        case MHLO_EW_NOT: return boolean ? (a == 0) : ~a;
-        case MHLO_EW_POPCNT: return __popcll(ua & wmask);
-        case MHLO_EW_CLZ: return __clzll(static_cast<int64_t>(ua & wmask)) - (64 - bits);
-        case MHLO_EW_CMP_EQ: return a == b;
-        case MHLO_EW_CMP_NE: return a != b;
-        case MHLO_EW_CMP_LT: return uns ? ua < ub : a < b;
-        case MHLO_EW_CMP_LE: return uns ? ua <= ub : a <= b;
-        case MHLO_EW_CMP_GT: return uns ? ua > ub : a > b;
-        case MHLO_EW_CMP_GE: return uns ? ua >= ub : a >= b;
-        case MHLO_EW_SELECT: return a != 0 ? b : c;
-        case MHLO_EW_CLAMP: {
-            if (uns) { uint64_t lo = ub < ua ? ua : ub; uint64_t uc = static_cast<uint64_t>(c); return static_cast<int64_t>(lo > uc ? uc : lo); }
-            int64_t lo = b < a ? a : b; return lo > c ? c : lo;
-        }
-        case MHLO_EW_RELU: return a > 0 ? a : 0;
-        case MHLO_EW_IS_FINITE: return 1;
-        default: return a;
-    }
-}
-
-template <typename C>
-__global__ void __launch_bounds__(256) ew_kernel(const __grid_constant__ EwParams p) {
-    constexpr int kRegs = MHLO_CUDA_EW_MAX_INPUTS + MHLO_CUDA_EW_MAX_INSTS;
-    const int64_t step = static_cast<int64_t>(gridDim.x) * blockDim.x;
-    for (int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < p.n; i += step) {
-        int64_t idx[MHLO_CUDA_MAX_RANK];
-        {
-            int64_t rem = i;
-#pragma unroll
-            for (int d = MHLO_CUDA_MAX_RANK - 1; d >= 0; --d) {
-                if (d < p.rank) {
-                    const int64_t e = p.out_shape[d];
-                    idx[d] = rem % e;
-                    rem /= e;
-                } else {
-                    idx[d] = 0;
-                }
-            }
-        }
-        C r[kRegs];
-        for (int k = 0; k < p.n_inputs; ++k) {
-            int64_t off = i;
-            if (!((p.contiguous_mask >> k) & 1)) {
-                off = 0;
-#pragma unroll
-                for (int d = 0; d < MHLO_CUDA_MAX_RANK; ++d)
-                    if (d < p.rank) off += idx[d] * p.in[k].stride[d];
-            }
-            r[k] = load_as<C>(p.in[k].base, p.in[k].dtype, off);
-        }
-        for (int k = 0; k < p.n_insts; ++k) {
-            const mhlo_cuda_ew_inst& in = p.prog[k];
-            C res;
-            if (in.op == MHLO_EW_IOTA) {
-                res = static_cast<C>(idx[static_cast<int>(in.imm)]);
-            } else {
-                const C a = r[in.a], b = r[in.b], c = r[in.c];
-                if constexpr (std::is_floating_point<C>::value) res = ew_float_op<C>(in.op, a, b, c, in.imm);
-                else res = ew_int_op(in.op, a, b, c, in.imm, p.unsigned_mode != 0, p.bool_mode != 0, p.int_bits);
-            }
-            r[p.n_inputs + k] = res;
-        }
-        int64_t oo = i;
-        if (p.out_strided) {
-            oo = 0;
-#pragma unroll
-            for (int d = 0; d < MHLO_CUDA_MAX_RANK; ++d)
-                if (d < p.rank) oo += idx[d] * p.out_stride[d];
-        }
-        store_as<C>(p.out, p.out_dtype, oo, r[p.n_inputs + p.n_insts - 1]);
-    }
-}
-
-// Fast path of the elementwise program: one instruction, float tensors, every input either dense over the output or
-// a single broadcast element. Eight elements per thread through 16-byte accesses; the opcode switch is uniform and
-// works on registers, so residual adds, bias-free activations, converts and dense copies run at memory speed.
-template <typename T>
-__device__ __forceinline__ void load8(const T* p, float* f) {
-    if constexpr (sizeof(T) == 4) {
-        const float4 a = reinterpret_cast<const float4*>(p)[0], b = reinterpret_cast<const float4*>(p)[1];
-        f[0] = a.x; f[1] = a.y; f[2] = a.z; f[3] = a.w; f[4] = b.x; f[5] = b.y; f[6] = b.z; f[7] = b.w;
-    } else {
-        const uint4 v = *reinterpret_cast<const uint4*>(p);
-        VecTraits<T>::unpack(v, f);
-    }
-}
-template <typename T>
-__device__ __forceinline__ void store8(T* p, const float* f) {
-    if constexpr (sizeof(T) == 4) {
-        reinterpret_cast<float4*>(p)[0] = make_float4(f[0], f[1], f[2], f[3]);
-        reinterpret_cast<float4*>(p)[1] = make_float4(f[4], f[5], f[6], f[7]);
-    } else {
-        *reinterpret_cast<uint4*>(p) = VecTraits<T>::pack(f);
-    }
-}
-
-struct EwVecParams {
-    const void* in[3];
-    void* out;
-    int64_t n;
-    int32_t scalar_mask;  // bit k: input k is one broadcast element
-    int32_t n_inputs, op;
-    double imm;
-    int64_t period[3];    // > 0: input k is dense over its trailing dimensions and repeats every `period` elements
-                          // (broadcast over the leading ones: a bias row, a position table); a multiple of 8
-};
-
-template <typename TI, typename TO>
-__global__ void __launch_bounds__(256) ew_vec_kernel(const EwVecParams p) {
-    const int64_t nvec = p.n / 8;
-    const int64_t step = static_cast<int64_t>(gridDim.x) * blockDim.x;
-    float sc[3] = {0.f, 0.f, 0.f};
-    for (int k = 0; k < p.n_inputs; ++k)
-        if ((p.scalar_mask >> k) & 1) sc[k] = VecTraits<TI>::to_float(static_cast<const TI*>(p.in[k])[0]);
-    for (int64_t v = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; v < nvec; v += step) {
-        float x[3][8], r[8];
-#pragma unroll
-        for (int k = 0; k < 3; ++k) {
-            if (k < p.n_inputs && !((p.scalar_mask >> k) & 1)) {
-                const int64_t at = p.period[k] > 0 ? (v * 8) % p.period[k] : v * 8;
-                load8(static_cast<const TI*>(p.in[k]) + at, x[k]);
-            } else {
-#pragma unroll
-                for (int e = 0; e < 8; ++e) x[k][e] = sc[k];
-            }
-        }
-#pragma unroll
-        for (int e = 0; e < 8; ++e) r[e] = ew_float_op<float>(p.op, x[0][e], x[1][e], x[2][e], p.imm);
-        store8(static_cast<TO*>(p.out) + v * 8, r);
-    }
-    // ragged tail
-    if (blockIdx.x == 0 && threadIdx.x < p.n % 8) {
-        const int64_t i = nvec * 8 + threadIdx.x;
-        float x[3];
-        for (int k = 0; k < 3; ++k)
-            x[k] = k < p.n_inputs ? (((p.scalar_mask >> k) & 1) ? sc[k]
-                                                                : VecTraits<TI>::to_float(static_cast<const TI*>(p.in[k])[p.period[k] > 0 ? i % p.period[k] : i]))
-                                  : 0.f;
-        static_cast<TO*>(p.out)[i] = VecTraits<TO>::from_float(ew_float_op<float>(p.op, x[0], x[1], x[2], p.imm));
-    }
-}
-
-template <typename TI>
-bool launch_ew_vec_out(int out_dtype, const EwVecParams& p, int grid, cudaStream_t s) {
-    switch (out_dtype) {
-        case MHLO_DT_F32: ew_vec_kernel<TI, float><<<grid, 256, 0, s>>>(p); return true;
-        case MHLO_DT_F16: ew_vec_kernel<TI, __half><<<grid, 256, 0, s>>>(p); return true;
-        case MHLO_DT_BF16: ew_vec_kernel<TI, __nv_bfloat16><<<grid, 256, 0, s>>>(p); return true;
-        default: return false;
-    }
-}
-
-// Collapses adjacent dimensions that are mergeable in the output and in every input, drops extent-1 dims.
-void collapse_dims(EwParams* p) {
-    int64_t shape[MHLO_CUDA_MAX_RANK];
-    int64_t strides[MHLO_CUDA_EW_MAX_INPUTS][MHLO_CUDA_MAX_RANK];
-    int64_t ostr[MHLO_CUDA_MAX_RANK] = {0};
-    int r = 0;
-    for (int d = 0; d < p->rank; ++d) {
-        if (p->out_shape[d] == 1) continue;
-        bool merge = r > 0;
-        if (merge)
-            for (int k = 0; k < p->n_inputs; ++k)
-                if (strides[k][r - 1] != p->in[k].stride[d] * p->out_shape[d]) { merge = false; break; }
-        if (merge && p->out_strided && ostr[r - 1] != p->out_stride[d] * p->out_shape[d]) merge = false;
-        if (merge) {
-            shape[r - 1] *= p->out_shape[d];
-            for (int k = 0; k < p->n_inputs; ++k) strides[k][r - 1] = p->in[k].stride[d];
-            ostr[r - 1] = p->out_stride[d];
-        } else {
-            shape[r] = p->out_shape[d];
-            for (int k = 0; k < p->n_inputs; ++k) strides[k][r] = p->in[k].stride[d];
-            ostr[r] = p->out_stride[d];
-            ++r;
-        }
-    }
-    p->rank = r;
-    for (int d = 0; d < MHLO_CUDA_MAX_RANK; ++d) p->out_stride[d] = d < r ? ostr[d] : 0;
-    for (int d = 0; d < MHLO_CUDA_MAX_RANK; ++d) {
-        p->out_shape[d] = d < r ? shape[d] : 1;
-        for (int k = 0; k < p->n_inputs; ++k) {
-            p->in[k].stride[d] = d < r ? strides[k][d] : 0;
-            p->in[k].shape[d] = p->out_shape[d];
-        }
-    }
-    for (int k = 0; k < p->n_inputs; ++k) {
-        p->in[k].rank = r;
-        bool dense = true;
-        int64_t expect = 1;
-        for (int d = r - 1; d >= 0; --d) {
-            if (p->in[k].stride[d] != expect) { dense = false; break; }
-            expect *= p->out_shape[d];
-        }
-        if (dense) p->contiguous_mask |= 1 << k;
-    }
-}
 
 // ---- reduce ------------------------------------------------------------------------------------------------------
 
@@ -846,8 +444,6 @@ int grid_for(int64_t n, int threads) {
     return static_cast<int>(g < 1 ? 1 : (g > cap ? cap : g));
 }
 
-bool is_float_dt(int dt) { return dt == MHLO_DT_F16 || dt == MHLO_DT_F32 || dt == MHLO_DT_F64 || dt == MHLO_DT_BF16; }
-
 }  // namespace
 }  // namespace mhlo
 
@@ -932,143 +528,6 @@ __global__ void __launch_bounds__(256) convert_many_kernel(const __grid_constant
 }
 
 extern "C" {
-
-static int elementwise_impl(const mhlo_cuda_view* inputs, int32_t n_inputs, const mhlo_cuda_ew_inst* prog,
-                            int32_t n_insts, void* out_dev, int32_t out_dtype, const int64_t* out_shape,
-                            int32_t out_rank, const int64_t* out_strides, mhlo_cuda_stream_t stream) {
-    if (n_inputs < 0 || n_inputs > MHLO_CUDA_EW_MAX_INPUTS || n_insts < 1 || n_insts > MHLO_CUDA_EW_MAX_INSTS)
-        return fail(MHLO_CUDA_INVALID_ARGUMENT, "elementwise: %d inputs / %d instructions outside the limits (%d / %d)",
-                    n_inputs, n_insts, MHLO_CUDA_EW_MAX_INPUTS, MHLO_CUDA_EW_MAX_INSTS);
-    if (out_rank < 0 || out_rank > MHLO_CUDA_MAX_RANK)
-        return fail(MHLO_CUDA_UNSUPPORTED, "elementwise: rank %d above %d", out_rank, MHLO_CUDA_MAX_RANK);
-    if (mhlo_cuda_dtype_size(out_dtype) == 0) return fail(MHLO_CUDA_INVALID_ARGUMENT, "elementwise: bad output dtype %d", out_dtype);
-    EwParams p;
-    memset(&p, 0, sizeof p);
-    p.n = 1;
-    p.rank = out_rank;
-    for (int d = 0; d < out_rank; ++d) {
-        if (out_shape[d] < 0) return fail(MHLO_CUDA_INVALID_ARGUMENT, "elementwise: negative extent");
-        p.out_shape[d] = out_shape[d];
-        p.n *= out_shape[d];
-    }
-    if (p.n == 0) return MHLO_CUDA_OK;
-    if (out_dev == nullptr) return fail(MHLO_CUDA_INVALID_ARGUMENT, "elementwise: null output");
-    bool any_f64 = out_dtype == MHLO_DT_F64, any_float = is_float_dt(out_dtype), any_u64 = out_dtype == MHLO_DT_UI64;
-    bool all_bool = out_dtype == MHLO_DT_I1;
-    for (int k = 0; k < n_inputs; ++k) {
-        if (inputs[k].rank != out_rank)
-            return fail(MHLO_CUDA_INVALID_ARGUMENT, "elementwise: input %d has rank %d, output has %d", k, inputs[k].rank, out_rank);
-        if (inputs[k].base == nullptr) return fail(MHLO_CUDA_INVALID_ARGUMENT, "elementwise: input %d is null", k);
-        if (mhlo_cuda_dtype_size(inputs[k].dtype) == 0) return fail(MHLO_CUDA_INVALID_ARGUMENT, "elementwise: bad dtype");
-        p.in[k] = inputs[k];
-        any_f64 |= inputs[k].dtype == MHLO_DT_F64;
-        any_float |= is_float_dt(inputs[k].dtype);
-        any_u64 |= inputs[k].dtype == MHLO_DT_UI64;
-        all_bool &= inputs[k].dtype == MHLO_DT_I1;
-    }
-    for (int k = 0; k < n_insts; ++k) {
-        const mhlo_cuda_ew_inst& in = prog[k];
-        const int limit = n_inputs + k;
-        if (in.op < 0 || in.op >= MHLO_EW_OP_COUNT) return fail(MHLO_CUDA_INVALID_ARGUMENT, "elementwise: bad opcode %d", in.op);
-        if (in.op == MHLO_EW_IOTA && (in.imm < 0 || in.imm >= out_rank))
-            return fail(MHLO_CUDA_INVALID_ARGUMENT, "elementwise: iota dimension out of range");
-        const bool nullary = in.op == MHLO_EW_IMM || in.op == MHLO_EW_IOTA;
-        if (!nullary && (in.a < 0 || in.a >= limit || in.b < 0 || in.b >= (limit > 0 ? limit : 1) || in.c < 0 || in.c >= (limit > 0 ? limit : 1)))
-            return fail(MHLO_CUDA_INVALID_ARGUMENT, "elementwise: instruction %d reads a register that is not defined yet", k);
-        p.prog[k] = in;
-        if (nullary) { p.prog[k].a = p.prog[k].b = p.prog[k].c = 0; }
-    }
-    p.n_inputs = n_inputs;
-    p.n_insts = n_insts;
-    p.out = out_dev;
-    p.out_dtype = out_dtype;
-    p.unsigned_mode = any_u64;
-    p.int_bits = static_cast<int>(8 * mhlo_cuda_dtype_size(n_inputs > 0 ? inputs[0].dtype : out_dtype));
-    p.bool_mode = all_bool;
-    if (out_strides != nullptr) {
-        p.out_strided = 1;
-        for (int d = 0; d < out_rank; ++d) p.out_stride[d] = out_strides[d];
-    }
-    // IOTA addresses output dimensions by their original number: keep the shape as is when a program uses it
-    bool uses_iota = false;
-    for (int k = 0; k < n_insts; ++k) uses_iota |= prog[k].op == MHLO_EW_IOTA;
-    if (!uses_iota) collapse_dims(&p);
-    else
-        for (int k = 0; k < n_inputs; ++k) {
-            bool dense = true;
-            int64_t expect = 1;
-            for (int d = out_rank - 1; d >= 0; --d) {
-                if (p.out_shape[d] != 1 && p.in[k].stride[d] != expect) { dense = false; break; }
-                expect *= p.out_shape[d];
-            }
-            if (dense) p.contiguous_mask |= 1 << k;
-        }
-    cudaStream_t s = static_cast<cudaStream_t>(stream);
-    // fast path: one non-iota instruction over dense / scalar float inputs of one dtype
-    if (n_insts == 1 && !uses_iota && out_strides == nullptr && !any_f64 && n_inputs >= 1 && n_inputs <= 3 &&
-        (out_dtype == MHLO_DT_F32 || out_dtype == MHLO_DT_F16 || out_dtype == MHLO_DT_BF16) && aligned16(out_dev)) {
-        const int in_dt = inputs[0].dtype;
-        bool ok = in_dt == MHLO_DT_F32 || in_dt == MHLO_DT_F16 || in_dt == MHLO_DT_BF16;
-        EwVecParams vp;
-        memset(&vp, 0, sizeof vp);
-        for (int k = 0; k < n_inputs && ok; ++k) {
-            bool scalar = true;
-            for (int d = 0; d < p.rank; ++d) scalar &= p.in[k].stride[d] == 0;
-            const bool dense = (p.contiguous_mask >> k) & 1;
-            // broadcast over leading dimensions, dense over the rest: the input repeats with a fixed period
-            int64_t period = 0;
-            if (!scalar && !dense) {
-                int q = 0;
-                while (q < p.rank && p.in[k].stride[q] == 0) ++q;
-                int64_t expect = 1;
-                bool tail_dense = q > 0 && q < p.rank;
-                for (int d = p.rank - 1; d >= q && tail_dense; --d) {
-                    tail_dense = p.out_shape[d] == 1 || p.in[k].stride[d] == expect;
-                    expect *= p.out_shape[d];
-                }
-                if (tail_dense && expect % 8 == 0) period = expect;
-            }
-            vp.period[k] = period;
-            ok = p.in[k].dtype == in_dt && (scalar || ((dense || period > 0) && aligned16(p.in[k].base)));
-            if (scalar && !(dense && p.n == 1)) vp.scalar_mask |= 1 << k;
-            vp.in[k] = p.in[k].base;
-        }
-        // instruction operands must name the inputs in order (a = 0, b = 1, c = 2), which is how single ops are built
-        ok = ok && prog[0].a == 0 && (n_inputs < 2 || prog[0].b == 1) && (n_inputs < 3 || prog[0].c == 2);
-        if (ok) {
-            vp.out = out_dev; vp.n = p.n; vp.n_inputs = n_inputs; vp.op = prog[0].op; vp.imm = prog[0].imm;
-            const int vgrid = grid_for((p.n + 7) / 8, 256);
-            bool launched = false;
-            if (in_dt == MHLO_DT_F32) launched = launch_ew_vec_out<float>(out_dtype, vp, vgrid, s);
-            else if (in_dt == MHLO_DT_F16) launched = launch_ew_vec_out<__half>(out_dtype, vp, vgrid, s);
-            else launched = launch_ew_vec_out<__nv_bfloat16>(out_dtype, vp, vgrid, s);
-            if (launched) {
-                MHLO_CUDA_CHECK_LAUNCH("elementwise_vec");
-                return MHLO_CUDA_OK;
-            }
-        }
-    }
-    const int grid = grid_for(p.n, 256);
-    if (any_f64) ew_kernel<double><<<grid, 256, 0, s>>>(p);
-    else if (any_float) ew_kernel<float><<<grid, 256, 0, s>>>(p);
-    else ew_kernel<int64_t><<<grid, 256, 0, s>>>(p);
-    MHLO_CUDA_CHECK_LAUNCH("elementwise");
-    return MHLO_CUDA_OK;
-}
-
-int mhlo_cuda_elementwise(const mhlo_cuda_view* inputs, int32_t n_inputs, const mhlo_cuda_ew_inst* prog,
-                          int32_t n_insts, void* out_dev, int32_t out_dtype, const int64_t* out_shape,
-                          int32_t out_rank, mhlo_cuda_stream_t stream) {
-    return elementwise_impl(inputs, n_inputs, prog, n_insts, out_dev, out_dtype, out_shape, out_rank, nullptr, stream);
-}
-
-int mhlo_cuda_elementwise_to_view(const mhlo_cuda_view* inputs, int32_t n_inputs, const mhlo_cuda_ew_inst* prog,
-                                  int32_t n_insts, const mhlo_cuda_view* out, mhlo_cuda_stream_t stream) {
-    if (!out || out->rank < 0 || out->rank > MHLO_CUDA_MAX_RANK)
-        return fail(MHLO_CUDA_INVALID_ARGUMENT, "elementwise_to_view: bad destination view");
-    return elementwise_impl(inputs, n_inputs, prog, n_insts, const_cast<void*>(out->base), out->dtype, out->shape,
-                            out->rank, out->stride, stream);
-}
 
 namespace {
 // Enqueues both kernels of a split reduce over `scratch` (plan.scratch_bytes, no initial contents required).

@@ -50,6 +50,9 @@ struct AttnShape {
 // Tensor-core (tcgen05 + TMA + TMEM) paths; *_supported() says whether the problem meets their layout rules.
 bool gemm_tc_supported(const GemmProblem& p);
 int gemm_tc_launch(const GemmProblem& p, cudaStream_t stream);
+// fp32 operands and results on the FMA units, any strides.
+bool gemm_fp32_supported(const GemmProblem& p);
+int gemm_fp32_launch(const GemmProblem& p, cudaStream_t stream);
 int gemm_device_error();       // synchronises; returns and clears the GEMM kernel's error word (-1: CUDA error)
 int attention_device_error();  // same for the attention kernel
 // Stream-ordered copies of the error words into pinned host memory, and host stores into them (clearing, or the test hook).

@@ -5,7 +5,7 @@
 
 #include <mutex>
 
-#include "common.cuh"
+#include "contraction.cuh"
 #include "element_access.cuh"
 
 #include <algorithm>
@@ -897,6 +897,14 @@ int mhlo_cuda_dot_strided(int32_t in_dtype, int32_t out_dtype, const void* a_dev
     if (batch0 * batch1 * m * n == 0) return MHLO_CUDA_OK;
     if (!c_dev || (k > 0 && (!a_dev || !b_dev))) return fail(MHLO_CUDA_INVALID_ARGUMENT, "dot: null pointer");
     if (batch0 * batch1 > 65535) return fail(MHLO_CUDA_UNSUPPORTED, "dot: more than 65535 batch entries");
+    if (in_dtype == MHLO_DT_F32 && out_dtype == MHLO_DT_F32) {
+        GemmProblem g;
+        g.a = a_dev; g.b = b_dev; g.c = c_dev; g.bias = nullptr;
+        for (int i = 0; i < 4; ++i) { g.as[i] = a_strides[i]; g.bs[i] = b_strides[i]; }
+        g.batch0 = batch0; g.batch1 = batch1; g.m = m; g.n = n; g.k = k;
+        g.in_dtype = in_dtype; g.out_dtype = out_dtype; g.epilogue = MHLO_EPILOGUE_NONE;
+        if (gemm_fp32_supported(g)) return gemm_fp32_launch(g, static_cast<cudaStream_t>(stream));
+    }
     DotParams p;
     p.a = a_dev; p.b = b_dev; p.c = c_dev;
     for (int i = 0; i < 4; ++i) { p.as[i] = a_strides[i]; p.bs[i] = b_strides[i]; }

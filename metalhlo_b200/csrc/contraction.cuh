@@ -64,6 +64,9 @@ bool gemm_wait_expiry_probe(uint64_t limit_ns, cudaStream_t stream);
 // One CTA: stores `epoch` into word `rank` of every other rank's flag array, then waits (at most limit_ns) until every word
 // of this rank's own array has reached `epoch`; an expired wait records code 95 in the GEMM error word.
 bool gemm_peer_barrier_launch(uint64_t* const* flag_arrays, int n_ranks, int rank, uint64_t epoch, uint64_t limit_ns, cudaStream_t stream);
+// fp32 on the FMA units: any strides, optional additive mask, head dimensions up to 128.
+bool attention_fp32_supported(int dtype, const AttnShape& s);
+int attention_fp32_launch(const void* q, const void* k, const void* v, const void* mask, void* o, const AttnShape& s, cudaStream_t stream);
 bool attention_tc_supported(int dtype, const AttnShape& s, const void* mask);
 int attention_tc_launch(int dtype, const void* q, const void* k, const void* v, void* o, const AttnShape& s,
                         cudaStream_t stream);

@@ -364,6 +364,7 @@ int mhlo_cuda_attention_tuned(int32_t dtype, const void* q_dev, const int64_t q_
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     if (attention_tc_supported(dtype, s, mask_dev) && aligned16(q_dev) && aligned16(k_dev) && aligned16(v_dev) && aligned16(o_dev))
         return attention_tc_launch(dtype, q_dev, k_dev, v_dev, o_dev, s, st);
+    if (attention_fp32_supported(dtype, s)) return attention_fp32_launch(q_dev, k_dev, v_dev, mask_dev, o_dev, s, st);
     if (head_dim > 256) return fail(MHLO_CUDA_UNSUPPORTED, "attention: head_dim %lld above 256", (long long)head_dim);
     switch (dtype) {
         case MHLO_DT_F32: return launch_attention_rows<float>(q_dev, k_dev, v_dev, mask_dev, o_dev, s, st);

@@ -46,3 +46,31 @@ def test_gemm_fp32_batched_with_epilogue(batch, epilogue):
     want = a.double() @ b.double() + bias.double()
     want = {"none": lambda x: x, "relu": torch.relu, "gelu_tanh": lambda x: torch.nn.functional.gelu(x, approximate="tanh")}[epilogue](want)
     assert_close(to_np(got), want.numpy(), 1e-5, f"gemm fp32 {batch} {epilogue}")
+
+
+# row groups of 32, 64 and 128; one or two warps per group (head dimensions up to 64 and up to 128); keys shared by a cluster
+@pytest.mark.parametrize("causal", [False, True])
+@pytest.mark.parametrize("b,h,sq,sk,d", [(1, 1, 1, 1, 64), (1, 2, 33, 65, 64), (1, 1, 300, 1030, 64), (2, 40, 130, 96, 40), (3, 50, 129, 257, 64),
+                                         (1, 3, 31, 33, 128), (2, 5, 97, 300, 80), (3, 50, 128, 129, 128), (1, 2, 65, 64, 33)])
+def test_attention_fp32(causal, b, h, sq, sk, d):
+    g = torch.Generator().manual_seed(sq + sk + d)
+    q, k, v = (torch.randn(b, h, s, d, generator=g) for s in (sq, sk, sk))
+    scale = 1 / math.sqrt(d)
+    got = cuda_mod().attention(q.cuda(), k.cuda(), v.cuda(), scale, causal=causal)
+    assert_close(to_np(got), oracle.attention(q, k, v, scale, causal=causal), 1e-5, f"{sq}x{sk} d{d}",
+                 magnitude=oracle.attention(q, k, v.abs(), scale, causal=causal))
+
+
+@pytest.mark.parametrize("d", [64, 100])
+def test_attention_fp32_mask_and_interleaved_heads(d):
+    g = torch.Generator().manual_seed(d)
+    q, k, v = (torch.randn(2, s, 3, d, generator=g) for s in (70, 90, 90))
+    mask = torch.randn(70, 90, generator=g)
+    mask[3] = -math.inf  # a row that sees nothing
+    mask[5, 1:] = -math.inf
+    got = to_np(cuda_mod().attention(q.cuda(), k.cuda(), v.cuda(), 0.1, mask=mask.cuda(), layout="BSHD")).transpose(0, 2, 1, 3)
+    qt, kt, vt = (t.permute(0, 2, 1, 3).contiguous() for t in (q, k, v))
+    s = qt.double() @ kt.double().transpose(-1, -2) * 0.1 + mask.double()
+    p = torch.nan_to_num(torch.softmax(s, -1), nan=0.0)
+    assert np.all(got[:, :, 3] == 0)
+    assert_close(got, (p @ vt.double()).numpy(), 1e-5, "masked", magnitude=(p @ vt.double().abs()).numpy())

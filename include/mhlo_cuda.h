@@ -541,6 +541,8 @@ int mhlo_cuda_gemm(int32_t in_dtype, int32_t out_dtype, const void* a_dev, const
  *   stages     depth of the TMA operand ring, 2 .. the kernel's maximum (4 for 128x256 tiles, 6 otherwise)
  *   cta_group  1: one CTA per 128-row tile; 2: a pair of CTAs on neighbouring SMs per 256 x 256 tile, each staging
  *              its own rows of A and its own half of B (tcgen05 cta_group::2; no load is multicast)
+ *   split_k    1: K may be split over a cluster of CTAs where that is faster and the knobs above are 0 (what compiled programs
+ *              ask for); 0: one running sum over K, the same bits for every value of the other knobs
  * mhlo_cuda_gemm_tuned is mhlo_cuda_gemm with these knobs; tuning == NULL is mhlo_cuda_gemm. Problems outside the
  * tensor-core path ignore the knobs.
  */
@@ -548,7 +550,7 @@ typedef struct {
     int32_t tile_n;
     int32_t stages;
     int32_t cta_group;
-    int32_t reserved;
+    int32_t split_k;
 } mhlo_cuda_gemm_tuning;
 
 int mhlo_cuda_gemm_tuned(int32_t in_dtype, int32_t out_dtype, const void* a_dev, const int64_t a_strides[4],

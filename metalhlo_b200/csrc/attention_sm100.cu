@@ -724,7 +724,7 @@ int launch_attention(int dtype, const void* q, const void* k, const void* v, voi
     if (s.tile_order == 1) p.by_length = 0;
     else if (s.tile_order == 2 && tiles < (int64_t{1} << 30)) p.by_length = 1;
     const unsigned grid = static_cast<unsigned>(p.by_length ? std::min<int64_t>(tiles, sm_count) : std::min<int64_t>((tiles + 1) / 2, sm_count));
-    const cudaError_t launched = launch_dependent(kernel, dim3(grid), dim3(kAttnThreads), L::kTotal, stream, mq, mk, mv, p);
+    const cudaError_t launched = launch_dependent(kernel, dim3(grid), dim3(kAttnThreads), L::kTotal, stream, 1, grid < kNumSMs, mq, mk, mv, p);
     if (launched != cudaSuccess) return fail(MHLO_CUDA_EXECUTION_FAILED, "launch of attention_tcgen05 failed: %s", cudaGetErrorString(launched));
     MHLO_CUDA_CHECK_LAUNCH("attention_tcgen05");
     return MHLO_CUDA_OK;

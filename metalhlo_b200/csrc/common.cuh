@@ -75,29 +75,16 @@ struct FastDiv {
 __device__ __forceinline__ void grid_dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void grid_dependency_release() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
-// METALHLO_PDL=0 turns the overlap off (every launch then waits for the previous kernel to finish, as usual).
-bool dependent_launch_enabled();
+// METALHLO_PDL=0 / 1 turns the overlap off / on for every kernel; otherwise a launch says for itself whether it wants it.
+bool dependent_launch_enabled(bool wanted);
 
-// Launches `kernel`, which calls grid_dependency_wait(), with the programmatic-serialisation attribute when enabled.
+// Launches `kernel`, which calls grid_dependency_wait(), as thread-block clusters of `cluster_x` CTAs along x (1 = no cluster
+// attribute). overlap: with the programmatic-serialisation attribute, for grids that leave SMs idle - the next kernel's
+// launch, barrier set-up and tensor-memory allocation then run beside the tail of this one (about 1.2 us per kernel in a
+// graph of layer products of 201 rows). A grid that fills the machine gains nothing: its successor's CTAs find no room.
 template <typename... KArgs, typename... Args>
-cudaError_t launch_dependent(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, Args&&... args) {
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = grid;
-    cfg.blockDim = block;
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = stream;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = dependent_launch_enabled() ? 1 : 0;
-    return cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
-}
-
-// The same for a kernel that runs as thread-block clusters of `cluster_x` CTAs along x (1 = no cluster attribute).
-template <typename... KArgs, typename... Args>
-cudaError_t launch_dependent_cluster(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, int cluster_x,
-                                     Args&&... args) {
+cudaError_t launch_dependent(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, int cluster_x, bool overlap,
+                             Args&&... args) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = grid;
     cfg.blockDim = block;
@@ -105,7 +92,7 @@ cudaError_t launch_dependent_cluster(void (*kernel)(KArgs...), dim3 grid, dim3 b
     cfg.stream = stream;
     cudaLaunchAttribute attr[2];
     int n = 0;
-    if (dependent_launch_enabled()) {
+    if (dependent_launch_enabled(overlap)) {
         attr[n].id = cudaLaunchAttributeProgrammaticStreamSerialization;
         attr[n].val.programmaticStreamSerializationAllowed = 1;
         ++n;

@@ -23,6 +23,7 @@ struct GemmProblem {
     // Launch knobs of the tensor-core kernel; 0 = chosen by the library. tile_n: 128 or 256 columns per tile; stages: depth
     // of the TMA ring; cta_group: 1 = one CTA per 128-row tile, 2 = a pair of CTAs per 256-row tile.
     int32_t tile_n = 0, stages = 0, cta_group = 0;
+    int32_t split_k = 0;  // 1: the sum over K may be split (see mhlo_cuda_gemm_tuning)
 };
 
 // A 2-D convolution of dense NHWC input with dense HWIO filters into dense NHWC output, stride 1, one feature group: the

@@ -188,7 +188,7 @@ int mhlo_cuda_gemm_tuned(int32_t in_dtype, int32_t out_dtype, const void* a_dev,
     for (int i = 0; i < 4; ++i) { p.as[i] = a_strides[i]; p.bs[i] = b_strides[i]; }
     p.batch0 = batch0; p.batch1 = batch1; p.m = m; p.n = n; p.k = k;
     p.in_dtype = in_dtype; p.out_dtype = out_dtype; p.epilogue = epilogue;
-    if (tuning) { p.tile_n = tuning->tile_n; p.stages = tuning->stages; p.cta_group = tuning->cta_group; }
+    if (tuning) { p.tile_n = tuning->tile_n; p.stages = tuning->stages; p.cta_group = tuning->cta_group; p.split_k = tuning->split_k; }
     if (gemm_tc_supported(p)) return gemm_tc_launch(p, static_cast<cudaStream_t>(stream));
     if (gemm_fp32_supported(p)) return gemm_fp32_launch(p, static_cast<cudaStream_t>(stream));
     int st = mhlo_cuda_dot_strided(in_dtype, out_dtype, a_dev, a_strides, b_dev, b_strides, c_dev, batch0, batch1, m, n, k, stream);

@@ -25,6 +25,7 @@
 
 #include <algorithm>
 #include <string>
+#include <type_traits>
 
 #include "contraction.cuh"
 #include "tc_ptx.cuh"
@@ -131,6 +132,8 @@ __device__ __forceinline__ void tile_coords(int64_t tile, const GemmParams& p, i
     *tm = band * kBand + static_cast<int>(t % rows_in_band);
     *tn = static_cast<int>(t / rows_in_band);
 }
+
+#include "gemm_cluster.cuh"
 
 // MODE: 0 = the plain product, 1 = with the tensor maps of further copies of C (bulk stores into peers), 2 = with a residual
 // matrix added in the epilogue, 3 = a 2-D convolution read straight from its NHWC input: the A tile of k-block (tap, 64
@@ -690,7 +693,7 @@ bool gemm_tc_supported(const GemmProblem& p) {
     if (!f16 && !bf16) return false;
     if (p.out_dtype != p.in_dtype && p.out_dtype != MHLO_DT_F32) return false;
     if (p.m <= 0 || p.n <= 0 || p.k <= 0 || p.batch0 <= 0 || p.batch1 <= 0) return false;
-    if (p.m * p.n < 64 * 64) return false;  // tiny products: the general kernel has less fixed cost
+    if (p.m * p.n * p.k < 32 * 1024) return false;  // a few panels of the general kernel take less than the fixed cost
     if (!aligned16(p.a) || !aligned16(p.b)) return false;
     // one of (row, col) strides must be 1; the other, and the batch strides, 16-byte multiples
     const bool a_k = p.as[3] == 1 || p.k == 1, a_m = p.as[2] == 1 || p.m == 1;
@@ -804,7 +807,7 @@ static int launch_gemm_act(const GemmProblem& pr, cudaStream_t stream) {
         walkers = pairs;
     }
     const int grid = CTAS * static_cast<int>(std::min<int64_t>(p.num_tiles, walkers));
-    const cudaError_t launched = launch_dependent_cluster(kernel, dim3(grid), dim3(kGemmThreads), L::kTotal, stream, CTAS, map_a, map_b, map_c, p, peer_maps);
+    const cudaError_t launched = launch_dependent(kernel, dim3(grid), dim3(kGemmThreads), L::kTotal, stream, CTAS, grid < kNumSMs, map_a, map_b, map_c, p, peer_maps);
     if (launched != cudaSuccess) return fail(MHLO_CUDA_EXECUTION_FAILED, "launch of gemm_tcgen05 failed: %s", cudaGetErrorString(launched));
     MHLO_CUDA_CHECK_LAUNCH("gemm_tcgen05");
     return MHLO_CUDA_OK;
@@ -830,6 +833,77 @@ static int launch_gemm(const GemmProblem& p, cudaStream_t stream) {
         case MHLO_EPILOGUE_SIGMOID: return launch_gemm_act<BN, STAGES, MHLO_EPILOGUE_SIGMOID, CTAS>(p, stream);
         default: return launch_gemm_act<BN, STAGES, MHLO_EPILOGUE_NONE, CTAS>(p, stream);
     }
+}
+
+// ---- few tiles: K split over a cluster (gemm_cluster.cuh) ----
+
+template <int BN>
+static int launch_cluster(const GemmProblem& pr, int splits, cudaStream_t stream) {
+    using L = ClusterLayout<BN>;
+    const bool a_k = pr.as[3] == 1 || pr.k == 1, b_k = pr.bs[2] == 1 || pr.k == 1;
+    CUtensorMap map_a, map_b;
+    std::string why;
+    bool ok;
+    if (a_k) ok = operand_map(&map_a, pr.a, pr.k, pr.m, pr.as[2], pr.batch1, pr.as[1], pr.batch0, pr.as[0], BK, BM, &why);
+    else ok = operand_map(&map_a, pr.a, pr.m, pr.k, pr.as[3], pr.batch1, pr.as[1], pr.batch0, pr.as[0], 64, BK, &why);
+    if (!ok) return fail(MHLO_CUDA_EXECUTION_FAILED, "gemm: tensor map for A: %s", why.c_str());
+    if (b_k) ok = operand_map(&map_b, pr.b, pr.k, pr.n, pr.bs[3], pr.batch1, pr.bs[1], pr.batch0, pr.bs[0], BK, BN, &why);
+    else ok = operand_map(&map_b, pr.b, pr.n, pr.k, pr.bs[2], pr.batch1, pr.bs[1], pr.batch0, pr.bs[0], 64, BK, &why);
+    if (!ok) return fail(MHLO_CUDA_EXECUTION_FAILED, "gemm: tensor map for B: %s", why.c_str());
+    GemmParams p;
+    memset(&p, 0, sizeof p);
+    p.c = pr.c;
+    p.bias = pr.bias;
+    p.m = pr.m; p.n = pr.n; p.k = pr.k;
+    p.batch0 = pr.batch0; p.batch1 = pr.batch1;
+    p.tiles_m = static_cast<int>((pr.m + BM - 1) / BM);
+    p.tiles_n = static_cast<int>((pr.n + BN - 1) / BN);
+    p.num_tiles = static_cast<int64_t>(p.tiles_m) * p.tiles_n * pr.batch0 * pr.batch1;
+    p.a_mn_major = a_k ? 0 : 1;
+    p.b_mn_major = b_k ? 0 : 1;
+    p.in_bf16 = pr.in_dtype == MHLO_DT_BF16;
+    p.out_dtype = pr.out_dtype;
+    p.epilogue = pr.epilogue;
+    const uintptr_t grid = pr.out_dtype == MHLO_DT_F32 ? 16 : 8;  // four results per store
+    p.c_vec_ok = pr.n % 4 == 0 && reinterpret_cast<uintptr_t>(pr.c) % grid == 0;
+    static std::atomic<bool> attr_set[64];
+    int dev = 0;
+    MHLO_CUDA_TRY(cudaGetDevice(&dev), MHLO_CUDA_EXECUTION_FAILED);
+    if (dev < 0 || dev >= 64 || !attr_set[dev].load(std::memory_order_acquire)) {
+        MHLO_CUDA_TRY(cudaFuncSetAttribute(gemm_cluster_kernel<BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, L::kTotal), MHLO_CUDA_EXECUTION_FAILED);
+        if (dev >= 0 && dev < 64) attr_set[dev].store(true, std::memory_order_release);
+    }
+    const cudaError_t launched = launch_dependent(gemm_cluster_kernel<BN>, dim3(static_cast<unsigned>(p.num_tiles * splits)), dim3(kClusterThreads),
+                                                          L::kTotal, stream, splits, true, map_a, map_b, p, splits);
+    if (launched != cudaSuccess) return fail(MHLO_CUDA_EXECUTION_FAILED, "launch of gemm_cluster failed: %s", cudaGetErrorString(launched));
+    MHLO_CUDA_CHECK_LAUNCH("gemm_cluster");
+    return MHLO_CUDA_OK;
+}
+
+// Whether K is split over a cluster, and how: the cheaper of the configurations by a model of measured times (us, kernels
+// behind one another in a graph). One CTA per 128-column tile: 4.5 + 0.27 per 64-deep step of K. A cluster: 4.2, 0.25 or 0.275
+// per step of a 64- or 128-column tile, 0.5 to 0.7 for the exchange; steps cost half as much again once the CTAs outnumber the
+// SMs (two then share a port to L2), and clusters of four and eight do not pack the GPCs completely from about 112 CTAs on.
+// A saving below one microsecond leaves the sum over K in one piece.
+// Measured, [rows, K] . [K, N]: 201 x 768 x 768 8.6 -> 4.8, 201 x 3072 x 768 18.8 -> 7.7, 201 x 768 x 2304 8.4 -> 5.8,
+// 201 x 768 x 3072 9.3 -> 7.2, 1024 x 3072 x 768 19.1 -> 13.1, 256 x 8192 x 256 41.3 -> 8.1; 512 x 768 x 3072 stays with whole tiles.
+// Returns the CTAs per cluster, 0 = no split.
+static int cluster_plan(const GemmProblem& p, int* bn) {
+    if (p.n_copies > 0 || p.residual != nullptr || p.c_col0 != 0 || (p.ldc != 0 && p.ldc != p.n)) return 0;
+    const int64_t rows = (p.m + BM - 1) / BM * p.batch0 * p.batch1, steps = (p.k + BK - 1) / BK;
+    const int64_t whole = rows * ((p.n + 127) / 128);
+    if (whole > kNumSMs || steps < 2) return 0;
+    double best = 4.5 + 0.27 * static_cast<double>(steps) - 1.0;
+    int splits = 0;
+    for (const int width : {64, 128})
+        for (const int s : {2, 4, 8}) {
+            const int64_t ctas = rows * ((p.n + width - 1) / width) * s;
+            if (steps < s || ctas > 2 * kNumSMs) continue;
+            const double load = ctas <= (s == 2 ? kNumSMs : 112) ? 1.0 : ctas <= kNumSMs ? 1.3 : 1.5;
+            const double t = 4.2 + load * static_cast<double>((steps + s - 1) / s) * (width == 64 ? 0.25 : 0.275) + (s == 8 ? 0.7 : s == 4 ? 0.5 : 0.6);
+            if (t < best) { best = t; splits = s; *bn = width; }
+        }
+    return splits;
 }
 
 // ---- convolution without a patch matrix (MODE 3) ----
@@ -937,7 +1011,7 @@ static int launch_conv_act(const ConvProblem& c, cudaStream_t stream) {
     }
     const int grid = static_cast<int>(std::min<int64_t>(p.num_tiles, kNumSMs));
     PeerMaps<false> none;
-    const cudaError_t launched = launch_dependent_cluster(kernel, dim3(grid), dim3(kGemmThreads), L::kTotal, stream, 1, map_a, map_b, map_c, p, none);
+    const cudaError_t launched = launch_dependent(kernel, dim3(grid), dim3(kGemmThreads), L::kTotal, stream, 1, grid < kNumSMs, map_a, map_b, map_c, p, none);
     if (launched != cudaSuccess) return fail(MHLO_CUDA_EXECUTION_FAILED, "launch of the convolution failed: %s", cudaGetErrorString(launched));
     MHLO_CUDA_CHECK_LAUNCH("convolution (tcgen05)");
     return MHLO_CUDA_OK;
@@ -966,6 +1040,11 @@ int gemm_tc_launch(const GemmProblem& p, cudaStream_t stream) {
     }();
     int cta_group = p.cta_group;
     if (cta_group == 0 && pair_env >= 0 && p.n_copies == 0) cta_group = pair_env + 1;
+    if (p.split_k == 1 && cta_group == 0 && p.tile_n == 0 && p.stages == 0) {
+        int bn = 0;
+        const int splits = cluster_plan(p, &bn);
+        if (splits > 0) return bn == 64 ? launch_cluster<64>(p, splits, stream) : launch_cluster<128>(p, splits, stream);
+    }
     if (cta_group == 2) return launch_gemm<256, 6, 2>(p, stream);
     if (p.tile_n == 256) return launch_gemm<256, 4>(p, stream);
     if (p.tile_n == 128) return launch_gemm<128, 6>(p, stream);

@@ -946,12 +946,12 @@ class Lowering {
                 GemmCase gc;
                 gc.dtype = in_dt; gc.out_dtype = out_dt; gc.batch = b0 * b1; gc.m = M; gc.n = N; gc.k = K;
                 gc.a_k_major = as[3] == 1 || K == 1; gc.b_k_major = bs[2] == 1 || K == 1;
-                mhlo_cuda_gemm_tuning gt{0, 0, 0, 0};
+                mhlo_cuda_gemm_tuning gt{0, 0, 0, 1};  // K may be split over a cluster
                 const bool tuned = lookup_gemm_tuning(gc, &gt);
                 add_step(tuned ? "dot_general [tuned]" : "dot_general", [=](const Ctx& c) {
                     return mhlo_cuda_gemm_tuned(in_dt, out_dt, bind(da, c).base, asv.data(), bind(db, c).base, bsv.data(),
                                                 const_cast<void*>(bind(dc, c).base), b0, b1, M, N, K, nullptr, MHLO_EPILOGUE_NONE,
-                                                tuned ? &gt : nullptr, c.stream);
+                                                &gt, c.stream);
                 });
                 return set(op.results[0], out);
             }
@@ -1217,8 +1217,9 @@ class Lowering {
         const int epi = in_epilogue ? epilogue : MHLO_EPILOGUE_NONE;
         if (fused) *fused = in_epilogue;
         add_step(in_epilogue ? "convolution.gemm+epilogue" : "convolution.gemm", [=](const Ctx& cx) {
-            return mhlo_cuda_gemm(dt, dt, bind(dcols, cx).base, as.data(), bind(dwm, cx).base, bs.data(), const_cast<void*>(bind(dprod, cx).base), 1, G,
-                                  M, Og, Kc, with_bias ? bind(dbias, cx).base : nullptr, epi, cx.stream);
+            const mhlo_cuda_gemm_tuning gt{0, 0, 0, 1};  // K may be split over a cluster
+            return mhlo_cuda_gemm_tuned(dt, dt, bind(dcols, cx).base, as.data(), bind(dwm, cx).base, bs.data(), const_cast<void*>(bind(dprod, cx).base),
+                                        1, G, M, Og, Kc, with_bias ? bind(dbias, cx).base : nullptr, epi, &gt, cx.stream);
         });
         // [G, batch, spatial.., Og] -> canonical [batch, spatial.., O] -> the result's own dimension order
         View canon = prod;
@@ -2062,7 +2063,7 @@ void Lowering::lower_custom_call(const Op& op) {
         GemmCase gc;
         gc.dtype = in_dt; gc.out_dtype = out_dt; gc.batch = 1; gc.m = M; gc.n = N; gc.k = K;
         gc.a_k_major = true; gc.b_k_major = w.strides[0] == 1 || K == 1;
-        mhlo_cuda_gemm_tuning gt{0, 0, 0, 0};
+        mhlo_cuda_gemm_tuning gt{0, 0, 0, 1};  // K may be split over a cluster
         const bool tuned = lookup_gemm_tuning(gc, &gt);
         add_step(tuned ? target + " [tuned]" : target, [=](const Ctx& c) {
             if (has_residual)
@@ -2071,7 +2072,7 @@ void Lowering::lower_custom_call(const Op& op) {
                                                bind(dres, c).base, tuned ? &gt : nullptr, c.stream);
             return mhlo_cuda_gemm_tuned(in_dt, out_dt, bind(dx, c).base, as.data(), bind(dw, c).base, bs.data(),
                                         const_cast<void*>(bind(dout, c).base), 1, 1, M, N, K, has_bias ? bind(dbias, c).base : nullptr,
-                                        epi, tuned ? &gt : nullptr, c.stream);
+                                        epi, &gt, c.stream);
         });
         return set(op.results[0], out);
     }

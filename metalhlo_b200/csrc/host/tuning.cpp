@@ -660,8 +660,8 @@ int tune_gemm(const GemmCase& c, int max_trials, TuningDatabase* db, TuningRecor
     best.measured_time_s = 1e30;
     int tried = 0;
     for (const TuningConfig& cand : candidates) {
-        mhlo_cuda_gemm_tuning t{cand.tile_n, cand.stages, cand.cta_group, 0};
-        const mhlo_cuda_gemm_tuning* tp = cand.is_default() ? nullptr : &t;
+        mhlo_cuda_gemm_tuning t{cand.tile_n, cand.stages, cand.cta_group, 1};  // the default is timed as compiled programs launch it
+        const mhlo_cuda_gemm_tuning* tp = &t;
         const double sec = median_seconds([&] {
             return mhlo_cuda_gemm_tuned(c.dtype, c.out_dtype, a, as, b, bs, d, 1, c.batch, c.m, c.n, c.k, nullptr, MHLO_EPILOGUE_NONE, tp, nullptr);
         }, e0, e1);

@@ -467,7 +467,8 @@ int launch_rows(const void* x, const void* gamma, const void* beta, void* y, int
         if (grid > static_cast<int64_t>(kNumSMs) * per_sm) grid = static_cast<int64_t>(kNumSMs) * per_sm;
     }
     if (grid > 0x7fffffffLL) grid = 0x7fffffffLL;
-    const cudaError_t launched = launch_dependent(kernel, dim3(static_cast<unsigned>(grid)), dim3(static_cast<unsigned>(threads)), smem, stream, xp, gp, bp, yp,
+    const cudaError_t launched = launch_dependent(kernel, dim3(static_cast<unsigned>(grid)), dim3(static_cast<unsigned>(threads)), smem, stream, 1,
+                                                  grid * threads <= 512 * kNumSMs, xp, gp, bp, yp,
                                                   rows, static_cast<int>(len), eps, static_cast<const T*>(res), static_cast<T*>(sum_out), res_rows);
     if (launched != cudaSuccess) return fail(MHLO_CUDA_EXECUTION_FAILED, "launch of %s failed: %s", what, cudaGetErrorString(launched));
     MHLO_CUDA_CHECK_LAUNCH(what);

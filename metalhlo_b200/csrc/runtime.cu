@@ -10,12 +10,12 @@
 
 namespace mhlo {
 
-bool dependent_launch_enabled() {
-    static const bool on = [] {
+bool dependent_launch_enabled(bool wanted) {
+    static const int forced = [] {
         const char* v = getenv("METALHLO_PDL");
-        return v != nullptr && v[0] == '1';
+        return v != nullptr && (v[0] == '0' || v[0] == '1') ? v[0] - '0' : -1;
     }();
-    return on;
+    return forced < 0 ? wanted : forced == 1;
 }
 
 static thread_local char g_error[1024] = "";

@@ -351,7 +351,7 @@ class Plan:
 
 
 class GemmTuning(C.Structure):
-    _fields_ = [("tile_n", C.c_int32), ("stages", C.c_int32), ("cta_group", C.c_int32), ("reserved", C.c_int32)]
+    _fields_ = [("tile_n", C.c_int32), ("stages", C.c_int32), ("cta_group", C.c_int32), ("split_k", C.c_int32)]
 
 
 def gemm(a, b, bias=None, epilogue: str = "none", out_dtype=None, trans_a: bool = False, trans_b: bool = False,

@@ -109,6 +109,14 @@ cudaError_t launch_dependent(void (*kernel)(KArgs...), dim3 grid, dim3 block, si
     return cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
 }
 
+// Stream-ordered scratch: valid for work queued on `stream` between the two calls (inside a stream capture they become
+// nodes of the graph). It comes from a memory pool of the library's own, one per device, that keeps at most kScratchKept
+// bytes between uses; those go back to the driver when an allocation of the library fails and is tried again.
+constexpr size_t kScratchKept = size_t{256} << 20;
+int scratch_alloc(void** out, size_t bytes, cudaStream_t stream);
+int scratch_free(void* p, cudaStream_t stream);
+void scratch_trim();  // current device
+
 inline bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
 
 // ---- 16-byte vectors of T <-> fp32 ------------------------------------------------------------------

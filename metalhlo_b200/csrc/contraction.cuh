@@ -51,6 +51,9 @@ struct AttnShape {
 // Tensor-core (tcgen05 + TMA + TMEM) paths; *_supported() says whether the problem meets their layout rules.
 bool gemm_tc_supported(const GemmProblem& p);
 int gemm_tc_launch(const GemmProblem& p, cudaStream_t stream);
+// 16-bit operands that have to be copied onto the 16-byte grid first.
+bool gemm_pack_supported(const GemmProblem& p);
+int gemm_pack_launch(GemmProblem p, cudaStream_t stream);
 // fp32 operands and results on the FMA units, any strides.
 bool gemm_fp32_supported(const GemmProblem& p);
 int gemm_fp32_launch(const GemmProblem& p, cudaStream_t stream);

@@ -585,10 +585,10 @@ int mhlo_cuda_reduce(const mhlo_cuda_view* in, int32_t n_kept, int32_t op, const
     if (wants_split(p.n_out, p.n_red) && plan_split(p.n_out, p.n_red, 0, &plan) && plan.splits > 1) {
         // partial accumulators live in stream-ordered scratch: allocated, used and released on `stream`
         void* scratch = nullptr;
-        MHLO_CUDA_TRY(cudaMallocAsync(&scratch, plan.scratch_bytes, s), MHLO_CUDA_BUFFER_FAILED);
+        if (const int failed = scratch_alloc(&scratch, plan.scratch_bytes, s)) return failed;
         const int st = launch_split_reduce(p, plan, scratch, s);
-        MHLO_CUDA_TRY(cudaFreeAsync(scratch, s), MHLO_CUDA_EXECUTION_FAILED);
-        return st;
+        const int freed = scratch_free(scratch, s);
+        return st != MHLO_CUDA_OK ? st : freed;
     }
 #define MHLO_RED_LAUNCH(A)                                                                                   \
     do {                                                                                                     \

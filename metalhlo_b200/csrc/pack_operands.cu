@@ -1,0 +1,117 @@
+// 16-bit products whose operands the tensor-core kernels cannot read in place: rows off the 16-byte grid (an odd pitch),
+// bases off it, or no contiguous dimension. Such an operand is copied once into a buffer whose rows are on the grid (one
+// launch for both operands, stream-ordered scratch) and the product then runs on the tensor cores. The copy reads and
+// writes the operand once, 2 (MK + KN) * 2 bytes from HBM or L2, against 2 MNK operations that otherwise ran as scalar
+// fp32 FMAs over scalar loads: [1021,1111] . [1111,3001] + bias + GELU took 509 us that way.
+#include "contraction.cuh"
+
+namespace mhlo {
+namespace {
+
+struct PackJob {
+    const uint16_t* src;
+    uint16_t* dst;
+    int64_t s_batch0, s_batch1, s_row, s_col;  // element strides of the source
+    int64_t batch1, rows, cols, pitch;         // destination: [batch0][batch1][rows][pitch]
+    int64_t all_rows;                          // batch0 * batch1 * rows
+};
+struct PackJobs {
+    PackJob job[2];
+    int64_t blocks0;  // blocks of the first job
+};
+
+// A warp per row, consecutive lanes on consecutive columns (64 bytes per load and store instruction).
+__global__ void __launch_bounds__(256) pack_operands_kernel(const __grid_constant__ PackJobs jobs) {
+    const bool second = blockIdx.x >= jobs.blocks0;
+    const PackJob& j = jobs.job[second];
+    const int64_t block = blockIdx.x - (second ? jobs.blocks0 : 0);
+    const int lane = threadIdx.x & 31;
+    const int64_t row = block * 8 + (threadIdx.x >> 5);
+    if (row >= j.all_rows) return;
+    const int64_t b = row / j.rows, r = row % j.rows;
+    const uint16_t* s = j.src + b / j.batch1 * j.s_batch0 + b % j.batch1 * j.s_batch1 + r * j.s_row;
+    uint16_t* d = j.dst + row * j.pitch;
+#pragma unroll 8
+    for (int64_t c = lane; c < j.cols; c += 32) d[c] = s[c * j.s_col];
+}
+
+bool pitch_ok(int64_t s) { return s > 0 && s % 8 == 0; }
+
+// Whether the tensor-core kernels read the operand [rows, cols] with these strides in place, in either major.
+bool readable(const void* p, const int64_t* st, int64_t batch0, int64_t batch1, int64_t rows, int64_t cols) {
+    if (!aligned16(p) || (batch0 > 1 && !pitch_ok(st[0])) || (batch1 > 1 && !pitch_ok(st[1]))) return false;
+    if (st[3] == 1 || cols == 1) return rows == 1 || pitch_ok(st[2]);
+    if (st[2] == 1 || rows == 1) return cols == 1 || pitch_ok(st[3]);
+    return false;
+}
+
+// Packs along whichever dimension is contiguous (the columns if neither is) and rewrites the operand's strides.
+void plan(PackJob* j, const void* p, int64_t* st, int64_t batch0, int64_t batch1, int64_t rows, int64_t cols) {
+    const bool along_rows = st[3] != 1 && st[2] == 1;
+    j->src = static_cast<const uint16_t*>(p);
+    j->s_batch0 = st[0]; j->s_batch1 = st[1];
+    j->s_row = along_rows ? st[3] : st[2];
+    j->s_col = along_rows ? st[2] : st[3];
+    j->batch1 = batch1;
+    j->rows = along_rows ? cols : rows;
+    j->cols = along_rows ? rows : cols;
+    j->pitch = (j->cols + 7) / 8 * 8;
+    j->all_rows = batch0 * batch1 * j->rows;
+    const int64_t matrix = j->rows * j->pitch;
+    st[0] = batch1 * matrix;
+    st[1] = matrix;
+    st[2] = along_rows ? 1 : j->pitch;
+    st[3] = along_rows ? j->pitch : 1;
+}
+
+}  // namespace
+
+bool gemm_pack_supported(const GemmProblem& p) {
+    if (p.in_dtype != MHLO_DT_F16 && p.in_dtype != MHLO_DT_BF16) return false;
+    if (p.out_dtype != p.in_dtype && p.out_dtype != MHLO_DT_F32) return false;
+    if (p.a == nullptr || p.b == nullptr || p.n_copies > 0 || p.batch0 * p.batch1 < 1) return false;
+    if (p.m > 0x7fffffff || p.n > 0x7fffffff || p.k > 0x7fffffff || p.batch0 * p.batch1 > 0x7fffffff) return false;
+    // the copy and the product's fixed cost are about 6 us: the general kernel is quicker for a few panels of one tile
+    return p.m * p.n * p.k >= 64 * 1024 && p.k > 0;
+}
+
+int gemm_pack_launch(GemmProblem p, cudaStream_t stream) {
+    PackJobs jobs;
+    memset(&jobs, 0, sizeof jobs);
+    int n = 0;
+    size_t bytes = 0, offset[2] = {0, 0};
+    const void** base[2] = {&p.a, &p.b};
+    const void** packed[2] = {nullptr, nullptr};
+    for (int i = 0; i < 2; ++i) {
+        int64_t* st = i == 0 ? p.as : p.bs;
+        const int64_t rows = i == 0 ? p.m : p.k, cols = i == 0 ? p.k : p.n;
+        if (readable(*base[i], st, p.batch0, p.batch1, rows, cols)) continue;
+        plan(&jobs.job[n], *base[i], st, p.batch0, p.batch1, rows, cols);
+        offset[n] = bytes;
+        packed[n] = base[i];
+        bytes += static_cast<size_t>(jobs.job[n].all_rows * jobs.job[n].pitch * 2 + 255) / 256 * 256;
+        ++n;
+    }
+    if (n == 0) return fail(MHLO_CUDA_EXECUTION_FAILED, "gemm: nothing to pack");
+    void* scratch = nullptr;
+    int st = scratch_alloc(&scratch, bytes, stream);
+    if (st != MHLO_CUDA_OK) return st;
+    int64_t blocks[2] = {0, 0};
+    for (int i = 0; i < n; ++i) {
+        jobs.job[i].dst = reinterpret_cast<uint16_t*>(static_cast<char*>(scratch) + offset[i]);
+        *packed[i] = jobs.job[i].dst;
+        blocks[i] = (jobs.job[i].all_rows + 7) / 8;
+    }
+    jobs.blocks0 = blocks[0];
+    if (blocks[0] + blocks[1] > 0x7fffffff) st = fail(MHLO_CUDA_UNSUPPORTED, "gemm: too many rows to pack");
+    if (st == MHLO_CUDA_OK) {
+        pack_operands_kernel<<<static_cast<unsigned>(blocks[0] + blocks[1]), 256, 0, stream>>>(jobs);
+        const cudaError_t e = cudaGetLastError();
+        if (e != cudaSuccess) st = fail(MHLO_CUDA_EXECUTION_FAILED, "launch of pack_operands failed: %s", cudaGetErrorString(e));
+    }
+    if (st == MHLO_CUDA_OK) st = gemm_tc_launch(p, stream);
+    const int freed = scratch_free(scratch, stream);
+    return st != MHLO_CUDA_OK ? st : freed;
+}
+
+}  // namespace mhlo

@@ -3,6 +3,7 @@
 // (Sources/MetalHLOCore/Runtime/IntegratedExecutor.swift:106-141,182-190,232-252).
 #include <atomic>
 #include <cstring>
+#include <mutex>
 
 #include <cstdlib>
 
@@ -29,6 +30,47 @@ int fail(int code, const char* fmt, ...) {
 }
 
 void clear_error() { g_error[0] = '\0'; }
+
+namespace {
+std::mutex g_scratch_mu;
+cudaMemPool_t g_scratch_pool[64] = {};
+
+// The current device's pool, created on first use and kept until exit; null where it cannot be had.
+cudaMemPool_t scratch_pool(bool create) {
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return nullptr;
+    std::lock_guard<std::mutex> lock(g_scratch_mu);
+    if (!g_scratch_pool[dev] && create) {
+        cudaMemPoolProps props = {};
+        props.allocType = cudaMemAllocationTypePinned;
+        props.location.type = cudaMemLocationTypeDevice;
+        props.location.id = dev;
+        cudaMemPool_t pool = nullptr;
+        if (cudaMemPoolCreate(&pool, &props) != cudaSuccess) { cudaGetLastError(); return nullptr; }
+        uint64_t kept = kScratchKept;
+        cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &kept);
+        g_scratch_pool[dev] = pool;
+    }
+    return g_scratch_pool[dev];
+}
+}  // namespace
+
+int scratch_alloc(void** out, size_t bytes, cudaStream_t stream) {
+    *out = nullptr;
+    cudaMemPool_t pool = scratch_pool(true);
+    if (pool == nullptr) return fail(MHLO_CUDA_BUFFER_FAILED, "scratch of %zu bytes: no memory pool", bytes);
+    MHLO_CUDA_TRY(cudaMallocFromPoolAsync(out, bytes, pool, stream), MHLO_CUDA_BUFFER_FAILED);
+    return MHLO_CUDA_OK;
+}
+
+int scratch_free(void* p, cudaStream_t stream) {
+    MHLO_CUDA_TRY(cudaFreeAsync(p, stream), MHLO_CUDA_EXECUTION_FAILED);
+    return MHLO_CUDA_OK;
+}
+
+void scratch_trim() {
+    if (cudaMemPool_t pool = scratch_pool(false)) cudaMemPoolTrimTo(pool, 0);
+}
 
 }  // namespace mhlo
 
@@ -182,6 +224,9 @@ int mhlo_cuda_alloc(size_t bytes, void** out_dev) {
     int left = g_refuse_allocs.load();
     while (left > 0 && !g_refuse_allocs.compare_exchange_weak(left, left - 1)) {}
     if (left > 0) return fail(MHLO_CUDA_BUFFER_FAILED, "alloc of %zu bytes refused (test hook)", bytes);
+    if (cudaMalloc(out_dev, bytes) == cudaSuccess) return MHLO_CUDA_OK;
+    cudaGetLastError();
+    mhlo::scratch_trim();  // what the scratch pool keeps goes back to the driver before the second try
     MHLO_CUDA_TRY(cudaMalloc(out_dev, bytes), MHLO_CUDA_BUFFER_FAILED);
     return MHLO_CUDA_OK;
 }

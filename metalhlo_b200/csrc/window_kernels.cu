@@ -1,6 +1,6 @@
 // Operators either side of the fused hot path that need kernels of their own: reduce_window (pooling, windowed
 // sums; a vector kernel for channel-last pooling and a general one), scatter and select_and_scatter (indexed updates
-// with atomics) and sort (bitonic networks in shared and global memory). HBM / L2-bound integer and byte work: one
+// with atomics) and sort (radix passes and bitonic networks in shared memory, network stages over global memory). HBM / L2-bound integer and byte work: one
 // thread per output element or 16-byte vector, or one CTA per sorted slice; grids sized in multiples of the SM count.
 #include <algorithm>
 #include <cstring>
@@ -678,17 +678,208 @@ __device__ __forceinline__ uint32_t load_order_key32(const void* base, int dtype
     return descending ? ~k : k;
 }
 
-__device__ __forceinline__ void bitonic_stages_packed(uint64_t* v, int count, int k, int j_first) {
+__device__ __forceinline__ void bitonic_stages_packed(uint64_t* v, int count, int64_t origin, int64_t k, int j_first) {
     for (int j = j_first; j > 0; j >>= 1) {
         for (int t = threadIdx.x; t < count / 2; t += blockDim.x) {
             const int i = 2 * t - (t & (j - 1));
             const int l = i + j;
-            const bool ascending = (i & k) == 0;
+            const bool ascending = ((origin + i) & k) == 0;
             const uint64_t a = v[i], b = v[l];
             if ((a > b) == ascending) { v[i] = b; v[l] = a; }
         }
         __syncthreads();
     }
+}
+
+// Radix sort of one slice by one CTA. The network over pairs takes log2(n) * (log2(n) + 1) / 2 stages (78 at 4096 keys), each
+// a pass over shared memory and a barrier; four stable 8-bit counting passes take 4 * 4 barriers and about 60 instructions per
+// key each, which is what bounds them: issue slots, then shared-memory conflicts of the scatter.
+//
+// Warp w holds keys [w * 32 * E, (w + 1) * 32 * E) of the tile, item e of lane l being number e * 32 + l, so (warp, item, lane)
+// is the order of the slice. A lane's rank among its warp's equal digits is what the warp's own counter of that digit held plus
+// the equal lanes below it (eight ballots, whatever the distribution of the digits); the scan over (digit, warp) adds the
+// rest. E = 16 spreads the 256 counters of a warp over 512 keys and leaves 32 warps to an SM (64 registers).
+// fp32 keys with i32 places, network -> radix: 4096 x 4096 972 -> 364 us, 2048 x 8192 1033 -> 382 us, 8192 x 1000 380 -> 196 us;
+// slices beyond shared memory, chunks by radix and packed words: 256 x 65536 3065 -> 1226 us, 1 x 20000 181 -> 83 us.
+constexpr int kRadixItems = 16;
+constexpr int kRadixDigits = 256;
+
+template <int WARPS>
+struct RadixTile {
+    static constexpr int kThreads = WARPS * 32;
+    static constexpr int kKeys = kThreads * kRadixItems;
+    uint32_t keys[kKeys];
+    uint32_t count[WARPS][kRadixDigits];
+    uint32_t warp_total[WARPS];
+    uint16_t place[kKeys];  // place of the key in the tile before the sort
+};
+
+// Lanes of the warp whose digit is this lane's.
+__device__ __forceinline__ uint32_t equal_digit_lanes(uint32_t digit) {
+    uint32_t mask = 0xffffffffu;
+#pragma unroll
+    for (int b = 0; b < 8; ++b) {
+        const bool set = (digit >> b) & 1u;
+        const uint32_t vote = __ballot_sync(0xffffffffu, set);
+        mask &= set ? vote : ~vote;
+    }
+    return mask;
+}
+
+// Sorts t.keys (visible to the CTA, filled with the largest key from n to the next multiple of 32) and leaves the places beside
+// them, visible to the CTA.
+template <int WARPS>
+__device__ __forceinline__ void radix_sort_tile(RadixTile<WARPS>& t, int n) {
+    constexpr int kThreads = RadixTile<WARPS>::kThreads;
+    constexpr int kPer = kRadixDigits > kThreads ? kRadixDigits / kThreads : 1;  // digits a thread scans
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int first = warp * 32 * kRadixItems;
+    const uint32_t below = (1u << lane) - 1;
+    uint32_t key[kRadixItems], place_rank[kRadixItems];  // place in the upper half, rank in the lower
+#pragma unroll
+    for (int e = 0; e < kRadixItems; ++e) {
+        key[e] = t.keys[first + e * 32 + lane];
+        place_rank[e] = static_cast<uint32_t>(first + e * 32 + lane) << 16;
+    }
+#pragma unroll 1
+    for (int shift = 0; shift < 32; shift += 8) {
+#pragma unroll
+        for (int d = lane; d < kRadixDigits; d += 32) t.count[warp][d] = 0;
+        __syncwarp();
+#pragma unroll
+        for (int e = 0; e < kRadixItems; ++e) {
+            if (first + e * 32 >= n) continue;  // the same for the whole warp
+            const uint32_t digit = (key[e] >> shift) & 255u;
+            const uint32_t mask = equal_digit_lanes(digit);
+            const uint32_t before = t.count[warp][digit];
+            const uint32_t rank = __popc(mask & below);
+            __syncwarp();
+            if (rank == 0) t.count[warp][digit] = before + __popc(mask);
+            __syncwarp();
+            place_rank[e] = (place_rank[e] & 0xffff0000u) | (before + rank);
+        }
+        __syncthreads();
+        // counters become first places: exclusive sums over (digit, warp)
+        uint32_t sum[kPer], own = 0;
+        const int d0 = threadIdx.x * kPer;
+        const bool scans = d0 < kRadixDigits;
+#pragma unroll
+        for (int q = 0; q < kPer; ++q) {
+            sum[q] = own;
+            if (scans) {
+#pragma unroll
+                for (int w = 0; w < WARPS; ++w) own += t.count[w][d0 + q];
+            }
+        }
+        uint32_t upto = own;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t v = __shfl_up_sync(0xffffffffu, upto, o);
+            if (lane >= o) upto += v;
+        }
+        if (lane == 31) t.warp_total[warp] = upto;
+        __syncthreads();
+        uint32_t base = upto - own;
+#pragma unroll
+        for (int w = 0; w < WARPS; ++w) base += w < warp ? t.warp_total[w] : 0u;
+        if (scans) {
+#pragma unroll
+            for (int q = 0; q < kPer; ++q) {
+                uint32_t at = base + sum[q];
+#pragma unroll
+                for (int w = 0; w < WARPS; ++w) {
+                    const uint32_t c = t.count[w][d0 + q];
+                    t.count[w][d0 + q] = at;
+                    at += c;
+                }
+            }
+        }
+        __syncthreads();
+#pragma unroll
+        for (int e = 0; e < kRadixItems; ++e) {
+            if (first + e * 32 >= n) continue;
+            const uint32_t to = t.count[warp][(key[e] >> shift) & 255u] + (place_rank[e] & 0xffffu);
+            t.keys[to] = key[e];
+            t.place[to] = static_cast<uint16_t>(place_rank[e] >> 16);
+        }
+        __syncthreads();
+        if (shift == 24) break;
+#pragma unroll
+        for (int e = 0; e < kRadixItems; ++e) {
+            const int i = first + e * 32;
+            if (i >= n) continue;
+            key[e] = t.keys[i + lane];
+            place_rank[e] = static_cast<uint32_t>(t.place[i + lane]) << 16;
+        }
+    }
+}
+
+// Can the key's bits be had back from its order? (32-bit types whose keys are all different for different bits.)
+__device__ __forceinline__ bool order_key32_inverts(int dtype, int flags) {
+    return dtype == MHLO_DT_I32 || dtype == MHLO_DT_UI32 || (dtype == MHLO_DT_F32 && (flags & 2) == 0);
+}
+
+__device__ __forceinline__ uint32_t bits_of_order_key32(uint32_t k, int dtype, int flags) {
+    if (flags & 1) k = ~k;
+    if (dtype == MHLO_DT_UI32) return k;
+    if (dtype == MHLO_DT_I32) return k ^ 0x80000000u;
+    return k ^ ((k >> 31) ? 0x80000000u : 0xffffffffu);
+}
+
+// Operands of up to four bytes are staged in the tile and permuted there: a warp's gather from global memory touches up to 32
+// lines of L1, a gather from shared memory a few conflicts.
+template <typename E, int WARPS>
+__device__ __forceinline__ void permute_staged(RadixTile<WARPS>& t, const void* in, void* out, int64_t base, int64_t inner, int n) {
+    __syncthreads();
+    E* stage = reinterpret_cast<E*>(t.keys);
+#pragma unroll 4
+    for (int i = threadIdx.x; i < n; i += WARPS * 32) stage[i] = static_cast<const E*>(in)[base + i * inner];
+    __syncthreads();
+#pragma unroll 4
+    for (int i = threadIdx.x; i < n; i += WARPS * 32) static_cast<E*>(out)[base + i * inner] = stage[t.place[i]];
+}
+
+template <int WARPS>
+__global__ void __launch_bounds__(WARPS * 32, 32 / WARPS) sort_slices_radix_kernel(const __grid_constant__ SortParams p) {
+    extern __shared__ __align__(16) unsigned char sort_smem[];
+    auto& t = *reinterpret_cast<RadixTile<WARPS>*>(sort_smem);
+    const int n = static_cast<int>(p.n);
+    const int filled = (n + 31) & ~31;
+    for (int64_t row = blockIdx.x; row < p.rows; row += gridDim.x) {
+        const int64_t base = slice_base(p, row);
+#pragma unroll 4
+        for (int i = threadIdx.x; i < filled; i += WARPS * 32)
+            t.keys[i] = i < n ? load_order_key32(p.in[0], p.key_dtype, base + i * p.inner, p.descending) : 0xffffffffu;
+        __syncthreads();
+        radix_sort_tile<WARPS>(t, n);
+        int j = 0;
+        if (order_key32_inverts(p.key_dtype, p.descending)) {
+#pragma unroll 4
+            for (int i = threadIdx.x; i < n; i += WARPS * 32)
+                static_cast<uint32_t*>(p.out[0])[base + i * p.inner] = bits_of_order_key32(t.keys[i], p.key_dtype, p.descending);
+            j = 1;
+        }
+        for (; j < p.n_operands; ++j) {
+            switch (p.elem_size[j]) {
+                case 1: permute_staged<uint8_t>(t, p.in[j], p.out[j], base, p.inner, n); break;
+                case 2: permute_staged<uint16_t>(t, p.in[j], p.out[j], base, p.inner, n); break;
+                case 4: permute_staged<uint32_t>(t, p.in[j], p.out[j], base, p.inner, n); break;
+                default:
+                    for (int i = threadIdx.x; i < n; i += WARPS * 32) move_element(p, j, base + i * p.inner, base + t.place[i] * p.inner);
+            }
+        }
+        __syncthreads();
+    }
+}
+
+template <int WARPS>
+int launch_sort_slices_radix(const SortParams& p, cudaStream_t s) {
+    const int smem = static_cast<int>(sizeof(RadixTile<WARPS>));
+    MHLO_CUDA_TRY(cudaFuncSetAttribute(sort_slices_radix_kernel<WARPS>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem), MHLO_CUDA_EXECUTION_FAILED);
+    const int64_t most = int64_t{kNumSMs} * 32;
+    sort_slices_radix_kernel<WARPS><<<static_cast<int>(p.rows < most ? p.rows : most), WARPS * 32, smem, s>>>(p);
+    MHLO_CUDA_CHECK_LAUNCH("sort (shared memory, radix)");
+    return MHLO_CUDA_OK;
 }
 
 __global__ void __launch_bounds__(kSortThreads) sort_slices_packed_kernel(const __grid_constant__ SortParams p) {
@@ -701,7 +892,7 @@ __global__ void __launch_bounds__(kSortThreads) sort_slices_packed_kernel(const 
             v[i] = i < p.n ? (static_cast<uint64_t>(load_order_key32(p.in[0], p.key_dtype, base + i * p.inner, p.descending)) << 32) | static_cast<uint32_t>(i)
                            : ~0ull;
         __syncthreads();
-        for (int k = 2; k <= padded; k <<= 1) bitonic_stages_packed(v, padded, k, k >> 1);
+        for (int k = 2; k <= padded; k <<= 1) bitonic_stages_packed(v, padded, 0, k, k >> 1);
         for (int j = 0; j < p.n_operands; ++j)
             for (int i = threadIdx.x; i < p.n; i += blockDim.x)
                 move_element(p, j, base + i * p.inner, base + static_cast<int64_t>(static_cast<uint32_t>(v[i])) * p.inner);
@@ -784,13 +975,74 @@ __global__ void __launch_bounds__(256) sort_global_stage_kernel(const __grid_con
     }
 }
 
+// The same steps for keys of at most 32 bits: packed words of 8 bytes instead of 12-byte pairs, and the chunks sorted by radix.
+// Padding takes the largest key at its own place, which is behind every real one.
+__global__ void __launch_bounds__(256) sort_init_packed_kernel(const __grid_constant__ SortParams p) {
+    const int64_t total = p.rows * p.padded;
+    const int64_t step = static_cast<int64_t>(gridDim.x) * blockDim.x;
+    for (int64_t g = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; g < total; g += step) {
+        const int64_t row = g / p.padded, i = g & (p.padded - 1);
+        const uint32_t key = i < p.n ? load_order_key32(p.in[0], p.key_dtype, slice_base(p, row) + i * p.inner, p.descending) : 0xffffffffu;
+        p.keys[g] = (static_cast<uint64_t>(key) << 32) | static_cast<uint32_t>(i);
+    }
+}
+
+constexpr int kChunkWarps = kSortChunk / (32 * kRadixItems);
+
+__global__ void __launch_bounds__(kChunkWarps * 32, 2) sort_chunks_radix_kernel(const __grid_constant__ SortParams p) {
+    extern __shared__ __align__(16) unsigned char sort_smem[];
+    auto& t = *reinterpret_cast<RadixTile<kChunkWarps>*>(sort_smem);
+    const int64_t chunks = p.rows * p.padded / kSortChunk;
+    for (int64_t c = blockIdx.x; c < chunks; c += gridDim.x) {
+        uint64_t* v = p.keys + c * kSortChunk;
+        const int64_t origin = (c * kSortChunk) & (p.padded - 1);
+#pragma unroll 4
+        for (int i = threadIdx.x; i < kSortChunk; i += kChunkWarps * 32) t.keys[i] = static_cast<uint32_t>(v[i] >> 32);
+        __syncthreads();
+        radix_sort_tile<kChunkWarps>(t, kSortChunk);
+        const bool ascending = (origin & kSortChunk) == 0;  // the next merge wants every other chunk backwards
+#pragma unroll 4
+        for (int i = threadIdx.x; i < kSortChunk; i += kChunkWarps * 32)
+            v[ascending ? i : kSortChunk - 1 - i] = (static_cast<uint64_t>(t.keys[i]) << 32) | static_cast<uint32_t>(origin + t.place[i]);
+        __syncthreads();
+    }
+}
+
+__global__ void __launch_bounds__(kSortThreads, 2) merge_chunks_packed_kernel(const __grid_constant__ SortParams p, int64_t k) {
+    extern __shared__ __align__(16) unsigned char sort_smem[];
+    uint64_t* v = reinterpret_cast<uint64_t*>(sort_smem);
+    const int64_t chunks = p.rows * p.padded / kSortChunk;
+    for (int64_t c = blockIdx.x; c < chunks; c += gridDim.x) {
+        const int64_t g0 = c * kSortChunk;
+        for (int i = threadIdx.x; i < kSortChunk; i += blockDim.x) v[i] = p.keys[g0 + i];
+        __syncthreads();
+        bitonic_stages_packed(v, kSortChunk, g0 & (p.padded - 1), k, kSortChunk >> 1);
+        for (int i = threadIdx.x; i < kSortChunk; i += blockDim.x) p.keys[g0 + i] = v[i];
+        __syncthreads();
+    }
+}
+
+__global__ void __launch_bounds__(256) sort_global_stage_packed_kernel(const __grid_constant__ SortParams p, int64_t k, int64_t j) {
+    const int64_t half = p.padded / 2, total = p.rows * half;
+    const int64_t step = static_cast<int64_t>(gridDim.x) * blockDim.x;
+    for (int64_t g = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; g < total; g += step) {
+        const int64_t t = g & (half - 1);
+        const int64_t i = 2 * t - (t & (j - 1)), l = i + j;
+        uint64_t* v = p.keys + 2 * (g - t);  // 2 * half = padded words per slice
+        const uint64_t a = v[i], b = v[l];
+        if ((a > b) == ((i & k) == 0)) { v[i] = b; v[l] = a; }
+    }
+}
+
+template <bool PACKED>
 __global__ void __launch_bounds__(256) sort_apply_kernel(const __grid_constant__ SortParams p) {
     const int64_t total = p.rows * p.n;
     const int64_t step = static_cast<int64_t>(gridDim.x) * blockDim.x;
     for (int64_t g = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; g < total; g += step) {
         const int64_t row = g / p.n, i = g % p.n;
         const int64_t base = slice_base(p, row);
-        const int64_t src = base + static_cast<int64_t>(p.order[row * p.padded + i]) * p.inner;
+        const uint32_t place = PACKED ? static_cast<uint32_t>(p.keys[row * p.padded + i]) : p.order[row * p.padded + i];
+        const int64_t src = base + static_cast<int64_t>(place) * p.inner;
         for (int j = 0; j < p.n_operands; ++j) move_element(p, j, base + i * p.inner, src);
     }
 }
@@ -1006,18 +1258,27 @@ extern "C" int mhlo_cuda_sort(const void* const* operands_dev, void* const* outs
     const size_t pair_bytes = sizeof(uint64_t) + sizeof(uint32_t);
     if (p.n <= kSortChunk) {
         const size_t smem = static_cast<size_t>(p.padded) * pair_bytes;
-        MHLO_CUDA_TRY(cudaFuncSetAttribute(sort_slices_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kSortChunk * pair_bytes)),
-                      MHLO_CUDA_EXECUTION_FAILED);
         int threads = static_cast<int>(p.padded / 2);
         threads = threads < 32 ? 32 : (threads > kSortThreads ? kSortThreads : threads);
         const int grid = static_cast<int>(p.rows < kNumSMs * 8 ? p.rows : kNumSMs * 8);
-        if (p.elem_size[0] <= 4) {  // keys of up to 32 bits: packed (key, position) words
-            MHLO_CUDA_TRY(cudaFuncSetAttribute(sort_slices_packed_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kSortChunk * sizeof(uint64_t))),
-                          MHLO_CUDA_EXECUTION_FAILED);
+        if (p.elem_size[0] <= 4) {  // keys of up to 32 bits
+            // The network while its threads (one per pair) fit the SMs at once and slices are short: it has the shorter chain
+            // (one slice of 512 keys 13 us against 30, of 4096 keys 46 against 36). Up to 128 keys the radix passes gain nothing
+            // (65536 x 100: 331 us against 339; 32768 x 200: 286 against 239).
+            const bool network = p.n <= 128 || (p.n <= 2048 && p.rows * p.padded / 2 <= kNumSMs * int64_t{2048});
+            if (!network) {
+                if (p.n <= 512) return launch_sort_slices_radix<1>(p, s);
+                if (p.n <= 1024) return launch_sort_slices_radix<2>(p, s);
+                if (p.n <= 2048) return launch_sort_slices_radix<4>(p, s);
+                if (p.n <= 4096) return launch_sort_slices_radix<8>(p, s);
+                return launch_sort_slices_radix<16>(p, s);
+            }
             sort_slices_packed_kernel<<<grid, threads, static_cast<size_t>(p.padded) * sizeof(uint64_t), s>>>(p);
             MHLO_CUDA_CHECK_LAUNCH("sort (shared memory, packed keys)");
             return MHLO_CUDA_OK;
         }
+        MHLO_CUDA_TRY(cudaFuncSetAttribute(sort_slices_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kSortChunk * pair_bytes)),
+                      MHLO_CUDA_EXECUTION_FAILED);
         sort_slices_kernel<<<grid, threads, smem, s>>>(p);
         MHLO_CUDA_CHECK_LAUNCH("sort (shared memory)");
         return MHLO_CUDA_OK;
@@ -1028,10 +1289,30 @@ extern "C" int mhlo_cuda_sort(const void* const* operands_dev, void* const* outs
                     static_cast<long long>(need), static_cast<long long>(scratch_bytes));
     p.keys = static_cast<uint64_t*>(scratch_dev);
     p.order = reinterpret_cast<uint32_t*>(p.keys + p.rows * p.padded);
-    MHLO_CUDA_TRY(cudaFuncSetAttribute(sort_chunks_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kSortChunk * pair_bytes)),
-                  MHLO_CUDA_EXECUTION_FAILED);
     const int64_t chunks = p.rows * p.padded / kSortChunk;
     const int chunk_grid = static_cast<int>(chunks < kNumSMs * 2 ? chunks : kNumSMs * 2);
+    if (p.elem_size[0] <= 4) {
+        const int radix_smem = static_cast<int>(sizeof(RadixTile<kChunkWarps>)), merge_smem = static_cast<int>(kSortChunk * sizeof(uint64_t));
+        MHLO_CUDA_TRY(cudaFuncSetAttribute(sort_chunks_radix_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, radix_smem), MHLO_CUDA_EXECUTION_FAILED);
+        MHLO_CUDA_TRY(cudaFuncSetAttribute(merge_chunks_packed_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, merge_smem), MHLO_CUDA_EXECUTION_FAILED);
+        sort_init_packed_kernel<<<grid_of(p.rows * p.padded, 256), 256, 0, s>>>(p);
+        MHLO_CUDA_CHECK_LAUNCH("sort (packed keys)");
+        sort_chunks_radix_kernel<<<chunk_grid, kChunkWarps * 32, radix_smem, s>>>(p);
+        MHLO_CUDA_CHECK_LAUNCH("sort (radix chunks)");
+        for (int64_t k = 2 * static_cast<int64_t>(kSortChunk); k <= p.padded; k <<= 1) {
+            for (int64_t j = k >> 1; j >= kSortChunk; j >>= 1) {
+                sort_global_stage_packed_kernel<<<grid_of(p.rows * p.padded / 2, 256), 256, 0, s>>>(p, k, j);
+                MHLO_CUDA_CHECK_LAUNCH("sort (global stage, packed keys)");
+            }
+            merge_chunks_packed_kernel<<<chunk_grid, kSortThreads, merge_smem, s>>>(p, k);
+            MHLO_CUDA_CHECK_LAUNCH("sort (chunk merge, packed keys)");
+        }
+        sort_apply_kernel<true><<<grid_of(p.rows * p.n, 256), 256, 0, s>>>(p);
+        MHLO_CUDA_CHECK_LAUNCH("sort (apply)");
+        return MHLO_CUDA_OK;
+    }
+    MHLO_CUDA_TRY(cudaFuncSetAttribute(sort_chunks_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kSortChunk * pair_bytes)),
+                  MHLO_CUDA_EXECUTION_FAILED);
     const size_t chunk_smem = kSortChunk * pair_bytes;
     sort_init_kernel<<<grid_of(p.rows * p.padded, 256), 256, 0, s>>>(p);
     MHLO_CUDA_CHECK_LAUNCH("sort (keys)");
@@ -1045,7 +1326,7 @@ extern "C" int mhlo_cuda_sort(const void* const* operands_dev, void* const* outs
         sort_chunks_kernel<<<chunk_grid, kSortThreads, chunk_smem, s>>>(p, k);
         MHLO_CUDA_CHECK_LAUNCH("sort (chunk merge)");
     }
-    sort_apply_kernel<<<grid_of(p.rows * p.n, 256), 256, 0, s>>>(p);
+    sort_apply_kernel<false><<<grid_of(p.rows * p.n, 256), 256, 0, s>>>(p);
     MHLO_CUDA_CHECK_LAUNCH("sort (apply)");
     return MHLO_CUDA_OK;
 }

@@ -191,6 +191,27 @@ int mhlo_cuda_add_rms_norm_rows(int dtype, const void* x_dev, const void* residu
 int mhlo_cuda_softmax(int dtype, const void* x_dev, void* y_dev, int64_t outer, int64_t axis_len,
                       int64_t inner, const mhlo_cuda_row_tuning* tuning, mhlo_cuda_stream_t stream);
 
+/*
+ * Up to MHLO_CUDA_ROW_HEADS_MAX row operations of one input x [rows, hidden], x read once: each head is a LayerNorm (op 0;
+ * gamma and beta may be null, value = eps), an RMSNorm (op 1) or a softmax over the last axis of x * value rounded to the
+ * element type (op 2; one at most, value finite and not zero, 1 = x itself). The results are those of the single entry points.
+ * No y may overlap x or another y.
+ */
+#define MHLO_CUDA_ROW_HEADS_MAX 3
+typedef struct mhlo_cuda_row_head {
+    const void* gamma;
+    const void* beta;
+    void* y;
+    float value;
+    int32_t op;
+} mhlo_cuda_row_head;
+typedef struct mhlo_cuda_row_heads {
+    mhlo_cuda_row_head head[MHLO_CUDA_ROW_HEADS_MAX];
+    int32_t count;
+} mhlo_cuda_row_heads;
+int mhlo_cuda_row_group(int dtype, const void* x_dev, const mhlo_cuda_row_heads* heads, int64_t rows, int64_t hidden,
+                        mhlo_cuda_stream_t stream);
+
 
 /* ---- generic tensor kernels (strided views) --------------------------------------------------------- */
 

@@ -13,6 +13,7 @@
 #include <cstring>
 #include <map>
 #include <numeric>
+#include <set>
 
 #include "../../../include/mhlo_cuda.h"
 #include "compiler.h"
@@ -283,10 +284,14 @@ class Lowering {
             exe_->input_types_.back().was_complex = i < f_.arg_complex.size() && f_.arg_complex[i];
         }
         open_parameter_converts();
-        for (const Op& op : f_.ops) {
-            if (op.dead) continue;
+        find_row_groups();
+        for (size_t i = 0; i < f_.ops.size(); ++i) {
+            const Op& op = f_.ops[i];
+            if (op.dead || grouped_ops_.count(i)) continue;
             if (op.name == "return") { lower_return(op); break; }
-            lower(op);
+            auto group = row_groups_.find(i);
+            if (group != row_groups_.end()) lower_row_group(group->second);
+            else lower(op);
         }
         plan();
     }
@@ -1875,7 +1880,172 @@ class Lowering {
     void lower_custom_call(const Op& op);
     void lower_return(const Op& op);
     void plan();
+
+    // ---- row operations of one input, gathered into one launch at the place of the first ------------------------------
+    struct RowGroup {
+        int x;
+        std::vector<size_t> members;  // positions in the program of the norms and the softmax
+        std::vector<float> scale;     // of a softmax member's input; 1 elsewhere
+    };
+    std::map<size_t, RowGroup> row_groups_;  // by the position of the first member
+    std::set<size_t> grouped_ops_;           // positions that a group takes the place of
+    void find_row_groups();
+    void lower_row_group(const RowGroup& group);
+    static bool splat_value(const Op& op, double* value);
+    static void count_uses(const std::vector<Op>& ops, std::vector<int>* uses);
 };
+
+// Value of a splat float constant.
+bool Lowering::splat_value(const Op& op, double* value) {
+    const Attr* a = op.attr("value");
+    if (op.name != "constant" || !a || a->kind != Attr::Dense) return false;
+    const DType dt = op.result_types[0].dtype;
+    const size_t es = dtype_size(dt);
+    if (a->dense.size() != es || (!a->splat && op.result_types[0].count() != 1)) return false;
+    if (dt == DType::F32) {
+        float v;
+        std::memcpy(&v, a->dense.data(), sizeof v);
+        *value = v;
+        return true;
+    }
+    uint16_t bits = 0;
+    if (dt != DType::F16 && dt != DType::BF16) return false;
+    std::memcpy(&bits, a->dense.data(), sizeof bits);
+    if (dt == DType::BF16) {
+        const uint32_t wide = static_cast<uint32_t>(bits) << 16;
+        float v;
+        std::memcpy(&v, &wide, sizeof v);
+        *value = v;
+        return true;
+    }
+    const int exponent = (bits >> 10) & 31, fraction = bits & 1023;
+    if (exponent == 31) return false;
+    *value = (bits >> 15 ? -1.0 : 1.0) * (exponent ? std::ldexp(1024 + fraction, exponent - 25) : std::ldexp(fraction, -24));
+    return true;
+}
+
+void Lowering::count_uses(const std::vector<Op>& ops, std::vector<int>* uses) {
+    for (const Op& op : ops) {
+        if (op.dead) continue;
+        for (int v : op.operands) ++(*uses)[static_cast<size_t>(v)];
+        for (const auto& r : op.regions) count_uses(r->ops, uses);
+    }
+}
+
+// LayerNorm, RMSNorm and softmax (of x or of x * constant) over the rows of the same x: the first one reads x for all, as long
+// as the others' gamma and beta exist there. A row kernel is bound by the bytes it moves, so two results cost 3 row passes
+// instead of 4, three 4 instead of 6 (8 with a scaled softmax input). Rows that the group kernel does not hold, and operations
+// with a tuning record of their own, stay single.
+void Lowering::find_row_groups() {
+    std::vector<int> uses(f_.values.size(), 0);
+    std::vector<int> def(f_.values.size(), -1);
+    count_uses(f_.ops, &uses);
+    for (size_t i = 0; i < f_.ops.size(); ++i)
+        if (!f_.ops[i].dead)
+            for (int r : f_.ops[i].results) def[static_cast<size_t>(r)] = static_cast<int>(i);
+    std::map<int, RowGroup> open;  // by x
+    std::map<int, std::vector<size_t>> scaled;
+    for (size_t i = 0; i < f_.ops.size(); ++i) {
+        const Op& op = f_.ops[i];
+        if (op.dead || op.name != "custom_call" || op.results.size() != 1 || op.operands.empty()) continue;
+        const std::string target = op.str_attr("call_target_name");
+        const bool ln = target == "fused_layer_norm", rms = target == "fused_rms_norm", softmax = target == "fused_softmax";
+        if (!ln && !rms && !softmax) continue;
+        const std::string cfg = op.str_attr("backend_config");
+        int x = op.operands[0];
+        const TensorType t = f_.type_of(x);
+        if (t.rank() < 1 || !batchable_float(t.dtype) || !(op.result_types[0] == t)) continue;
+        const int64_t hidden = t.shape.back(), rows = hidden ? t.count() / hidden : 0;
+        if (rows == 0 || hidden % (16 / static_cast<int64_t>(dtype_size(t.dtype))) != 0 || hidden > 16384) continue;
+        mhlo_cuda_row_tuning tuning{0, 0, 0};
+        if (lookup_row_tuning(target, rows, hidden, t.dtype, &tuning)) continue;
+        float scale = 1.f;
+        int product = -1;
+        if (softmax) {
+            const int64_t axis = static_cast<int64_t>(json_number(cfg, "axis", -1));
+            if (axis != -1 && axis != t.rank() - 1) continue;
+            const int d = def[static_cast<size_t>(x)];
+            if (d >= 0 && f_.ops[static_cast<size_t>(d)].name == "multiply" && uses[static_cast<size_t>(x)] == 1) {
+                const Op& mul = f_.ops[static_cast<size_t>(d)];
+                for (int side = 0; side < 2; ++side) {
+                    const int c = def[static_cast<size_t>(mul.operands[static_cast<size_t>(side)])];
+                    double value = 0.0;
+                    if (c < 0 || !splat_value(f_.ops[static_cast<size_t>(c)], &value) || !std::isfinite(value) || value == 0.0) continue;
+                    x = mul.operands[static_cast<size_t>(1 - side)];
+                    scale = static_cast<float>(value);
+                    product = d;
+                    break;
+                }
+                if (product >= 0 && !(f_.type_of(x) == t)) continue;
+            }
+        } else {
+            const std::vector<int64_t> axes = json_int_array(cfg, "axes");
+            if (!axes.empty() && !(axes.size() == 1 && (axes[0] == -1 || axes[0] == t.rank() - 1))) continue;
+        }
+        auto it = open.find(x);
+        bool joins = it != open.end() && it->second.members.size() < MHLO_CUDA_ROW_HEADS_MAX;
+        bool sound = true;
+        for (size_t k = 1; k < op.operands.size(); ++k) {
+            const TensorType& pt = f_.type_of(op.operands[k]);
+            sound = sound && pt.dtype == t.dtype && pt.shape == std::vector<int64_t>{hidden};
+            if (joins) joins = def[static_cast<size_t>(op.operands[k])] < static_cast<int>(it->second.members[0]);
+        }
+        if (!sound) continue;
+        if (joins && softmax)
+            for (size_t m : it->second.members) joins = joins && f_.ops[m].str_attr("call_target_name") != "fused_softmax";
+        if (joins) {
+            it->second.members.push_back(i);
+            it->second.scale.push_back(scale);
+        } else {
+            open[x] = RowGroup{x, {i}, {scale}};  // a later operation joins this one, no longer an earlier group
+            scaled[x].clear();
+        }
+        if (product >= 0) scaled[x].push_back(static_cast<size_t>(product));
+        RowGroup& g = open[x];
+        if (g.members.size() < 2) continue;
+        row_groups_[g.members[0]] = g;
+        for (size_t k = 1; k < g.members.size(); ++k) grouped_ops_.insert(g.members[k]);
+        for (size_t p : scaled[x]) grouped_ops_.insert(p);
+    }
+}
+
+void Lowering::lower_row_group(const RowGroup& group) {
+    View x = materialize(get(group.x), "row_group");
+    const int64_t hidden = x.type.shape.back(), rows = x.type.count() / hidden;
+    struct Head { DevView g, b, y; bool has_g, has_b; float value; int op; };
+    std::vector<Head> heads;
+    std::vector<View> used = {x};
+    for (size_t k = 0; k < group.members.size(); ++k) {
+        const Op& op = f_.ops[group.members[k]];
+        const std::string target = op.str_attr("call_target_name"), cfg = op.str_attr("backend_config");
+        Head h{};
+        h.op = target == "fused_layer_norm" ? 0 : target == "fused_rms_norm" ? 1 : 2;
+        h.value = h.op == 2 ? group.scale[k] : static_cast<float>(json_number(cfg, "eps", json_number(cfg, "epsilon", 1e-5)));
+        h.has_g = h.op != 2 && op.operands.size() > 1;
+        h.has_b = h.op == 0 && op.operands.size() > 2;
+        if (h.has_g) { used.push_back(materialize(get(op.operands[1]), target + ".gamma")); h.g = dev(used.back()); }
+        if (h.has_b) { used.push_back(materialize(get(op.operands[2]), target + ".beta")); h.b = dev(used.back()); }
+        used.push_back(dense_view(new_arena(op.result_types[0].bytes()), op.result_types[0]));
+        h.y = dev(used.back());
+        set(op.results[0], used.back());
+        heads.push_back(h);
+    }
+    for (const View& v : used) keep_alive(v);
+    DevView dx = dev(x);
+    const int dt = static_cast<int>(x.type.dtype);
+    detail_ = x.type.str();
+    add_step("fused_row_group(x" + std::to_string(heads.size()) + ")", [=](const Ctx& c) {
+        mhlo_cuda_row_heads list;
+        std::memset(&list, 0, sizeof list);
+        list.count = static_cast<int32_t>(heads.size());
+        for (size_t k = 0; k < heads.size(); ++k) {
+            const Head& h = heads[k];
+            list.head[k] = mhlo_cuda_row_head{h.has_g ? bind(h.g, c).base : nullptr, h.has_b ? bind(h.b, c).base : nullptr,
+                                              const_cast<void*>(bind(h.y, c).base), h.value, h.op};
+        }
+        return mhlo_cuda_row_group(dt, bind(dx, c).base, &list, rows, hidden, c.stream);
+    });
+}
 
 // ---- fused custom calls ------------------------------------------------------------------------------------------------
 

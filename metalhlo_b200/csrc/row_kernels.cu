@@ -13,6 +13,8 @@
 // Semantics follow the reference's fused custom-call handlers
 // (Sources/MetalHLOCore/Compiler/CustomCallHandlers.swift:285-394 and :644-672): LayerNorm uses the biased
 // variance of the centred row, RMSNorm adds eps to the mean square, softmax subtracts the row maximum.
+#include <cmath>
+
 #include "common.cuh"
 
 namespace mhlo {
@@ -47,6 +49,15 @@ __device__ __forceinline__ float ex2_approx(float x) {
     return y;
 }
 
+template <typename Op>
+__device__ __forceinline__ float read_partials(const float* scratch, int nwarps) {
+    if (nwarps <= 4) {
+        const float4 r = *reinterpret_cast<const float4*>(scratch);
+        return Op::apply(Op::apply(r.x, r.y), Op::apply(r.z, r.w));
+    }
+    return warp_reduce<Op>(scratch[threadIdx.x & 31]);
+}
+
 // CTA all-reduce with one barrier. `scratch` is 32 floats whose slots at and above the warp count hold the
 // identity (written once at kernel start); the caller never reuses a scratch array for two consecutive
 // reductions, which is what makes a single __syncthreads() per reduction safe.
@@ -56,11 +67,7 @@ __device__ __forceinline__ float cta_reduce1(float v, float* scratch, int nwarps
     if (nwarps == 1) return v;
     if ((threadIdx.x & 31) == 0) scratch[threadIdx.x >> 5] = v;
     __syncthreads();
-    if (nwarps <= 4) {
-        const float4 r = *reinterpret_cast<const float4*>(scratch);
-        return Op::apply(Op::apply(r.x, r.y), Op::apply(r.z, r.w));
-    }
-    return warp_reduce<Op>(scratch[threadIdx.x & 31]);
+    return read_partials<Op>(scratch, nwarps);
 }
 
 // One CTA walks rows blockIdx.x, blockIdx.x + gridDim.x, ... Each thread owns VPT 16-byte vectors of the row
@@ -288,6 +295,212 @@ row_vec_kernel(const T* __restrict__ x, const T* __restrict__ gamma, const T* __
     }
 }
 
+template <typename T, int VPT>
+constexpr int row_group_max_threads() {
+    return VPT * VecTraits<T>::kElems >= 16 ? 512 : 1024;  // values and exponentials in registers
+}
+
+// Several row operations of one input in one pass: x is read once and every result written once. HBM-bound; the separate
+// kernels read x once each, and a scaled softmax input was written and read again besides. All row statistics share the two
+// reductions (sum, sum of squares and maximum, then the centred squares and the exponentials), so a row costs two barriers
+// whatever the number of its results; gamma and beta come 16 bytes at a time from L1. A thread holds the row's share and its
+// exponentials (64 fp32 registers at most), which leaves four 128-thread CTAs to an SM and one prefetched row each: with three
+// streams leaving for one arriving, a second row in flight has nothing to hide.
+// LayerNorm, RMSNorm and softmax(4 x) of [32768, 4096] bf16: 391 us as four launches, 195 us as one (5.5 TB/s).
+// The split of a row over threads and the order of every sum are the separate kernels' (rows of 16 values a thread and more than
+// 512 threads excepted).
+template <typename T, int VPT, bool FULL>
+__global__ void __launch_bounds__((row_group_max_threads<T, VPT>()))
+row_group_kernel(const T* __restrict__ x, const __grid_constant__ mhlo_cuda_row_heads heads, int64_t rows, int hidden) {
+    using VT = VecTraits<T>;
+    constexpr int E = VT::kElems;
+    constexpr int H = E / 2;
+    __shared__ __align__(16) float red[5][32];
+    const int tid = threadIdx.x, nthreads = blockDim.x, nwarps = nthreads >> 5;
+    const int nvec = hidden / E;
+    const float inv_n = 1.0f / static_cast<float>(hidden);
+    bool wants[3] = {false, false, false};
+    float scale = 1.f;
+#pragma unroll
+    for (int h = 0; h < MHLO_CUDA_ROW_HEADS_MAX; ++h)
+        if (h < heads.count) {
+            wants[0] |= heads.head[h].op == kLayerNorm;
+            wants[1] |= heads.head[h].op == kRmsNorm;
+            if (heads.head[h].op == kSoftmax) { wants[2] = true; scale = heads.head[h].value; }
+        }
+    bool live[VPT];
+#pragma unroll
+    for (int i = 0; i < VPT; ++i) live[i] = FULL || (tid + i * nthreads < nvec);
+    grid_dependency_wait();
+    grid_dependency_release();
+    if (tid < 32) {
+#pragma unroll
+        for (int r = 0; r < 5; ++r) red[r][tid] = r == 2 ? -INFINITY : 0.f;
+    }
+    __syncthreads();
+
+    uint4 raw[VPT];
+    if (blockIdx.x < rows) {
+        const uint4* xr = reinterpret_cast<const uint4*>(x + static_cast<int64_t>(blockIdx.x) * hidden);
+#pragma unroll
+        for (int i = 0; i < VPT; ++i)
+            if (live[i]) raw[i] = ld_stream16(xr + tid + i * nthreads);
+    }
+    for (int64_t row = blockIdx.x; row < rows; row += gridDim.x) {
+        float2 v[VPT][H];
+#pragma unroll
+        for (int i = 0; i < VPT; ++i) {
+            if (live[i]) {
+                VT::unpack2(raw[i], v[i]);
+            } else {
+#pragma unroll
+                for (int h = 0; h < H; ++h) v[i][h] = splat2(0.f);
+            }
+        }
+        if (row + gridDim.x < rows) {
+            const uint4* xn = reinterpret_cast<const uint4*>(x + (row + gridDim.x) * hidden);
+#pragma unroll
+            for (int i = 0; i < VPT; ++i)
+                if (live[i]) raw[i] = ld_stream16(xn + tid + i * nthreads);
+        }
+        float2 s2 = splat2(0.f), q2 = splat2(0.f);
+        float m = -INFINITY;
+        if (wants[0]) {
+#pragma unroll
+            for (int i = 0; i < VPT; ++i)
+#pragma unroll
+                for (int h = 0; h < H; ++h) s2 = add2(s2, v[i][h]);
+        }
+        if (wants[1]) {
+#pragma unroll
+            for (int i = 0; i < VPT; ++i)
+#pragma unroll
+                for (int h = 0; h < H; ++h) q2 = fma2(v[i][h], v[i][h], q2);
+        }
+        if (wants[2]) {  // rounding keeps the order: the largest scaled value is the scaled largest (or, below zero, smallest) one
+            const float2 sign = splat2(scale < 0.f ? -1.f : 1.f);
+#pragma unroll
+            for (int i = 0; i < VPT; ++i) {
+                if (!live[i]) continue;
+#pragma unroll
+                for (int h = 0; h < H; ++h) {
+                    const float2 t = mul2(v[i][h], sign);
+                    m = fmaxf(m, fmaxf(t.x, t.y));
+                }
+            }
+        }
+        const float part0 = warp_reduce<SumOp>(s2.x + s2.y), part1 = warp_reduce<SumOp>(q2.x + q2.y), part2 = warp_reduce<MaxOp>(m);
+        float sum = part0, squares = part1;
+        m = part2;
+        if (nwarps > 1) {
+            if ((tid & 31) == 0) {
+                red[0][tid >> 5] = part0;
+                red[1][tid >> 5] = part1;
+                red[2][tid >> 5] = part2;
+            }
+            __syncthreads();
+            sum = read_partials<SumOp>(red[0], nwarps);
+            squares = read_partials<SumOp>(red[1], nwarps);
+            m = read_partials<MaxOp>(red[2], nwarps);
+        }
+        const float2 neg_mean = splat2(-(sum * inv_n));
+        float2 c2 = splat2(0.f), e2 = splat2(0.f);
+        float2 ex[VPT][H];
+        if (wants[0]) {
+#pragma unroll
+            for (int i = 0; i < VPT; ++i) {
+                if (!live[i]) continue;
+#pragma unroll
+                for (int h = 0; h < H; ++h) {
+                    const float2 d = add2(v[i][h], neg_mean);
+                    c2 = fma2(d, d, c2);
+                }
+            }
+        }
+        if (wants[2]) {
+            const float top = VT::to_float(VT::from_float(__fmul_rn(fabsf(scale), m)));  // as the element type holds the scaled value
+            const float2 sc = splat2(scale);
+            const float2 l2 = splat2(1.4426950408889634f), nb = splat2(-top * 1.4426950408889634f);
+#pragma unroll
+            for (int i = 0; i < VPT; ++i) {
+                float2 u[H];
+#pragma unroll
+                for (int h = 0; h < H; ++h) u[h] = mul2(v[i][h], sc);
+                if constexpr (sizeof(T) == 2) VT::unpack2(VT::pack2(u), u);
+#pragma unroll
+                for (int h = 0; h < H; ++h) {
+                    if constexpr (sizeof(T) == 2) {
+                        const float2 t = fma2(u[h], l2, nb);
+                        ex[i][h] = make_float2(ex2_approx(t.x), ex2_approx(t.y));
+                    } else {
+                        ex[i][h] = make_float2(expf(u[h].x - top), expf(u[h].y - top));
+                    }
+                    if (!live[i]) ex[i][h] = splat2(0.f);
+                    e2 = add2(e2, ex[i][h]);
+                }
+            }
+        }
+        float centred = warp_reduce<SumOp>(c2.x + c2.y), total = warp_reduce<SumOp>(e2.x + e2.y);
+        if (nwarps > 1) {
+            if ((tid & 31) == 0) {
+                red[3][tid >> 5] = centred;
+                red[4][tid >> 5] = total;
+            }
+            __syncthreads();
+            centred = read_partials<SumOp>(red[3], nwarps);
+            total = read_partials<SumOp>(red[4], nwarps);
+        }
+#pragma unroll
+        for (int k = 0; k < MHLO_CUDA_ROW_HEADS_MAX; ++k) {
+            if (k >= heads.count) break;
+            const int op = heads.head[k].op;
+            uint4* yr = reinterpret_cast<uint4*>(static_cast<T*>(heads.head[k].y) + row * hidden);
+            if (op == kSoftmax) {
+                const float2 inv = splat2(__frcp_rn(total));
+#pragma unroll
+                for (int i = 0; i < VPT; ++i) {
+                    if (!live[i]) continue;
+                    float2 o[H];
+#pragma unroll
+                    for (int h = 0; h < H; ++h) o[h] = mul2(ex[i][h], inv);
+                    st_stream16(yr + tid + i * nthreads, VT::pack2(o));
+                }
+                continue;
+            }
+            const bool ln = op == kLayerNorm;
+            const float2 r2 = splat2(rsqrtf((ln ? centred : squares) * inv_n + heads.head[k].value));
+            const uint4* gamma = static_cast<const uint4*>(heads.head[k].gamma);
+            const uint4* beta = static_cast<const uint4*>(heads.head[k].beta);
+#pragma unroll
+            for (int i = 0; i < VPT; ++i) {
+                if (!live[i]) continue;
+                const int idx = tid + i * nthreads;
+                float2 g[H], b[H], o[H];
+#pragma unroll
+                for (int h = 0; h < H; ++h) { g[h] = splat2(1.f); b[h] = splat2(0.f); }
+                if (gamma) VT::unpack2(__ldg(gamma + idx), g);
+                if (ln) {
+                    if (beta) VT::unpack2(__ldg(beta + idx), b);
+#pragma unroll
+                    for (int h = 0; h < H; ++h) o[h] = fma2(mul2(add2(v[i][h], neg_mean), r2), g[h], b[h]);
+                } else {
+#pragma unroll
+                    for (int h = 0; h < H; ++h) o[h] = mul2(mul2(v[i][h], r2), g[h]);
+                }
+                st_stream16(yr + idx, VT::pack2(o));
+            }
+        }
+    }
+}
+
+// out = round(x * scale): the softmax input where a group's pointers do not allow its kernel.
+template <typename T>
+__global__ void __launch_bounds__(256) scale_rows_kernel(const T* __restrict__ x, T* __restrict__ out, int64_t n, float scale) {
+    const int64_t step = static_cast<int64_t>(gridDim.x) * blockDim.x;
+    for (int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < n; i += step)
+        out[i] = VecTraits<T>::from_float(VecTraits<T>::to_float(x[i]) * scale);
+}
+
 // Any shape, any alignment: logical row r = (o, i) of a tensor viewed as [outer, len, inner]; element j of
 // that row sits at base + j*inner. One CTA per row; each pass re-reads the row (L2 serves the repeats).
 template <typename T, int OP>
@@ -346,6 +559,21 @@ __global__ void __launch_bounds__(256) add_rows_kernel(const T* __restrict__ a, 
         out[i] = static_cast<T>(static_cast<float>(a[i]) + static_cast<float>(b[i % b_period]));
 }
 
+template <int E>
+int default_vecs_per_thread(int64_t nvec) {
+    // 32 fp32 values per thread measured best on B200 (128 threads for a 4096-wide bf16 row); short rows
+    // shrink the share so that a CTA still has at least one full warp.
+    int vpt = 32 / E;
+    while (vpt > 1 && nvec < 32LL * vpt) vpt /= 2;
+    while (vpt < 8 && (nvec + vpt - 1) / vpt > (vpt * E > 32 ? 256 : (vpt * E > 16 ? 512 : 1024))) vpt *= 2;
+    // a CTA of whole warps that covers the row exactly runs without predicates: worth fewer vectors per thread
+    // (a 768-wide 16-bit row: 96 threads x 1 vector measured 35 % faster than 64 threads x 2 with a third of them idle)
+    if (nvec % (32LL * vpt) != 0)
+        for (int v = vpt / 2; v >= 1; v /= 2)
+            if (nvec % (32LL * v) == 0 && nvec / v <= (v * E > 32 ? 256 : (v * E > 16 ? 512 : 1024))) { vpt = v; break; }
+    return vpt;
+}
+
 template <typename T, int OP>
 int launch_rows(const void* x, const void* gamma, const void* beta, void* y, int64_t outer, int64_t len,
                 int64_t inner, float eps, const mhlo_cuda_row_tuning* tuning, cudaStream_t stream,
@@ -394,18 +622,7 @@ int launch_rows(const void* x, const void* gamma, const void* beta, void* y, int
         vpt = nvec > 1024 ? 2 : 1;
         threads = 0;
     }
-    if (vpt == 0) {
-        // 32 fp32 values per thread measured best on B200 (128 threads for a 4096-wide bf16 row); short rows
-        // shrink the share so that a CTA still has at least one full warp.
-        vpt = 32 / E;
-        while (vpt > 1 && nvec < 32LL * vpt) vpt /= 2;
-        while (vpt < 8 && (nvec + vpt - 1) / vpt > (vpt * E > 32 ? 256 : (vpt * E > 16 ? 512 : 1024))) vpt *= 2;
-        // a CTA of whole warps that covers the row exactly runs without predicates: worth fewer vectors per thread
-        // (a 768-wide 16-bit row: 96 threads x 1 vector measured 35 % faster than 64 threads x 2 with a third of them idle)
-        if (nvec % (32LL * vpt) != 0)
-            for (int v = vpt / 2; v >= 1; v /= 2)
-                if (nvec % (32LL * v) == 0 && nvec / v <= (v * E > 32 ? 256 : (v * E > 16 ? 512 : 1024))) { vpt = v; break; }
-    }
+    if (vpt == 0) vpt = default_vecs_per_thread<E>(nvec);
     if (vpt != 1 && vpt != 2 && vpt != 4 && vpt != 8)
         return fail(MHLO_CUDA_INVALID_ARGUMENT, "%s: vecs_per_thread must be 1, 2, 4 or 8 (got %d)", what, vpt);
     if (threads == 0) threads = static_cast<int>(((nvec + vpt - 1) / vpt + 31) / 32 * 32);
@@ -472,6 +689,56 @@ int launch_rows(const void* x, const void* gamma, const void* beta, void* y, int
                                                   rows, static_cast<int>(len), eps, static_cast<const T*>(res), static_cast<T*>(sum_out), res_rows);
     if (launched != cudaSuccess) return fail(MHLO_CUDA_EXECUTION_FAILED, "launch of %s failed: %s", what, cudaGetErrorString(launched));
     MHLO_CUDA_CHECK_LAUNCH(what);
+    return MHLO_CUDA_OK;
+}
+
+// The group kernel where it reaches (whole 16-byte vectors, at most 32 values a thread); otherwise one launch per result.
+template <typename T>
+int launch_row_group(const void* x, const mhlo_cuda_row_heads& heads, int64_t rows, int64_t hidden, cudaStream_t stream) {
+    constexpr int E = VecTraits<T>::kElems;
+    bool vec_ok = hidden % E == 0 && aligned16(x);
+    for (int k = 0; k < heads.count; ++k)
+        vec_ok = vec_ok && aligned16(heads.head[k].gamma) && aligned16(heads.head[k].beta) && aligned16(heads.head[k].y);
+    const int64_t nvec = hidden / E;
+    int vpt = vec_ok ? default_vecs_per_thread<E>(nvec) : 0;
+    if (vpt * E == 16 && nvec > 512LL * vpt) vpt *= 2;
+    if (!vec_ok || vpt * E > 32 || nvec > (vpt * E >= 16 ? 512LL : 1024LL) * vpt) {
+        for (int k = 0; k < heads.count; ++k) {
+            const mhlo_cuda_row_head& h = heads.head[k];
+            const void* from = x;
+            if (h.op == kSoftmax && h.value != 1.f) {
+                const int64_t n = rows * hidden;
+                scale_rows_kernel<T><<<static_cast<int>(n < 148LL * 2048 ? (n + 255) / 256 : 148 * 8), 256, 0, stream>>>(
+                    static_cast<const T*>(x), static_cast<T*>(h.y), n, h.value);
+                MHLO_CUDA_CHECK_LAUNCH("row_group (scale)");
+                from = h.y;  // a row is read before it is written
+            }
+            const int r = h.op == kLayerNorm ? launch_rows<T, kLayerNorm>(x, h.gamma, h.beta, h.y, rows, hidden, 1, h.value, nullptr, stream, "layer_norm")
+                          : h.op == kRmsNorm ? launch_rows<T, kRmsNorm>(x, h.gamma, nullptr, h.y, rows, hidden, 1, h.value, nullptr, stream, "rms_norm")
+                                             : launch_rows<T, kSoftmax>(from, nullptr, nullptr, h.y, rows, hidden, 1, 0.f, nullptr, stream, "softmax");
+            if (r != MHLO_CUDA_OK) return r;
+        }
+        return MHLO_CUDA_OK;
+    }
+    const int threads = static_cast<int>(((nvec + vpt - 1) / vpt + 31) / 32 * 32);
+    const bool full = static_cast<int64_t>(threads) * vpt == nvec;
+    using Kernel = void (*)(const T*, const mhlo_cuda_row_heads, int64_t, int);
+    Kernel kernel = nullptr;
+    switch (vpt) {
+        case 1: kernel = full ? row_group_kernel<T, 1, true> : row_group_kernel<T, 1, false>; break;
+        case 2: kernel = full ? row_group_kernel<T, 2, true> : row_group_kernel<T, 2, false>; break;
+        case 4: kernel = full ? row_group_kernel<T, 4, true> : row_group_kernel<T, 4, false>; break;
+        default:
+            if constexpr (8 * E <= 32) kernel = full ? row_group_kernel<T, 8, true> : row_group_kernel<T, 8, false>;
+    }
+    int per_sm = 0;
+    MHLO_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, threads, 0), MHLO_CUDA_NO_DEVICE);
+    const int64_t most = static_cast<int64_t>(kNumSMs) * (per_sm < 1 ? 1 : per_sm);
+    const int64_t grid = rows < most ? rows : most;
+    const cudaError_t launched = launch_dependent(kernel, dim3(static_cast<unsigned>(grid)), dim3(static_cast<unsigned>(threads)), 0, stream, 1,
+                                                  grid * threads <= 512 * kNumSMs, static_cast<const T*>(x), heads, rows, static_cast<int>(hidden));
+    if (launched != cudaSuccess) return fail(MHLO_CUDA_EXECUTION_FAILED, "launch of row_group failed: %s", cudaGetErrorString(launched));
+    MHLO_CUDA_CHECK_LAUNCH("row_group");
     return MHLO_CUDA_OK;
 }
 
@@ -558,6 +825,31 @@ int mhlo_cuda_softmax(int dtype, const void* x_dev, void* y_dev, int64_t outer, 
                       const mhlo_cuda_row_tuning* tuning, mhlo_cuda_stream_t stream) {
     return mhlo::dispatch_rows<mhlo::kSoftmax>(dtype, x_dev, nullptr, nullptr, y_dev, outer, axis_len, inner, 0.f,
                                                tuning, stream, "softmax");
+}
+
+int mhlo_cuda_row_group(int dtype, const void* x_dev, const mhlo_cuda_row_heads* heads, int64_t rows, int64_t hidden,
+                        mhlo_cuda_stream_t stream) {
+    using namespace mhlo;
+    if (!heads || heads->count < 1 || heads->count > MHLO_CUDA_ROW_HEADS_MAX)
+        return fail(MHLO_CUDA_INVALID_ARGUMENT, "row_group: between 1 and %d results expected", MHLO_CUDA_ROW_HEADS_MAX);
+    if (rows < 0 || hidden < 0) return fail(MHLO_CUDA_INVALID_ARGUMENT, "row_group: negative extent");
+    if (rows == 0 || hidden == 0) return MHLO_CUDA_OK;
+    if (!x_dev) return fail(MHLO_CUDA_INVALID_ARGUMENT, "row_group: null tensor pointer");
+    int softmaxes = 0;
+    for (int k = 0; k < heads->count; ++k) {
+        const mhlo_cuda_row_head& h = heads->head[k];
+        if (h.op < kLayerNorm || h.op > kSoftmax) return fail(MHLO_CUDA_INVALID_ARGUMENT, "row_group: operation %d", h.op);
+        if (!h.y || h.y == x_dev) return fail(MHLO_CUDA_INVALID_ARGUMENT, "row_group: result %d is null or the input", k);
+        if (h.op == kSoftmax && (++softmaxes > 1 || !std::isfinite(h.value) || h.value == 0.f))
+            return fail(MHLO_CUDA_INVALID_ARGUMENT, "row_group: one softmax at most, with a finite scale other than zero");
+    }
+    cudaStream_t s = static_cast<cudaStream_t>(stream);
+    switch (dtype) {
+        case MHLO_DT_F32: return launch_row_group<float>(x_dev, *heads, rows, hidden, s);
+        case MHLO_DT_F16: return launch_row_group<__half>(x_dev, *heads, rows, hidden, s);
+        case MHLO_DT_BF16: return launch_row_group<__nv_bfloat16>(x_dev, *heads, rows, hidden, s);
+        default: return fail(MHLO_CUDA_UNSUPPORTED, "row_group: dtype %d is not a float type this kernel handles", dtype);
+    }
 }
 
 }  // extern "C"

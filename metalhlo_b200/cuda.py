@@ -26,6 +26,14 @@ class RowTuning(C.Structure):
     _fields_ = [("threads", C.c_int32), ("vecs_per_thread", C.c_int32), ("ctas_per_sm", C.c_int32)]
 
 
+class RowHead(C.Structure):
+    _fields_ = [("gamma", C.c_void_p), ("beta", C.c_void_p), ("y", C.c_void_p), ("value", C.c_float), ("op", C.c_int32)]
+
+
+class RowHeads(C.Structure):
+    _fields_ = [("head", RowHead * 3), ("count", C.c_int32)]
+
+
 class View(C.Structure):
     _fields_ = [("base", C.c_void_p), ("dtype", C.c_int32), ("rank", C.c_int32), ("shape", C.c_int64 * 8),
                 ("stride", C.c_int64 * 8)]
@@ -104,6 +112,7 @@ _PROTOTYPES = {
     "mhlo_cuda_layer_norm": (C.c_int, [C.c_int, _vp, _vp, _vp, _vp, _i64, _i64, _f32, C.POINTER(RowTuning), _vp]),
     "mhlo_cuda_rms_norm": (C.c_int, [C.c_int, _vp, _vp, _vp, _i64, _i64, _f32, C.POINTER(RowTuning), _vp]),
     "mhlo_cuda_softmax": (C.c_int, [C.c_int, _vp, _vp, _i64, _i64, _i64, C.POINTER(RowTuning), _vp]),
+    "mhlo_cuda_row_group": (C.c_int, [C.c_int, _vp, C.POINTER(RowHeads), _i64, _i64, _vp]),
     "mhlo_cuda_elementwise": (C.c_int, [C.POINTER(View), _i32, C.POINTER(EwInst), _i32, _vp, _i32, C.POINTER(_i64), _i32, _vp]),
     "mhlo_cuda_elementwise_to_view": (C.c_int, [C.POINTER(View), _i32, C.POINTER(EwInst), _i32, C.POINTER(View), _vp]),
     "mhlo_cuda_reduce": (C.c_int, [C.POINTER(View), _i32, _i32, _vp, _vp, _vp, _i32, _vp]),

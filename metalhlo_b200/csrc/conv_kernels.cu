@@ -131,7 +131,8 @@ struct Im2colVecParams {
     uint32_t kernel_size[MHLO_CUDA_CONV_MAX_SPATIAL], out_size[MHLO_CUDA_CONV_MAX_SPATIAL], in_size[MHLO_CUDA_CONV_MAX_SPATIAL];
     int32_t stride[MHLO_CUDA_CONV_MAX_SPATIAL], pad_low[MHLO_CUDA_CONV_MAX_SPATIAL], lhs_dilation[MHLO_CUDA_CONV_MAX_SPATIAL],
         rhs_dilation[MHLO_CUDA_CONV_MAX_SPATIAL], reverse[MHLO_CUDA_CONV_MAX_SPATIAL];
-    int64_t in_batch_vecs, in_spatial_vecs[MHLO_CUDA_CONV_MAX_SPATIAL];  // strides in vectors
+    int64_t in_batch_vecs, in_spatial_vecs[MHLO_CUDA_CONV_MAX_SPATIAL];  // strides in vectors (in elements for im2col_narrow_kernel)
+    int64_t in_feature_stride;
 };
 
 // NS > 0: the number of spatial dimensions at compile time; DILATED = false promises lhs_dilation == 1 everywhere.
@@ -167,14 +168,79 @@ __global__ void __launch_bounds__(256) im2col_vec_kernel(const __grid_constant__
     }
 }
 
-// Fills the vector parameters; false when the layout does not allow the vector path.
-bool vec_im2col_params(const ConvParams& p, int elem_bytes, Im2colVecParams* q) {
+// Patches of images with few features per tap (RGB, odd counts) or any other input stride: one thread gathers the elements of
+// one 16-byte vector of a patch row. Bound by index arithmetic, not by the bytes: the row's place in the image is worked out
+// once per vector with multiply-high divisions, and the taps are walked. A thread per element with 64-bit divisions
+// took about 32 us for [256,32,32,3] bf16, 3 x 3, stride 2 (65536 rows of 32); this takes 9 us (ncu, cold caches), and the residual
+// CNN forward pass that it is part of 188 us instead of 211.
+template <typename E, int NS>
+__global__ void __launch_bounds__(256) im2col_narrow_kernel(const __grid_constant__ Im2colVecParams p) {
+    constexpr int V = 16 / static_cast<int>(sizeof(E));
+    constexpr int kMax = NS > 0 ? NS : MHLO_CUDA_CONV_MAX_SPATIAL;
+    const int ns = NS > 0 ? NS : p.ns;
+    const E* in = reinterpret_cast<const E*>(p.in);
+    const uint32_t step = gridDim.x * blockDim.x;
+    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < p.total_vecs; i += step) {
+        uint32_t kvec, rem, m, g, kv, ic;
+        p.by_pitch.divmod(i, &rem, &kvec);
+        p.by_rows.divmod(rem, &g, &m);
+        const uint32_t kk = kvec * V;
+        p.by_cg.divmod(kk, &kv, &ic);
+        int32_t origin[kMax];
+        uint32_t tap[kMax];
+#pragma unroll
+        for (int d = kMax - 1; d >= 0; --d) {
+            if (d >= ns) continue;
+            uint32_t od;
+            p.by_out[d].divmod(m, &m, &od);
+            p.by_kernel[d].divmod(kv, &kv, &tap[d]);
+            origin[d] = static_cast<int32_t>(od) * p.stride[d] - p.pad_low[d];
+        }
+        const E* image = in + m * p.in_batch_vecs + static_cast<int64_t>(g) * p.cg_vecs * p.in_feature_stride;
+        bool fresh = true, inside = false;
+        int64_t off = 0;
+        alignas(16) E v[V];
+#pragma unroll
+        for (int e = 0; e < V; ++e) {
+            if (fresh) {  // a tap begins: where it lies
+                off = 0;
+                inside = true;
+#pragma unroll
+                for (int d = 0; d < kMax; ++d) {
+                    if (d >= ns) continue;
+                    const uint32_t kd = p.reverse[d] ? p.kernel_size[d] - 1 - tap[d] : tap[d];
+                    const int32_t pos = origin[d] + static_cast<int32_t>(kd) * p.rhs_dilation[d];
+                    const int32_t src = p.lhs_dilation[d] == 1 ? pos : pos / p.lhs_dilation[d];
+                    inside = inside && pos >= 0 && src < static_cast<int32_t>(p.in_size[d]) && src * p.lhs_dilation[d] == pos;
+                    off += src * p.in_spatial_vecs[d];
+                }
+            }
+            v[e] = inside && kk + e < p.row_vecs ? image[off + ic * p.in_feature_stride] : E(0);
+            fresh = ++ic == p.cg_vecs;
+            if (fresh) {
+                ic = 0;
+                bool carry = true;
+#pragma unroll
+                for (int d = kMax - 1; d >= 0; --d) {
+                    if (d >= ns || !carry) continue;
+                    carry = ++tap[d] == p.kernel_size[d];
+                    if (carry) tap[d] = 0;
+                }
+            }
+        }
+        p.out[i] = *reinterpret_cast<const uint4*>(v);
+    }
+}
+
+// Fills the parameters of the two kernels above; false when the layout does not allow them. vectors: input strides in 16-byte
+// vectors, else in elements.
+bool vec_im2col_params(const ConvParams& p, int elem_bytes, bool vectors, Im2colVecParams* q) {
     const mhlo_cuda_conv& c = p.c;
-    const int64_t V = 16 / elem_bytes;
     if (elem_bytes > 16 || 16 % elem_bytes) return false;
-    if (c.in_feature_stride != 1 || p.features_per_group % V || p.row_pitch % V || c.in_batch_stride % V) return false;
-    if (!aligned16(p.in) || !aligned16(p.out)) return false;
-    const int64_t total = c.feature_group_count * p.n_rows * (p.row_pitch / V);
+    const int64_t W = 16 / elem_bytes, V = vectors ? W : 1;
+    if (vectors && (c.in_feature_stride != 1 || p.features_per_group % V || c.in_batch_stride % V || !aligned16(p.in))) return false;
+    if (p.row_pitch % W || p.row_pitch >= (int64_t{1} << 31) || !aligned16(p.out)) return false;
+    const int64_t total = c.feature_group_count * p.n_rows * (p.row_pitch / W);
     if (total >= (int64_t{1} << 31) || p.n_rows >= (int64_t{1} << 31)) return false;
     *q = Im2colVecParams{};
     for (int d = 0; d < c.n_spatial; ++d) {
@@ -194,13 +260,14 @@ bool vec_im2col_params(const ConvParams& p, int elem_bytes, Im2colVecParams* q) 
     q->in = static_cast<const uint4*>(p.in);
     q->out = static_cast<uint4*>(p.out);
     q->total_vecs = static_cast<uint32_t>(total);
-    q->pitch_vecs = static_cast<uint32_t>(p.row_pitch / V);
+    q->pitch_vecs = static_cast<uint32_t>(p.row_pitch / W);
     q->row_vecs = static_cast<uint32_t>(p.kernel_volume * p.features_per_group / V);
     q->cg_vecs = static_cast<uint32_t>(p.features_per_group / V);
     q->n_rows = static_cast<uint32_t>(p.n_rows);
     q->groups = static_cast<uint32_t>(c.feature_group_count);
     q->ns = c.n_spatial;
     q->in_batch_vecs = c.in_batch_stride / V;
+    q->in_feature_stride = c.in_feature_stride;
     q->by_pitch = FastDiv(q->pitch_vecs);
     q->by_rows = FastDiv(q->n_rows);
     q->by_cg = FastDiv(q->cg_vecs);
@@ -302,7 +369,7 @@ extern "C" int mhlo_cuda_im2col(int32_t dtype, const void* in_dev, void* cols_de
         default: break;
     }
     Im2colVecParams q;
-    if (elem_bytes && vec_im2col_params(p, elem_bytes, &q)) {
+    if (elem_bytes && vec_im2col_params(p, elem_bytes, true, &q)) {
         bool dilated = false;
         for (int d = 0; d < q.ns; ++d) dilated |= q.lhs_dilation[d] != 1;
         const int vgrid = conv_grid(q.total_vecs);
@@ -310,6 +377,16 @@ extern "C" int mhlo_cuda_im2col(int32_t dtype, const void* in_dev, void* cols_de
         else if (q.ns == 2) im2col_vec_kernel<2, false><<<vgrid, 256, 0, s>>>(q);
         else im2col_vec_kernel<0, false><<<vgrid, 256, 0, s>>>(q);
         MHLO_CUDA_CHECK_LAUNCH("im2col (vectors)");
+        return MHLO_CUDA_OK;
+    }
+    // 64-bit elements, two to a vector, and pitches off the vectors stay with the general kernel: they are rare in convolutions
+    if (dtype != MHLO_DT_I1 && elem_bytes && elem_bytes <= 4 && vec_im2col_params(p, elem_bytes, false, &q)) {
+        const int vgrid = conv_grid(q.total_vecs);
+        const bool plane = q.ns == 2;
+        if (elem_bytes == 1) plane ? im2col_narrow_kernel<uint8_t, 2><<<vgrid, 256, 0, s>>>(q) : im2col_narrow_kernel<uint8_t, 0><<<vgrid, 256, 0, s>>>(q);
+        else if (elem_bytes == 2) plane ? im2col_narrow_kernel<uint16_t, 2><<<vgrid, 256, 0, s>>>(q) : im2col_narrow_kernel<uint16_t, 0><<<vgrid, 256, 0, s>>>(q);
+        else plane ? im2col_narrow_kernel<uint32_t, 2><<<vgrid, 256, 0, s>>>(q) : im2col_narrow_kernel<uint32_t, 0><<<vgrid, 256, 0, s>>>(q);
+        MHLO_CUDA_CHECK_LAUNCH("im2col (gathered vectors)");
         return MHLO_CUDA_OK;
     }
     const int grid = conv_grid(total);

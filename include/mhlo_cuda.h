@@ -212,6 +212,13 @@ typedef struct mhlo_cuda_row_heads {
 int mhlo_cuda_row_group(int dtype, const void* x_dev, const mhlo_cuda_row_heads* heads, int64_t rows, int64_t hidden,
                         mhlo_cuda_stream_t stream);
 
+/*
+ * Batch norm at inference of x [rows, channels]: ((x - mean) / sqrt(variance + eps)) * scale + offset with the four statistics
+ * of `channels` elements, every operand of the same type (f32, f16 or bf16).
+ */
+int mhlo_cuda_batch_norm(int dtype, const void* x_dev, const void* scale_dev, const void* offset_dev, const void* mean_dev,
+                         const void* variance_dev, void* y_dev, int64_t rows, int64_t channels, float eps, mhlo_cuda_stream_t stream);
+
 
 /* ---- generic tensor kernels (strided views) --------------------------------------------------------- */
 

@@ -743,6 +743,27 @@ class Lowering {
         if (axis < 0 || axis >= rt.rank()) fail_compile("batch_norm_inference: feature_index out of range");
         const Attr* ea = op.attr("epsilon");
         const double eps = ea ? ea->as_float() : 0.0;
+        // Channels last and dense, one type throughout: the kernel that keeps a channel's statistics in registers. Other layouts
+        // (channels first, views, f64) are an elementwise program.
+        bool last = axis == rt.rank() - 1 && batchable_float(rt.dtype) && x.type.dtype == rt.dtype && x.type.shape == rt.shape && is_dense(x);
+        for (size_t i = 1; i < 5 && last; ++i) {
+            const View& s = get(op.operands[i]);
+            last = s.type.dtype == rt.dtype && s.type.shape == std::vector<int64_t>{rt.shape.back()} && is_dense(s);
+        }
+        if (last) {
+            const int64_t channels = rt.shape.back(), rows = channels ? rt.count() / channels : 0;
+            View out = dense_view(new_arena(rt.bytes()), rt);
+            std::vector<DevView> d;
+            for (int v : op.operands) { d.push_back(dev(get(v))); keep_alive(get(v)); }
+            keep_alive(out);
+            DevView dout = dev(out);
+            const int dt = static_cast<int>(rt.dtype);
+            add_step("batch_norm_inference", [=](const Ctx& c) {
+                return mhlo_cuda_batch_norm(dt, bind(d[0], c).base, bind(d[1], c).base, bind(d[2], c).base, bind(d[3], c).base, bind(d[4], c).base,
+                                            const_cast<void*>(bind(dout, c).base), rows, channels, static_cast<float>(eps), c.stream);
+            });
+            return set(op.results[0], out);
+        }
         std::vector<View> ins = {x};
         for (int i = 1; i < 5; ++i) {  // scale, offset, mean, variance: [C] viewed as [1, .., C, .., 1]
             const View& s = get(op.operands[static_cast<size_t>(i)]);

@@ -113,6 +113,7 @@ _PROTOTYPES = {
     "mhlo_cuda_rms_norm": (C.c_int, [C.c_int, _vp, _vp, _vp, _i64, _i64, _f32, C.POINTER(RowTuning), _vp]),
     "mhlo_cuda_softmax": (C.c_int, [C.c_int, _vp, _vp, _i64, _i64, _i64, C.POINTER(RowTuning), _vp]),
     "mhlo_cuda_row_group": (C.c_int, [C.c_int, _vp, C.POINTER(RowHeads), _i64, _i64, _vp]),
+    "mhlo_cuda_batch_norm": (C.c_int, [C.c_int, _vp, _vp, _vp, _vp, _vp, _vp, _i64, _i64, C.c_float, _vp]),
     "mhlo_cuda_elementwise": (C.c_int, [C.POINTER(View), _i32, C.POINTER(EwInst), _i32, _vp, _i32, C.POINTER(_i64), _i32, _vp]),
     "mhlo_cuda_elementwise_to_view": (C.c_int, [C.POINTER(View), _i32, C.POINTER(EwInst), _i32, C.POINTER(View), _vp]),
     "mhlo_cuda_reduce": (C.c_int, [C.POINTER(View), _i32, _i32, _vp, _vp, _vp, _i32, _vp]),

@@ -29,6 +29,7 @@ from __future__ import annotations
 
 import argparse
 import ctypes
+import itertools
 import json
 import os
 import statistics
@@ -350,17 +351,51 @@ def measure_norms(r: Ranks, cuda, rows_total, steps, warmup, peaks):
 class CApiHost:
     """The e2e loop's calls over the mhlo_* C API, for a build without the PJRT plugin (which is layered on the same API)."""
 
-    def __init__(self):
-        from metalhlo_b200 import capi
+    # One completion callback for the whole process, never freed: the driver's thread may still be returning through it when
+    # the event it sets lets the caller go on. `user` is the transfer's number.
+    _landed = {}
+    _numbers = itertools.count(1)
+    _done_type = ctypes.CFUNCTYPE(None, ctypes.c_void_p)
+    _done = _done_type(lambda user, landed=_landed: landed.pop(user).set())
 
+    def __init__(self, capi=None):
+        if capi is None:
+            from metalhlo_b200 import capi
         self.capi, self.client = capi, capi.Client()
-        self.done_type = ctypes.CFUNCTYPE(None, ctypes.c_void_p)
         self.to_host_async = capi.lib.mhlo_b200_buffer_to_host_async
         self.to_host_async.restype = ctypes.c_int
-        self.to_host_async.argtypes = [ctypes.c_void_p, ctypes.c_void_p, ctypes.c_size_t, self.done_type, ctypes.c_void_p]
+        self.to_host_async.argtypes = [ctypes.c_void_p, ctypes.c_void_p, ctypes.c_size_t, self._done_type, ctypes.c_void_p]
+
+    class Buffer:
+        """A device buffer of the host's client. It refers to the host and nothing refers back to it, so that dropping the last
+        reference frees the device memory there and then."""
+
+        def __init__(self, host, buffer):
+            self.host, self.buffer = host, buffer
+
+        def to_host_pointer(self, ptr, nbytes):
+            self.host.capi._check(self.host.capi.lib.mhlo_buffer_to_host(self.buffer._h, ptr, nbytes))
+
+        def to_host_pointer_start(self, ptr, nbytes):
+            """Starts the transfer; the function returned waits until it has landed."""
+            number, landed = next(CApiHost._numbers), threading.Event()
+            CApiHost._landed[number] = landed
+            try:
+                self.host.capi._check(self.host.to_host_async(self.buffer._h, ptr, nbytes, CApiHost._done, number))
+            except Exception:
+                CApiHost._landed.pop(number, None)
+                raise
+            return landed.wait
+
+    class Loaded:
+        def __init__(self, host, exe):
+            self.host, self.exe = host, exe
+
+        def execute(self, args):
+            return [CApiHost.Buffer(self.host, b) for b in self.exe.execute([a.buffer for a in args])]
 
     def buffer(self, array):
-        return self._wrap(self.client.buffer(array))
+        return CApiHost.Buffer(self, self.client.buffer(array))
 
     def buffer_from_pointer(self, ptr, dtype, shape):
         import numpy as np
@@ -370,28 +405,7 @@ class CApiHost:
         return self.buffer(view)
 
     def compile(self, text):
-        host, exe = self, self.client.compile(text, opt_level=3)
-
-        class Loaded:
-            def execute(self, args):
-                return [host._wrap(b) for b in exe.execute(args)]
-
-        return Loaded()
-
-    def _wrap(self, buffer):
-        def start(ptr, nbytes):
-            landed = threading.Event()
-            done = self.done_type(lambda _user: landed.set())
-            self.capi._check(self.to_host_async(buffer._h, ptr, nbytes, done, None))
-
-            def wait(keep=done):
-                landed.wait()
-
-            return wait
-
-        buffer.to_host_pointer_start = start
-        buffer.to_host_pointer = lambda ptr, nbytes: self.capi._check(self.capi.lib.mhlo_buffer_to_host(buffer._h, ptr, nbytes))
-        return buffer
+        return CApiHost.Loaded(self, self.client.compile(text, opt_level=3))
 
 
 def e2e_host():

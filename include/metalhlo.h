@@ -94,7 +94,8 @@ void mhlo_clear_error(void);
 size_t mhlo_element_type_size(MHLOElementType type); /* 0 for I1, as in the reference */
 void mhlo_free_string(const char* str);
 
-/* ---- client (reference: metalhlo.h:87-95) ---- */
+/* ---- client (reference: metalhlo.h:87-95) ----
+ * A client, its buffers and its executables may be destroyed in any order: what is still held stays usable. */
 MHLOStatusCode mhlo_client_create(MHLOClientRef* out_client);
 void mhlo_client_destroy(MHLOClientRef client);
 char* mhlo_client_device_name(MHLOClientRef client);

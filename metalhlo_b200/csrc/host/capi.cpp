@@ -2,6 +2,7 @@
 // Sources/CMetalHLO/CInterface.swift:202-1010: opaque retained handles, MHLOStatusCode returns, a process-global
 // last-error string that is NULL when clear, synchronous execution with new output buffers per call, and
 // per-executable execution statistics.
+#include <atomic>
 #include <chrono>
 #include <cstdlib>
 #include <cstring>
@@ -50,7 +51,25 @@ struct Client {
     // Bounded by METALHLO_BUFFER_POOL_MB (default 8192, 0 = off); everything goes back to the driver with the client.
     std::multimap<size_t, void*> pool;
     size_t pooled_bytes = 0, pool_limit = 0;
+    // The caller's handle, every buffer and every executable hold one reference each: they may be destroyed in any order
+    // (a garbage-collected host language destroys them in an order of its own).
+    std::atomic<int> references{1};
 };
+
+Client* retain(Client* c) {
+    c->references.fetch_add(1, std::memory_order_relaxed);
+    return c;
+}
+
+void release(Client* c) {
+    if (c->references.fetch_sub(1, std::memory_order_acq_rel) != 1) return;
+    mhlo_cuda_device_set(c->device);
+    for (auto& kv : c->pool) mhlo_cuda_free(kv.second);
+    if (c->copy_stream) { mhlo_cuda_stream_sync(c->copy_stream); mhlo_cuda_stream_destroy(c->copy_stream); }
+    if (c->copy_fence) mhlo_cuda_event_destroy(c->copy_fence);
+    if (c->stream) mhlo_cuda_stream_destroy(c->stream);
+    delete c;
+}
 
 size_t pool_limit_from_env() {
     const char* v = std::getenv("METALHLO_BUFFER_POOL_MB");
@@ -103,13 +122,20 @@ void pool_release(Client* c, void* dev, size_t bytes) {
 }
 
 struct ExecutableHandle {
-    Client* client;
+    explicit ExecutableHandle(Client* c) : client(retain(c)) {}
+    ~ExecutableHandle() {
+        exe.reset();
+        release(client);
+    }
+    Client* const client;
     std::shared_ptr<Executable> exe;
     ExecutionStats stats;
 };
 
 struct Buffer {
-    Client* client;
+    explicit Buffer(Client* c) : client(retain(c)) {}
+    ~Buffer() { release(client); }
+    Client* const client;
     void* dev = nullptr;
     TensorType type;
     size_t bytes = 0;
@@ -121,8 +147,7 @@ struct Buffer {
 size_t buffer_bytes(const TensorType& t) { return static_cast<size_t>(t.bytes()); }
 
 MHLOStatusCode make_buffer(Client* c, const TensorType& t, Buffer** out) {
-    std::unique_ptr<Buffer> b(new Buffer());
-    b->client = c;
+    std::unique_ptr<Buffer> b(new Buffer(c));
     b->type = t;
     b->bytes = buffer_bytes(t);
     if (mhlo_cuda_device_set(c->device) != 0) return static_cast<MHLOStatusCode>(set_error(MHLO_ERROR_NO_DEVICE, mhlo_cuda_last_error()));
@@ -254,8 +279,7 @@ MHLOStatusCode compile_impl(Client* c, const std::string& text, const MHLOCompil
         ++c->cache_misses;
         if (opt.enable_caching) c->cache[key] = exe;
     }
-    ExecutableHandle* h = new ExecutableHandle();
-    h->client = c;
+    ExecutableHandle* h = new ExecutableHandle(c);
     h->exe = exe;
     *out = h;
     return MHLO_OK;
@@ -334,13 +358,18 @@ void mhlo_client_destroy(MHLOClientRef client) {
     Client* c = static_cast<Client*>(client);
     if (!c) return;
     mhlo_cuda_device_set(c->device);
-    c->cache.clear();
-    for (auto& kv : c->pool) mhlo_cuda_free(kv.second);
-    c->pool.clear();
-    if (c->copy_stream) { mhlo_cuda_stream_sync(c->copy_stream); mhlo_cuda_stream_destroy(c->copy_stream); }
-    if (c->copy_fence) mhlo_cuda_event_destroy(c->copy_fence);
-    if (c->stream) mhlo_cuda_stream_destroy(c->stream);
-    delete c;
+    // What only the client kept goes now; buffers and executables that are still held keep the stream alive.
+    std::map<std::string, std::shared_ptr<Executable>> programs;
+    std::multimap<size_t, void*> blocks;
+    {
+        std::lock_guard<std::mutex> lock(c->mu);
+        programs.swap(c->cache);
+        blocks.swap(c->pool);
+        c->pooled_bytes = c->pool_limit = 0;
+    }
+    programs.clear();
+    for (auto& kv : blocks) mhlo_cuda_free(kv.second);
+    release(c);
 }
 
 char* mhlo_client_device_name(MHLOClientRef client) {

@@ -314,3 +314,24 @@ def test_pjrt_execute_surfaces_the_same_failure():
     with pytest.raises(pjrt.PjrtError, match="code 4"):
         exe.execute([a, a])
     np.testing.assert_array_equal(exe.execute([a, a])[0].to_numpy(), 2 * np.ones(4, np.float32))
+
+
+def test_client_buffers_and_executables_go_in_any_order(api):
+    """The client's handle first, then a run on what is still held, then executables and buffers in either order."""
+    for buffers_first in (False, True):
+        client = api.Client()
+        x = np.arange(4, dtype=np.float32)
+        big = client.buffer(np.ones(1 << 16, dtype=np.float32))  # large enough for the pool of released blocks
+        a, b = client.buffer(x), client.buffer(2 * x)
+        exe = client.compile(ADD_4)
+        again = client.compile(ADD_4)  # the same program out of the client's cache
+        api.lib.mhlo_client_destroy(client._h)
+        client._h = None
+        out, = exe.execute([a, b])
+        assert np.array_equal(out.to_numpy(), 3 * x)
+        held = [exe, again, a, b, out, big]
+        for h in reversed(held) if buffers_first else held:
+            (api.lib.mhlo_executable_destroy if isinstance(h, api.Executable) else api.lib.mhlo_buffer_destroy)(h._h)
+            h._h = None
+    client = api.Client()  # and a client made afterwards works
+    assert np.array_equal(client.run(ADD_4, [x, x])[0], 2 * x)

@@ -26,6 +26,26 @@ struct GemmProblem {
     int32_t split_k = 0;  // 1: the sum over K may be split (see mhlo_cuda_gemm_tuning)
 };
 
+// How the tensor-core kernels read a 16-bit operand [rows, cols] with element strides {batch0, batch1, row, col} in place: which
+// dimension its tensor map has as the contiguous one, kNoMajor if neither can be (TMA wants every other stride to be a positive
+// multiple of 16 bytes). A dimension of extent 1 is contiguous and on every grid, whatever its stride says. K comes first where
+// both would do. Support, packing and launch all go by this rule.
+enum OperandMajor : int32_t { kNoMajor = -1, kMajorK = 0, kMajorMN = 1 };
+inline bool tma_stride(int64_t elems) { return elems > 0 && elems % 8 == 0; }
+inline bool contiguous_along(int64_t stride, int64_t extent, int64_t other_stride, int64_t other_extent) {
+    return (stride == 1 || extent == 1) && (other_extent == 1 || tma_stride(other_stride));
+}
+inline OperandMajor a_major(const GemmProblem& p) {
+    return contiguous_along(p.as[3], p.k, p.as[2], p.m) ? kMajorK : contiguous_along(p.as[2], p.m, p.as[3], p.k) ? kMajorMN : kNoMajor;
+}
+inline OperandMajor b_major(const GemmProblem& p) {
+    return contiguous_along(p.bs[2], p.k, p.bs[3], p.n) ? kMajorK : contiguous_along(p.bs[3], p.n, p.bs[2], p.k) ? kMajorMN : kNoMajor;
+}
+// Base and batch strides of an operand on the grid.
+inline bool operand_on_grid(const GemmProblem& p, const void* base, const int64_t* st) {
+    return aligned16(base) && (p.batch0 == 1 || tma_stride(st[0])) && (p.batch1 == 1 || tma_stride(st[1]));
+}
+
 // A 2-D convolution of dense NHWC input with dense HWIO filters into dense NHWC output, stride 1, one feature group: the
 // form the tensor-core kernel reads without a patch matrix.
 struct ConvProblem {
@@ -51,9 +71,9 @@ struct AttnShape {
 // Tensor-core (tcgen05 + TMA + TMEM) paths; *_supported() says whether the problem meets their layout rules.
 bool gemm_tc_supported(const GemmProblem& p);
 int gemm_tc_launch(const GemmProblem& p, cudaStream_t stream);
-// 16-bit operands that have to be copied onto the 16-byte grid first.
-bool gemm_pack_supported(const GemmProblem& p);
-int gemm_pack_launch(GemmProblem p, cudaStream_t stream);
+// 16-bit operands that have to be copied onto the 16-byte grid first. False: not a product this applies to, nothing was queued and
+// the general kernel takes it; true: *status is the result of the launches.
+bool gemm_pack_launch(GemmProblem p, cudaStream_t stream, int* status);
 // fp32 operands and results on the FMA units, any strides.
 bool gemm_fp32_supported(const GemmProblem& p);
 int gemm_fp32_launch(const GemmProblem& p, cudaStream_t stream);

@@ -191,8 +191,9 @@ int mhlo_cuda_gemm_tuned(int32_t in_dtype, int32_t out_dtype, const void* a_dev,
     if (tuning) { p.tile_n = tuning->tile_n; p.stages = tuning->stages; p.cta_group = tuning->cta_group; p.split_k = tuning->split_k; }
     if (gemm_tc_supported(p)) return gemm_tc_launch(p, static_cast<cudaStream_t>(stream));
     if (gemm_fp32_supported(p)) return gemm_fp32_launch(p, static_cast<cudaStream_t>(stream));
-    if (gemm_pack_supported(p)) return gemm_pack_launch(p, static_cast<cudaStream_t>(stream));
-    int st = mhlo_cuda_dot_strided(in_dtype, out_dtype, a_dev, a_strides, b_dev, b_strides, c_dev, batch0, batch1, m, n, k, stream);
+    int st = MHLO_CUDA_OK;
+    if (gemm_pack_launch(p, static_cast<cudaStream_t>(stream), &st)) return st;
+    st = mhlo_cuda_dot_strided(in_dtype, out_dtype, a_dev, a_strides, b_dev, b_strides, c_dev, batch0, batch1, m, n, k, stream);
     if (st != MHLO_CUDA_OK || (bias_dev == nullptr && epilogue == MHLO_EPILOGUE_NONE)) return st;
     // bias / activation as an in-place elementwise pass over C
     mhlo_cuda_view in[2];

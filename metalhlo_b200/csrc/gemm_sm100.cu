@@ -653,8 +653,6 @@ bool operand_map(CUtensorMap* map, const void* base, int64_t inner, int64_t oute
     return encode_map(map, base, dims, strides, box, why);
 }
 
-bool stride_ok(int64_t elems) { return elems > 0 && (elems * 2) % 16 == 0; }
-
 // C [batch0, batch1, m, n] with row pitch ldc as a 4-D map {n, m, batch1, batch0}; one box = 128 bytes x 32 rows, the
 // staging tile of one epilogue warp.
 bool output_map(CUtensorMap* map, void* base, int out_dtype, int64_t n, int64_t m, int64_t ldc, int64_t b1, int64_t b0, std::string* why) {
@@ -694,17 +692,7 @@ bool gemm_tc_supported(const GemmProblem& p) {
     if (p.out_dtype != p.in_dtype && p.out_dtype != MHLO_DT_F32) return false;
     if (p.m <= 0 || p.n <= 0 || p.k <= 0 || p.batch0 <= 0 || p.batch1 <= 0) return false;
     if (p.m * p.n * p.k < 32 * 1024) return false;  // a few panels of the general kernel take less than the fixed cost
-    if (!aligned16(p.a) || !aligned16(p.b)) return false;
-    // one of (row, col) strides must be 1; the other, and the batch strides, 16-byte multiples
-    const bool a_k = p.as[3] == 1 || p.k == 1, a_m = p.as[2] == 1 || p.m == 1;
-    const bool b_n = p.bs[3] == 1 || p.n == 1, b_k = p.bs[2] == 1 || p.k == 1;
-    if (!(a_k || a_m) || !(b_n || b_k)) return false;
-    auto batch_ok = [&](const int64_t* s) {
-        return (p.batch0 == 1 || stride_ok(s[0])) && (p.batch1 == 1 || stride_ok(s[1]));
-    };
-    if (!batch_ok(p.as) || !batch_ok(p.bs)) return false;
-    if (a_k ? !(p.m == 1 || stride_ok(p.as[2])) : !(p.k == 1 || stride_ok(p.as[3]))) return false;
-    if (b_k ? !(p.n == 1 || stride_ok(p.bs[3])) : !(p.k == 1 || stride_ok(p.bs[2]))) return false;
+    if (!operand_on_grid(p, p.a, p.as) || !operand_on_grid(p, p.b, p.bs) || a_major(p) == kNoMajor || b_major(p) == kNoMajor) return false;
     if (p.batch0 * p.batch1 > 0x7fffffffLL || p.m > 0x7fffffffLL || p.n > 0x7fffffffLL || p.k > 0x7fffffffLL) return false;
     return true;
 }
@@ -713,8 +701,8 @@ template <int BN, int STAGES, int ACT, int CTAS, int MODE = 0>
 static int launch_gemm_act(const GemmProblem& pr, cudaStream_t stream) {
     constexpr bool PEER = MODE == 1;
     using L = SmemLayout<BN, STAGES, CTAS>;
-    const bool a_k = pr.as[3] == 1 || pr.k == 1;
-    const bool b_k = pr.bs[2] == 1 || pr.k == 1;  // K-major B = [n][k] with k contiguous
+    const bool a_k = a_major(pr) == kMajorK;
+    const bool b_k = b_major(pr) == kMajorK;  // B = [n][k] with k contiguous
     CUtensorMap map_a, map_b;
     std::string why;
     bool ok;
@@ -840,7 +828,7 @@ static int launch_gemm(const GemmProblem& p, cudaStream_t stream) {
 template <int BN>
 static int launch_cluster(const GemmProblem& pr, int splits, cudaStream_t stream) {
     using L = ClusterLayout<BN>;
-    const bool a_k = pr.as[3] == 1 || pr.k == 1, b_k = pr.bs[2] == 1 || pr.k == 1;
+    const bool a_k = a_major(pr) == kMajorK, b_k = b_major(pr) == kMajorK;
     CUtensorMap map_a, map_b;
     std::string why;
     bool ok;

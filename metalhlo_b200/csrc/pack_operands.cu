@@ -35,16 +35,6 @@ __global__ void __launch_bounds__(256) pack_operands_kernel(const __grid_constan
     for (int64_t c = lane; c < j.cols; c += 32) d[c] = s[c * j.s_col];
 }
 
-bool pitch_ok(int64_t s) { return s > 0 && s % 8 == 0; }
-
-// Whether the tensor-core kernels read the operand [rows, cols] with these strides in place, in either major.
-bool readable(const void* p, const int64_t* st, int64_t batch0, int64_t batch1, int64_t rows, int64_t cols) {
-    if (!aligned16(p) || (batch0 > 1 && !pitch_ok(st[0])) || (batch1 > 1 && !pitch_ok(st[1]))) return false;
-    if (st[3] == 1 || cols == 1) return rows == 1 || pitch_ok(st[2]);
-    if (st[2] == 1 || rows == 1) return cols == 1 || pitch_ok(st[3]);
-    return false;
-}
-
 // Packs along whichever dimension is contiguous (the columns if neither is) and rewrites the operand's strides.
 void plan(PackJob* j, const void* p, int64_t* st, int64_t batch0, int64_t batch1, int64_t rows, int64_t cols) {
     const bool along_rows = st[3] != 1 && st[2] == 1;
@@ -66,52 +56,48 @@ void plan(PackJob* j, const void* p, int64_t* st, int64_t batch0, int64_t batch1
 
 }  // namespace
 
-bool gemm_pack_supported(const GemmProblem& p) {
+bool gemm_pack_launch(GemmProblem p, cudaStream_t stream, int* status) {
     if (p.in_dtype != MHLO_DT_F16 && p.in_dtype != MHLO_DT_BF16) return false;
-    if (p.out_dtype != p.in_dtype && p.out_dtype != MHLO_DT_F32) return false;
-    if (p.a == nullptr || p.b == nullptr || p.n_copies > 0 || p.batch0 * p.batch1 < 1) return false;
+    if (p.a == nullptr || p.b == nullptr || p.n_copies > 0 || p.m <= 0 || p.n <= 0 || p.k <= 0 || p.batch0 <= 0 || p.batch1 <= 0) return false;
     if (p.m > 0x7fffffff || p.n > 0x7fffffff || p.k > 0x7fffffff || p.batch0 * p.batch1 > 0x7fffffff) return false;
     // the copy and the product's fixed cost are about 6 us: the general kernel is quicker for a few panels of one tile
-    return p.m * p.n * p.k >= 64 * 1024 && p.k > 0;
-}
-
-int gemm_pack_launch(GemmProblem p, cudaStream_t stream) {
+    if (p.m * p.n * p.k < 64 * 1024) return false;
     PackJobs jobs;
     memset(&jobs, 0, sizeof jobs);
     int n = 0;
     size_t bytes = 0, offset[2] = {0, 0};
-    const void** base[2] = {&p.a, &p.b};
     const void** packed[2] = {nullptr, nullptr};
-    for (int i = 0; i < 2; ++i) {
-        int64_t* st = i == 0 ? p.as : p.bs;
-        const int64_t rows = i == 0 ? p.m : p.k, cols = i == 0 ? p.k : p.n;
-        if (readable(*base[i], st, p.batch0, p.batch1, rows, cols)) continue;
-        plan(&jobs.job[n], *base[i], st, p.batch0, p.batch1, rows, cols);
+    for (const bool is_a : {true, false}) {
+        const void** base = is_a ? &p.a : &p.b;
+        int64_t* st = is_a ? p.as : p.bs;
+        if (operand_on_grid(p, *base, st) && (is_a ? a_major(p) : b_major(p)) != kNoMajor) continue;
+        plan(&jobs.job[n], *base, st, p.batch0, p.batch1, is_a ? p.m : p.k, is_a ? p.k : p.n);
         offset[n] = bytes;
-        packed[n] = base[i];
+        packed[n] = base;
+        *base = nullptr;  // on the grid; its address comes with the scratch
         bytes += static_cast<size_t>(jobs.job[n].all_rows * jobs.job[n].pitch * 2 + 255) / 256 * 256;
         ++n;
     }
-    if (n == 0) return fail(MHLO_CUDA_EXECUTION_FAILED, "gemm: nothing to pack");
+    const int64_t blocks[2] = {(jobs.job[0].all_rows + 7) / 8, (jobs.job[1].all_rows + 7) / 8};
+    if (n == 0 || !gemm_tc_supported(p) || blocks[0] + blocks[1] > 0x7fffffff) return false;
     void* scratch = nullptr;
     int st = scratch_alloc(&scratch, bytes, stream);
-    if (st != MHLO_CUDA_OK) return st;
-    int64_t blocks[2] = {0, 0};
+    if (st != MHLO_CUDA_OK) {
+        *status = st;
+        return true;
+    }
     for (int i = 0; i < n; ++i) {
         jobs.job[i].dst = reinterpret_cast<uint16_t*>(static_cast<char*>(scratch) + offset[i]);
         *packed[i] = jobs.job[i].dst;
-        blocks[i] = (jobs.job[i].all_rows + 7) / 8;
     }
     jobs.blocks0 = blocks[0];
-    if (blocks[0] + blocks[1] > 0x7fffffff) st = fail(MHLO_CUDA_UNSUPPORTED, "gemm: too many rows to pack");
-    if (st == MHLO_CUDA_OK) {
-        pack_operands_kernel<<<static_cast<unsigned>(blocks[0] + blocks[1]), 256, 0, stream>>>(jobs);
-        const cudaError_t e = cudaGetLastError();
-        if (e != cudaSuccess) st = fail(MHLO_CUDA_EXECUTION_FAILED, "launch of pack_operands failed: %s", cudaGetErrorString(e));
-    }
+    pack_operands_kernel<<<static_cast<unsigned>(blocks[0] + blocks[1]), 256, 0, stream>>>(jobs);
+    const cudaError_t e = cudaGetLastError();
+    if (e != cudaSuccess) st = fail(MHLO_CUDA_EXECUTION_FAILED, "launch of pack_operands failed: %s", cudaGetErrorString(e));
     if (st == MHLO_CUDA_OK) st = gemm_tc_launch(p, stream);
     const int freed = scratch_free(scratch, stream);
-    return st != MHLO_CUDA_OK ? st : freed;
+    *status = st != MHLO_CUDA_OK ? st : freed;
+    return true;
 }
 
 }  // namespace mhlo

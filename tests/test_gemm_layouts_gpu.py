@@ -1,0 +1,97 @@
+"""16-bit products by the layout of their operands: extents of 1, rows on and off the 16-byte grid, strides in either order."""
+import math
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+DT = {"f16": torch.float16, "bf16": torch.bfloat16}
+UNIT = {torch.float16: 2.0 ** -11, torch.bfloat16: 2.0 ** -8, torch.float32: 2.0 ** -24}
+
+
+def close(got, want, k, magnitude):
+    """One rounding of the result and the fp32 sum's error: k additions of at most `magnitude` (the sum of the absolute products)."""
+    assert got.shape == want.shape
+    bound = UNIT[got.dtype] * want.abs() + k * 2.0 ** -24 * magnitude + 2.0 ** -24
+    worst = ((got.double() - want).abs() / bound).max().item()
+    assert worst <= 1.0, worst
+
+
+def product(a, b, dt):
+    return a.double() @ b.double(), a.double().abs() @ b.double().abs()
+
+
+# above and below 32 768 and 65 536 multiplications, where the dispatch changes
+@pytest.mark.parametrize("dt", ["f16", "bf16"])
+@pytest.mark.parametrize("m,n,k", [(512, 512, 1), (4096, 77, 1), (100, 1000, 1), (1, 4096, 64), (1, 1001, 129), (4096, 1, 64), (1001, 1, 129), (1, 1, 70000),
+                                   (1, 65544, 1), (65543, 1, 1), (2, 3, 11000), (33, 31, 63), (64, 64, 8)])
+@pytest.mark.parametrize("trans_a,trans_b", [(False, False), (True, False), (False, True), (True, True)])
+def test_extents_of_one(m, n, k, trans_a, trans_b, dt):
+    from metalhlo_b200 import cuda
+
+    g = torch.Generator().manual_seed(m + n + k)
+    a, b = torch.randn(m, k, generator=g).to(DT[dt]).cuda(), (torch.randn(k, n, generator=g) / math.sqrt(k)).to(DT[dt]).cuda()
+    got = cuda.gemm(a.t().contiguous() if trans_a else a, b.t().contiguous() if trans_b else b, trans_a=trans_a, trans_b=trans_b)
+    close(got, *product(a, b, dt)[:1], k, product(a, b, dt)[1])
+
+
+@pytest.mark.parametrize("m,n,k", [(512, 512, 1), (300, 1001, 1), (1, 4096, 33), (2049, 1, 65)])
+@pytest.mark.parametrize("ca,cb", [(1, 0), (0, 0), (1, 1), (0, 1)])
+def test_extents_of_one_in_a_program(m, n, k, ca, cb):
+    from metalhlo_b200 import capi
+    from metalhlo_b200.modules import func, tt
+
+    g = torch.Generator().manual_seed(7 * m + n)
+    a, b = torch.randn(m, k, generator=g).half(), (torch.randn(k, n, generator=g) / math.sqrt(k)).half()
+    sa, sb = ((m, k) if ca else (k, m)), ((n, k) if cb else (k, n))
+    text = func([tt(sa, "f16"), tt(sb, "f16")], [tt((m, n), "f16")],
+                f"    %0 = stablehlo.dot_general %arg0, %arg1, contracting_dims = [{ca}] x [{cb}] : ({tt(sa, 'f16')}, {tt(sb, 'f16')}) -> {tt((m, n), 'f16')}", "%0")
+    got = torch.from_numpy(capi.Client().run(text, [(a if ca else a.t()).contiguous(), (b.t() if cb else b).contiguous()], opt_level=3)[0])
+    close(got, *product(a, b, "f16")[:1], k, product(a, b, "f16")[1])
+
+
+def strided(x, order, pitch, offset=0):
+    """x [rows, cols] in a larger buffer: `order` "row" or "col" major with that pitch, or every second element ("both")."""
+    rows, cols = x.shape
+    if order == "both":
+        buf = torch.zeros(offset + 2 * rows * pitch, dtype=x.dtype, device="cuda")
+        view = buf[offset:].as_strided((rows, cols), (2 * pitch, 2))
+    else:
+        buf = torch.zeros(offset + (rows if order == "row" else cols) * pitch, dtype=x.dtype, device="cuda")
+        view = buf[offset:].as_strided((rows, cols), (pitch, 1) if order == "row" else (1, pitch))
+    view.copy_(x)
+    return view
+
+
+def raw_gemm(a, b, dtype, b0=1, b1=1, a_batch=(0, 0), b_batch=(0, 0), bias=None, epilogue="none", tuning=None, out_dtype=None):
+    """mhlo_cuda_gemm_tuned on views: a [m, k], b [k, n]."""
+    import ctypes as C
+
+    from metalhlo_b200 import cuda
+
+    (m, k), n = a.shape[-2:], b.shape[-1]
+    out = torch.full((b0, b1, m, n), float("nan"), dtype=out_dtype or dtype, device="cuda")
+    t = cuda.GemmTuning(*tuning) if tuning else None
+    code = cuda.torch_dtype_code
+    cuda.check(cuda.lib.mhlo_cuda_gemm_tuned(code(dtype), code(out.dtype), a.data_ptr(), cuda._i64s([*a_batch, *a.stride()[-2:]]), b.data_ptr(),
+                                             cuda._i64s([*b_batch, *b.stride()[-2:]]), out.data_ptr(), b0, b1, m, n, k,
+                                             None if bias is None else bias.data_ptr(), cuda.EPILOGUES[epilogue], C.byref(t) if t else None,
+                                             torch.cuda.current_stream().cuda_stream))
+    torch.cuda.synchronize()
+    return out
+
+
+# rows that start on the grid, rows that do not, a base that does not, the other order, no contiguous dimension; K of 1 on the grid
+@pytest.mark.parametrize("m,n,k", [(300, 257, 65), (512, 512, 1), (1, 3000, 40), (3000, 1, 40)])
+@pytest.mark.parametrize("la", [("row", 0, 0), ("row", 1, 0), ("row", 0, 1), ("col", 0, 0), ("col", 3, 0), ("both", 0, 0)])
+@pytest.mark.parametrize("lb", [("row", 0, 0), ("row", 1, 0), ("col", 0, 0), ("col", 5, 2), ("both", 0, 0)])
+def test_views(m, n, k, la, lb):
+    g = torch.Generator().manual_seed(m)
+    a, b = torch.randn(m, k, generator=g).half().cuda(), (torch.randn(k, n, generator=g) / math.sqrt(k)).half().cuda()
+    views = []
+    for x, (order, extra, offset) in ((a, la), (b, lb)):
+        inner = x.shape[0] if order == "col" else x.shape[1]
+        views.append(strided(x, order, (inner + 7) // 8 * 8 + extra, offset))
+    want, magnitude = product(a, b, "f16")
+    close(raw_gemm(*views, torch.float16)[0, 0], want, k, magnitude)

@@ -231,7 +231,7 @@ attention_fp32_kernel(const __grid_constant__ Fp32Attention p) {
 #pragma unroll
             for (int e = 0; e < 4 * C; ++e) {
                 const float x = sf[r * 4 * C + e];
-                const float pr = x == -INFINITY || mn == -INFINITY ? 0.f : __expf(x - mn);
+                const float pr = x == -INFINITY ? 0.f : __expf(x - mn);  // a maximum of -inf leaves -inf and NaN: NaN stays NaN
                 sf[r * 4 * C + e] = pr;
                 sum += pr;
             }

@@ -53,7 +53,7 @@ __global__ void __launch_bounds__(128) attention_rows_kernel(const T* __restrict
         for (int x = 16; x > 0; x >>= 1) cm = fmaxf(cm, __shfl_xor_sync(0xffffffffu, cm, x));
         const float mn = fmaxf(m, cm);
         const float corr = (m == -INFINITY) ? 0.f : __expf(m - mn);
-        const float p = (sc == -INFINITY || mn == -INFINITY) ? 0.f : __expf(sc - mn);
+        const float p = sc == -INFINITY ? 0.f : __expf(sc - mn);  // a maximum of -inf leaves -inf and NaN: NaN stays NaN
         float ps = p;
 #pragma unroll
         for (int x = 16; x > 0; x >>= 1) ps += __shfl_xor_sync(0xffffffffu, ps, x);

@@ -74,3 +74,24 @@ def test_attention_fp32_mask_and_interleaved_heads(d):
     p = torch.nan_to_num(torch.softmax(s, -1), nan=0.0)
     assert np.all(got[:, :, 3] == 0)
     assert_close(got, (p @ vt.double()).numpy(), 1e-5, "masked", magnitude=(p @ vt.double().abs()).numpy())
+
+
+# the fp32 kernel with and without its keys shared by a cluster, one and two warps per row group; f16 rows of 33 take the general kernel
+@pytest.mark.parametrize("causal", [False, True])
+@pytest.mark.parametrize("dt,b,h,sq,sk,d", [(torch.float32, 1, 1, 300, 1030, 64), (torch.float32, 2, 40, 130, 96, 40), (torch.float32, 3, 50, 129, 257, 64),
+                                            (torch.float32, 1, 3, 31, 33, 128), (torch.float32, 3, 50, 128, 129, 128), (torch.float16, 1, 2, 50, 70, 33)])
+def test_attention_hands_nans_on(causal, dt, b, h, sq, sk, d):
+    g = torch.Generator().manual_seed(sq + d)
+    q, k, v = (torch.randn(b, h, s, d, generator=g).to(dt) for s in (sq, sk, sk))
+    scale = 1 / math.sqrt(d)
+    clean = cuda_mod().attention(q.cuda(), k.cuda(), v.cuda(), scale, causal=causal).cpu()
+    bad = q.clone()
+    bad[0, 0, 7, 0] = math.nan  # every score of one row
+    got = cuda_mod().attention(bad.cuda(), k.cuda(), v.cuda(), scale, causal=causal).cpu()
+    assert bool(torch.isnan(got[0, 0, 7]).all())
+    got[0, 0, 7] = clean[0, 0, 7]
+    assert torch.equal(got, clean)
+    bad = k.clone()
+    bad[0, 0, :64] = math.nan  # every key of the first blocks: all rows see key 0
+    got = cuda_mod().attention(q.cuda(), bad.cuda(), v.cuda(), scale, causal=causal).cpu()
+    assert bool(torch.isnan(got[0, 0]).all()) and torch.equal(got.flatten(0, 1)[1:], clean.flatten(0, 1)[1:])

@@ -779,9 +779,11 @@ static int elementwise_impl(const mhlo_cuda_view* inputs, int32_t n_inputs, cons
     p.bool_mode = all_bool;
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     // one instruction whose operands are the inputs in order (how single operators are built; an operand a unary operator
-    // does not read may name any of them)
+    // does not read may name any of them). With two inputs the kernel hands the first one to the third operand.
     const mhlo_cuda_ew_inst& first = insts[0];
-    const bool in_order = n_inputs == 0 || (first.a == 0 && (n_inputs < 2 || first.b == 1) && (n_inputs < 3 || first.c == 2));
+    const bool reads_c = first.op == MHLO_EW_SELECT || first.op == MHLO_EW_CLAMP;
+    const bool in_order = n_inputs == 0 || (first.a == 0 && (n_inputs < 2 || first.b == 1) && (n_inputs < 3 || first.c == 2) &&
+                                            (n_inputs != 2 || !reads_c || first.c == 0));
     if (n_insts == 1 && n_inputs <= 3 && in_order) {
         p.prog[0].op = static_cast<int16_t>(first.op);
         p.prog[0].imm = first.imm;

@@ -1,0 +1,56 @@
+"""mhlo_cuda_elementwise called directly: operands that name one register several times."""
+import ctypes as C
+import itertools
+import os
+import re
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+
+
+def opcodes():
+    with open(os.path.join(ROOT, "include", "mhlo_cuda.h")) as f:
+        body = re.search(r"MHLO_EW_COPY = 0.*?MHLO_EW_OP_COUNT", f.read(), re.S).group(0)
+    names = re.findall(r"MHLO_EW_\w+", re.sub(r"/\*.*?\*/", "", body, flags=re.S))
+    return {n[len("MHLO_EW_"):]: i for i, n in enumerate(names)}
+
+
+OP = opcodes()
+
+
+def run(inputs, prog, out):
+    from metalhlo_b200 import cuda
+
+    views = (cuda.View * max(len(inputs), 1))()
+    for v, t in zip(views, inputs):
+        v.base, v.dtype, v.rank = t.data_ptr(), cuda.torch_dtype_code(t.dtype), t.dim()
+        for d in range(t.dim()):
+            v.shape[d], v.stride[d] = t.shape[d], t.stride(d)
+    insts = (cuda.EwInst * len(prog))(*[cuda.EwInst(op, a, b, c, imm) for op, a, b, c, imm in prog])
+    cuda.check(cuda.lib.mhlo_cuda_elementwise(views, len(inputs), insts, len(prog), out.data_ptr(), cuda.torch_dtype_code(out.dtype),
+                                              cuda._i64s(out.shape), out.dim(), torch.cuda.current_stream().cuda_stream))
+
+
+def test_opcodes_are_read_from_the_header():
+    assert (OP["COPY"], OP["IMM"], OP["ADD"]) == (0, 1, 3) and OP["CLAMP"] == OP["SELECT"] + 1
+
+
+# every assignment of one to three inputs to the three operands, one instruction and the same behind another
+@pytest.mark.parametrize("dt", [torch.float32, torch.bfloat16, torch.float64, torch.int32, torch.int64])
+@pytest.mark.parametrize("n_inputs", [1, 2, 3])
+def test_operands_may_share_registers(n_inputs, dt):
+    g = torch.Generator().manual_seed(n_inputs)
+    x = [torch.randint(-2, 3, (37,), generator=g).to(dt).cuda() for _ in range(n_inputs)]
+    out = torch.empty_like(x[0])
+    for a, b, c in itertools.product(range(n_inputs), repeat=3):
+        want = {"SELECT": torch.where(x[a] != 0, x[b], x[c]), "CLAMP": torch.minimum(torch.maximum(x[b], x[a]), x[c]),
+                "SUB": x[a] - x[b], "NEG": -x[a]}
+        for name, w in want.items():
+            run(x, [(OP[name], a, b, c, 0.0)], out)
+            assert torch.equal(out, w), (name, a, b, c)
+            run(x, [(OP["NEG"], 0, 0, 0, 0.0), (OP[name], a, b, c, 0.0)], out)
+            assert torch.equal(out, w), (name, a, b, c, "second instruction")

@@ -43,7 +43,11 @@ __device__ int g_gemm_error = 0;
 
 template <int ACT>
 __device__ __forceinline__ float epilogue_act(float v) {
-    if constexpr (ACT == MHLO_EPILOGUE_RELU) return fmaxf(v, 0.f);
+    if constexpr (ACT == MHLO_EPILOGUE_RELU) {
+        float r;
+        asm("max.NaN.f32 %0, %1, 0f00000000;" : "=f"(r) : "f"(v));  // stablehlo.maximum hands a NaN on
+        return r;
+    }
     if constexpr (ACT == MHLO_EPILOGUE_GELU_TANH) {
         const float inner = 0.7978845608028654f * v * fmaf(0.044715f * v, v, 1.0f);
         float t;

@@ -95,3 +95,19 @@ def test_views(m, n, k, la, lb):
         views.append(strided(x, order, (inner + 7) // 8 * 8 + extra, offset))
     want, magnitude = product(a, b, "f16")
     close(raw_gemm(*views, torch.float16)[0, 0], want, k, magnitude)
+
+
+# packed; few results, read in place; K of 1; few results with K split over a cluster
+ODD = [(65, 67, 69, 0), (300, 1001, 77, 0), (16, 128, 256, 0), (512, 512, 1, 0), (33, 96, 4096, 1), (129, 70, 515, 1)]
+
+
+@pytest.mark.parametrize("m,n,k,split", ODD + [(512, 512, 64, 0), (512, 512, 512, 1)])
+@pytest.mark.parametrize("out_dtype", [torch.float16, torch.float32])
+def test_relu_hands_a_nan_on(m, n, k, split, out_dtype):
+    g = torch.Generator().manual_seed(m)
+    a, b = torch.randn(m, k, generator=g).half().cuda(), torch.randn(k, n, generator=g).half().cuda()
+    a[m // 2, 0] = math.nan
+    got = raw_gemm(a, b, torch.float16, epilogue="relu", tuning=(0, 0, 0, split), out_dtype=out_dtype)[0, 0]
+    bad = torch.isnan(got)
+    assert bool(bad[m // 2].all()) and int(bad.sum()) == n
+    assert float(got[~bad].min()) == 0.0

@@ -24,6 +24,7 @@ struct GemmProblem {
     // of the TMA ring; cta_group: 1 = one CTA per 128-row tile, 2 = a pair of CTAs per 256-row tile.
     int32_t tile_n = 0, stages = 0, cta_group = 0;
     int32_t split_k = 0;  // 1: the sum over K may be split (see mhlo_cuda_gemm_tuning)
+    int32_t exact_act = 0;  // 1: the activation in fp32 with the CUDA library's functions, as the elementwise programs have it
 };
 
 // How the tensor-core kernels read a 16-bit operand [rows, cols] with element strides {batch0, batch1, row, col} in place: which

@@ -170,6 +170,13 @@ int mhlo_cuda_gemm(int32_t in_dtype, int32_t out_dtype, const void* a_dev, const
                                 nullptr, stream);
 }
 
+namespace {
+// Whether the tensor-core epilogue takes the CUDA library's tanhf and expf rather than the hardware's approximations (2^-11
+// relative). The approximations are for products whose epilogue has to keep up with the MMAs: at least 64 x 64 results, K
+// above 1, operands read in place. Everything else (and every packed product) is bound elsewhere and keeps fp32 precision.
+bool exact_activation(const GemmProblem& p) { return p.m * p.n < 64 * 64 || p.k == 1; }
+}  // namespace
+
 int mhlo_cuda_gemm_tuned(int32_t in_dtype, int32_t out_dtype, const void* a_dev, const int64_t a_strides[4],
                          const void* b_dev, const int64_t b_strides[4], void* c_dev, int64_t batch0, int64_t batch1,
                          int64_t m, int64_t n, int64_t k, const void* bias_dev, int32_t epilogue,
@@ -189,6 +196,7 @@ int mhlo_cuda_gemm_tuned(int32_t in_dtype, int32_t out_dtype, const void* a_dev,
     p.batch0 = batch0; p.batch1 = batch1; p.m = m; p.n = n; p.k = k;
     p.in_dtype = in_dtype; p.out_dtype = out_dtype; p.epilogue = epilogue;
     if (tuning) { p.tile_n = tuning->tile_n; p.stages = tuning->stages; p.cta_group = tuning->cta_group; p.split_k = tuning->split_k; }
+    p.exact_act = exact_activation(p);
     if (gemm_tc_supported(p)) return gemm_tc_launch(p, static_cast<cudaStream_t>(stream));
     if (gemm_fp32_supported(p)) return gemm_fp32_launch(p, static_cast<cudaStream_t>(stream));
     int st = MHLO_CUDA_OK;

@@ -26,14 +26,21 @@ __device__ __forceinline__ float4 ld_cluster_f4(uint32_t addr) {
     return v;
 }
 
+// `epilogue` with or without kExactAct; four results a thread, so that a switch per result costs nothing beside the exchange.
 __device__ __forceinline__ float cluster_act(float v, int epilogue) {
     switch (epilogue) {
-        case MHLO_EPILOGUE_RELU: return epilogue_act<MHLO_EPILOGUE_RELU>(v);
         case MHLO_EPILOGUE_GELU_TANH: return epilogue_act<MHLO_EPILOGUE_GELU_TANH>(v);
-        case MHLO_EPILOGUE_GELU_ERF: return epilogue_act<MHLO_EPILOGUE_GELU_ERF>(v);
         case MHLO_EPILOGUE_SILU: return epilogue_act<MHLO_EPILOGUE_SILU>(v);
-        case MHLO_EPILOGUE_TANH: return epilogue_act<MHLO_EPILOGUE_TANH>(v);
         case MHLO_EPILOGUE_SIGMOID: return epilogue_act<MHLO_EPILOGUE_SIGMOID>(v);
+        default: break;
+    }
+    switch (epilogue & ~kExactAct) {
+        case MHLO_EPILOGUE_RELU: return epilogue_act<MHLO_EPILOGUE_RELU>(v);
+        case MHLO_EPILOGUE_GELU_TANH: return epilogue_act<MHLO_EPILOGUE_GELU_TANH | kExactAct>(v);
+        case MHLO_EPILOGUE_GELU_ERF: return epilogue_act<MHLO_EPILOGUE_GELU_ERF>(v);
+        case MHLO_EPILOGUE_SILU: return epilogue_act<MHLO_EPILOGUE_SILU | kExactAct>(v);
+        case MHLO_EPILOGUE_TANH: return epilogue_act<MHLO_EPILOGUE_TANH>(v);
+        case MHLO_EPILOGUE_SIGMOID: return epilogue_act<MHLO_EPILOGUE_SIGMOID | kExactAct>(v);
         default: return v;
     }
 }

@@ -41,9 +41,13 @@ constexpr int kGemmThreads = 32 * (2 + kEpilogueWarps);
 
 __device__ int g_gemm_error = 0;
 
+// ACT: an MHLO_EPILOGUE_* code; with kExactAct added, GELU, SiLU and sigmoid take the CUDA library's functions instead of the
+// hardware's approximations (see exact_activation in contraction_dispatch.cu).
+constexpr int kExactAct = 16;
+
 template <int ACT>
 __device__ __forceinline__ float epilogue_act(float v) {
-    if constexpr (ACT == MHLO_EPILOGUE_RELU) {
+    if constexpr ((ACT & ~kExactAct) == MHLO_EPILOGUE_RELU) {
         float r;
         asm("max.NaN.f32 %0, %1, 0f00000000;" : "=f"(r) : "f"(v));  // stablehlo.maximum hands a NaN on
         return r;
@@ -51,14 +55,17 @@ __device__ __forceinline__ float epilogue_act(float v) {
     if constexpr (ACT == MHLO_EPILOGUE_GELU_TANH) {
         const float inner = 0.7978845608028654f * v * fmaf(0.044715f * v, v, 1.0f);
         float t;
-        asm("tanh.approx.f32 %0, %1;" : "=f"(t) : "f"(inner));  // 2^-11 relative error: below the 16-bit output resolution
+        asm("tanh.approx.f32 %0, %1;" : "=f"(t) : "f"(inner));  // 2^-11 relative error: the resolution of f16, coarser than fp32's
         const float hv = 0.5f * v;
         return fmaf(hv, t, hv);
     }
-    if constexpr (ACT == MHLO_EPILOGUE_GELU_ERF) return 0.5f * v * (1.0f + erff(v * 0.70710678118654752440f));
+    if constexpr (ACT == (MHLO_EPILOGUE_GELU_TANH | kExactAct)) return 0.5f * v * (1.0f + tanhf(0.7978845608028654f * (v + 0.044715f * v * v * v)));
+    if constexpr ((ACT & ~kExactAct) == MHLO_EPILOGUE_GELU_ERF) return 0.5f * v * (1.0f + erff(v * 0.70710678118654752440f));
     if constexpr (ACT == MHLO_EPILOGUE_SILU) return v / (1.0f + __expf(-v));
-    if constexpr (ACT == MHLO_EPILOGUE_TANH) return tanhf(v);
+    if constexpr (ACT == (MHLO_EPILOGUE_SILU | kExactAct)) return v / (1.0f + expf(-v));
+    if constexpr ((ACT & ~kExactAct) == MHLO_EPILOGUE_TANH) return tanhf(v);
     if constexpr (ACT == MHLO_EPILOGUE_SIGMOID) return 1.0f / (1.0f + __expf(-v));
+    if constexpr (ACT == (MHLO_EPILOGUE_SIGMOID | kExactAct)) return 1.0f / (1.0f + expf(-v));
     return v;
 }
 
@@ -816,6 +823,13 @@ static int launch_gemm(const GemmProblem& p, cudaStream_t stream) {
             return fail(MHLO_CUDA_UNSUPPORTED, "gemm: a residual goes with a 16-bit result, no activation and no further copies of C");
         return launch_gemm_act<BN, STAGES, MHLO_EPILOGUE_NONE, CTAS, 2>(p, stream);
     }
+    if (p.exact_act)
+        switch (p.epilogue) {
+            case MHLO_EPILOGUE_GELU_TANH: return launch_gemm_act<BN, STAGES, MHLO_EPILOGUE_GELU_TANH | kExactAct, CTAS>(p, stream);
+            case MHLO_EPILOGUE_SILU: return launch_gemm_act<BN, STAGES, MHLO_EPILOGUE_SILU | kExactAct, CTAS>(p, stream);
+            case MHLO_EPILOGUE_SIGMOID: return launch_gemm_act<BN, STAGES, MHLO_EPILOGUE_SIGMOID | kExactAct, CTAS>(p, stream);
+            default: break;  // the others are exact anyway
+        }
     switch (p.epilogue) {
         case MHLO_EPILOGUE_RELU: return launch_gemm_act<BN, STAGES, MHLO_EPILOGUE_RELU, CTAS>(p, stream);
         case MHLO_EPILOGUE_GELU_TANH: return launch_gemm_act<BN, STAGES, MHLO_EPILOGUE_GELU_TANH, CTAS>(p, stream);
@@ -855,7 +869,7 @@ static int launch_cluster(const GemmProblem& pr, int splits, cudaStream_t stream
     p.b_mn_major = b_k ? 0 : 1;
     p.in_bf16 = pr.in_dtype == MHLO_DT_BF16;
     p.out_dtype = pr.out_dtype;
-    p.epilogue = pr.epilogue;
+    p.epilogue = pr.epilogue | (pr.exact_act ? kExactAct : 0);
     const uintptr_t grid = pr.out_dtype == MHLO_DT_F32 ? 16 : 8;  // four results per store
     p.c_vec_ok = pr.n % 4 == 0 && reinterpret_cast<uintptr_t>(pr.c) % grid == 0;
     static std::atomic<bool> attr_set[64];

@@ -79,6 +79,7 @@ bool gemm_pack_launch(GemmProblem p, cudaStream_t stream, int* status) {
         ++n;
     }
     const int64_t blocks[2] = {(jobs.job[0].all_rows + 7) / 8, (jobs.job[1].all_rows + 7) / 8};
+    p.exact_act = 1;
     if (n == 0 || !gemm_tc_supported(p) || blocks[0] + blocks[1] > 0x7fffffff) return false;
     void* scratch = nullptr;
     int st = scratch_alloc(&scratch, bytes, stream);

@@ -111,3 +111,23 @@ def test_relu_hands_a_nan_on(m, n, k, split, out_dtype):
     bad = torch.isnan(got)
     assert bool(bad[m // 2].all()) and int(bad.sum()) == n
     assert float(got[~bad].min()) == 0.0
+
+
+ACT = {"gelu_tanh": lambda x: torch.nn.functional.gelu(x, approximate="tanh"), "gelu_erf": torch.nn.functional.gelu,
+       "silu": torch.nn.functional.silu, "tanh": torch.tanh, "sigmoid": torch.sigmoid, "relu": torch.relu}
+
+
+@pytest.mark.parametrize("m,n,k,split", ODD)
+@pytest.mark.parametrize("epilogue", sorted(ACT))
+@pytest.mark.parametrize("dt,out_dtype", [("f16", torch.float16), ("bf16", torch.bfloat16), ("bf16", torch.float32)])
+def test_activations_in_fp32(m, n, k, split, epilogue, dt, out_dtype):
+    g = torch.Generator().manual_seed(m + k)
+    a, b = torch.randn(m, k, generator=g).to(DT[dt]).cuda(), (torch.randn(k, n, generator=g) * 1.5 / math.sqrt(k)).to(DT[dt]).cuda()
+    bias = torch.randn(n, generator=g).to(out_dtype).cuda()
+    got = raw_gemm(a, b, DT[dt], bias=bias, epilogue=epilogue, tuning=(0, 0, 0, split), out_dtype=out_dtype)[0, 0]
+    want, magnitude = product(a, b, dt)
+    x, u = want + bias.double(), 2.0 ** -24
+    # one rounding of the result; the sum's error through a slope of at most 1.13; a handful of fp32 operations on values up to |x| + 1
+    bound = UNIT[out_dtype] * ACT[epilogue](x).abs() + 1.13 * (k + 2) * u * (magnitude + bias.double().abs()) + 12 * u * (x.abs() + 1)
+    worst = ((got.double() - ACT[epilogue](x)).abs() / bound).max().item()
+    assert worst <= 1.0, worst

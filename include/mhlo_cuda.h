@@ -195,7 +195,7 @@ int mhlo_cuda_softmax(int dtype, const void* x_dev, void* y_dev, int64_t outer, 
  * Up to MHLO_CUDA_ROW_HEADS_MAX row operations of one input x [rows, hidden], x read once: each head is a LayerNorm (op 0;
  * gamma and beta may be null, value = eps), an RMSNorm (op 1) or a softmax over the last axis of x * value rounded to the
  * element type (op 2; one at most, value finite and not zero, 1 = x itself). The results are those of the single entry points.
- * No y may overlap x or another y.
+ * One y may be x itself (in place); apart from that no y may overlap x or another y.
  */
 #define MHLO_CUDA_ROW_HEADS_MAX 3
 typedef struct mhlo_cuda_row_head {

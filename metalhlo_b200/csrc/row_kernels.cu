@@ -692,7 +692,8 @@ int launch_rows(const void* x, const void* gamma, const void* beta, void* y, int
     return MHLO_CUDA_OK;
 }
 
-// The group kernel where it reaches (whole 16-byte vectors, at most 32 values a thread); otherwise one launch per result.
+// The group kernel where it reaches (whole 16-byte vectors, at most 32 values a thread); otherwise one launch per result. One
+// result may take x's place: a CTA has a row in registers before it writes any result of that row, and no other CTA reads it.
 template <typename T>
 int launch_row_group(const void* x, const mhlo_cuda_row_heads& heads, int64_t rows, int64_t hidden, cudaStream_t stream) {
     constexpr int E = VecTraits<T>::kElems;
@@ -703,8 +704,12 @@ int launch_row_group(const void* x, const mhlo_cuda_row_heads& heads, int64_t ro
     int vpt = vec_ok ? default_vecs_per_thread<E>(nvec) : 0;
     if (vpt * E == 16 && nvec > 512LL * vpt) vpt *= 2;
     if (!vec_ok || vpt * E > 32 || nvec > (vpt * E >= 16 ? 512LL : 1024LL) * vpt) {
+        int order[MHLO_CUDA_ROW_HEADS_MAX] = {}, n_order = 0;  // a result in place of x comes last
+        for (const bool in_place : {false, true})
+            for (int k = 0; k < heads.count; ++k)
+                if ((heads.head[k].y == x) == in_place) order[n_order++] = k;
         for (int k = 0; k < heads.count; ++k) {
-            const mhlo_cuda_row_head& h = heads.head[k];
+            const mhlo_cuda_row_head& h = heads.head[order[k]];
             const void* from = x;
             if (h.op == kSoftmax && h.value != 1.f) {
                 const int64_t n = rows * hidden;
@@ -892,7 +897,7 @@ int mhlo_cuda_row_group(int dtype, const void* x_dev, const mhlo_cuda_row_heads*
     for (int k = 0; k < heads->count; ++k) {
         const mhlo_cuda_row_head& h = heads->head[k];
         if (h.op < kLayerNorm || h.op > kSoftmax) return fail(MHLO_CUDA_INVALID_ARGUMENT, "row_group: operation %d", h.op);
-        if (!h.y || h.y == x_dev) return fail(MHLO_CUDA_INVALID_ARGUMENT, "row_group: result %d is null or the input", k);
+        if (!h.y) return fail(MHLO_CUDA_INVALID_ARGUMENT, "row_group: result %d is null", k);
         if (h.op == kSoftmax && (++softmaxes > 1 || !std::isfinite(h.value) || h.value == 0.f))
             return fail(MHLO_CUDA_INVALID_ARGUMENT, "row_group: one softmax at most, with a finite scale other than zero");
     }

@@ -128,3 +128,19 @@ def test_group_in_a_program(rows, hidden, dt):
     tol = 2e-2 if dt == "bf16" else 1e-5
     for got, want in zip(outs, (oracle.layer_norm(x, gamma, beta), oracle.rms_norm(x, gamma), oracle.softmax(x * 4))):
         assert_close(got, want, tol, f"group {dt}")
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("rows,hidden,offset", [(300, 1024, 0), (3, 40, 0), (2000, 4096, 0), (6, 512, 1), (5, 101, 0)])
+@pytest.mark.parametrize("place", [0, 1, 2])
+def test_one_result_may_take_the_place_of_x(rows, hidden, offset, place):
+    g = torch.Generator().manual_seed(hidden + place)
+    flat = torch.randn(rows * hidden + offset, generator=g).to(torch.bfloat16).cuda()
+    x = flat[offset:].view(rows, hidden)
+    gamma = (torch.randn(hidden, generator=g) * 0.1 + 1).to(torch.bfloat16).cuda()
+    heads = [(0, gamma, gamma, 1e-5), (1, gamma, None, 1e-6), (2, None, None, 3.0)]
+    want = row_group(x.clone() if not offset else flat.clone()[offset:].view(rows, hidden), heads)
+    outs = [torch.empty_like(flat)[offset:].view(rows, hidden) for _ in heads]
+    outs[place] = x
+    for got, w in zip(row_group_into(x, heads, outs), want):
+        assert same_bits(got, w)

@@ -1956,7 +1956,9 @@ void Lowering::count_uses(const std::vector<Op>& ops, std::vector<int>* uses) {
 // LayerNorm, RMSNorm and softmax (of x or of x * constant) over the rows of the same x: the first one reads x for all, as long
 // as the others' gamma and beta exist there. A row kernel is bound by the bytes it moves, so two results cost 3 row passes
 // instead of 4, three 4 instead of 6 (8 with a scaled softmax input). Rows that the group kernel does not hold, and operations
-// with a tuning record of their own, stay single.
+// with a tuning record of their own, stay single. A result that the program returns is written into the caller's memory, which
+// may be an argument's: such an operation joins only if nothing but the group itself stands between it and the first, so that
+// no step reads that argument after it has been overwritten.
 void Lowering::find_row_groups() {
     std::vector<int> uses(f_.values.size(), 0);
     std::vector<int> def(f_.values.size(), -1);
@@ -1964,8 +1966,26 @@ void Lowering::find_row_groups() {
     for (size_t i = 0; i < f_.ops.size(); ++i)
         if (!f_.ops[i].dead)
             for (int r : f_.ops[i].results) def[static_cast<size_t>(r)] = static_cast<int>(i);
+    std::vector<bool> returned(f_.values.size(), false);  // the value, or a view of it, leaves the program
+    for (size_t i = f_.ops.size(); i-- > 0;) {
+        const Op& op = f_.ops[i];
+        static const std::set<std::string> views = {"reshape", "transpose", "broadcast_in_dim", "slice", "reverse", "bitcast_convert"};
+        if (op.dead) continue;
+        if (op.name == "return") for (int v : op.operands) returned[static_cast<size_t>(v)] = true;
+        else if (views.count(op.name) && returned[static_cast<size_t>(op.results[0])]) returned[static_cast<size_t>(op.operands[0])] = true;
+    }
     std::map<int, RowGroup> open;  // by x
     std::map<int, std::vector<size_t>> scaled;
+    auto adjacent = [&](int x, const RowGroup& g, size_t i, int product) {
+        for (size_t j = g.members[0] + 1; j < i; ++j) {
+            const Op& op = f_.ops[j];
+            const std::vector<size_t>& products = scaled[x];
+            if (!op.dead && op.name != "constant" && static_cast<int>(j) != product && !std::count(g.members.begin(), g.members.end(), j) &&
+                !std::count(products.begin(), products.end(), j))
+                return false;
+        }
+        return true;
+    };
     for (size_t i = 0; i < f_.ops.size(); ++i) {
         const Op& op = f_.ops[i];
         if (op.dead || op.name != "custom_call" || op.results.size() != 1 || op.operands.empty()) continue;
@@ -2012,6 +2032,7 @@ void Lowering::find_row_groups() {
             if (joins) joins = def[static_cast<size_t>(op.operands[k])] < static_cast<int>(it->second.members[0]);
         }
         if (!sound) continue;
+        if (joins && returned[static_cast<size_t>(op.results[0])]) joins = adjacent(x, it->second, i, product);
         if (joins && softmax)
             for (size_t m : it->second.members) joins = joins && f_.ops[m].str_attr("call_target_name") != "fused_softmax";
         if (joins) {

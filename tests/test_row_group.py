@@ -144,3 +144,37 @@ def test_one_result_may_take_the_place_of_x(rows, hidden, offset, place):
     outs[place] = x
     for got, w in zip(row_group_into(x, heads, outs), want):
         assert same_bits(got, w)
+
+
+def program_with_a_step_between(hidden, dt, returned):
+    """LayerNorm(x), LayerNorm(x) + w, RMSNorm(x): the RMSNorm returned, or only read by a sum."""
+    t, tv = tt((4, hidden), dt), tt((hidden,), dt)
+    body, ln = layer_norm_text("%arg0", (4, hidden), dt, "%arg1", "%arg1", prefix="a")
+    body += f"    %w2 = stablehlo.add {ln}, %arg2 : {t}\n"
+    text, rms = layer_norm_text("%arg0", (4, hidden), dt, "%arg1", None, rms=True, prefix="b")
+    body += text
+    if not returned:
+        body, rms = body + f"    %last = stablehlo.add {rms}, {rms} : {t}\n", "%last"
+    return modules.func([t, tv, t], [t] * 2, body.rstrip("\n"), f"%w2, {rms}")
+
+
+def test_a_returned_result_does_not_move_across_other_steps():
+    steps = capi.plan_text(program_with_a_step_between(64, "f32", True), 3)[0]
+    assert "fused_layer_norm" in steps and "fused_rms_norm" in steps
+    assert "fused_row_group(x2)" in capi.plan_text(program_with_a_step_between(64, "f32", False), 3)[0]
+
+
+@pytest.mark.gpu
+def test_a_result_bound_to_an_argument_that_a_step_between_reads():
+    exe = capi.Client().compile(program_with_a_step_between(64, "f32", True), opt_level=3)
+    g = torch.Generator().manual_seed(3)
+    x, gamma, w = (torch.randn(4, 64, generator=g).cuda(), torch.randn(64, generator=g).cuda(), torch.randn(4, 64, generator=g).cuda())
+    torch.cuda.synchronize()
+    plain, bound = [torch.empty_like(x) for _ in range(2)], [torch.empty_like(x)]
+    stream = torch.cuda.current_stream().cuda_stream
+    exe.execute_on_device([t.data_ptr() for t in (x, gamma, w)], [t.data_ptr() for t in plain], stream)
+    mine = w.clone()
+    exe.execute_on_device([t.data_ptr() for t in (x, gamma, mine)], [t.data_ptr() for t in bound + [mine]], stream)
+    torch.cuda.synchronize()
+    for got, want in zip(bound + [mine], plain):
+        assert torch.equal(got, want)

@@ -100,8 +100,9 @@ __device__ __forceinline__ void load_rows(uint32_t dst, const float* base, int64
 }
 
 // acc[8][2C] += a . b for one step: 8 values of the left operand (two groups of four rows) against C groups of four columns.
-template <int C>
-__device__ __forceinline__ void step(float2 (*acc)[2 * C], const float* a, const float* b, int b_apart) {
+// MASKED: only the rows whose place in the warp's rows (less the thread's first) is at least `first` take part.
+template <int C, bool MASKED = false>
+__device__ __forceinline__ void step(float2 (*acc)[2 * C], const float* a, const float* b, int b_apart, int first = 0) {
     const float4 a0 = *reinterpret_cast<const float4*>(a), a1 = *reinterpret_cast<const float4*>(a + 16);
     const float av[8] = {a0.x, a0.y, a0.z, a0.w, a1.x, a1.y, a1.z, a1.w};
 #pragma unroll
@@ -110,6 +111,7 @@ __device__ __forceinline__ void step(float2 (*acc)[2 * C], const float* a, const
         const float2 lo = make_float2(x.x, x.y), hi = make_float2(x.z, x.w);
 #pragma unroll
         for (int r = 0; r < 8; ++r) {
+            if (MASKED && r / 4 * 16 + r % 4 < first) continue;
             const float2 d = make_float2(av[r], av[r]);
             acc[r][2 * c] = __ffma2_rn(d, lo, acc[r][2 * c]);
             acc[r][2 * c + 1] = __ffma2_rn(d, hi, acc[r][2 * c + 1]);
@@ -248,8 +250,17 @@ attention_fp32_kernel(const __grid_constant__ Fp32Attention p) {
         }
         cp_wait<1>();  // V of this block; the next K may still be on its way
         __syncthreads();
+        // keys of this block that some of the warp's rows do not see: those rows leave the key's V alone, which need not be finite
+        const int behind = j * kKeys - (q0 + group * 32);  // key - row of the block's first key and the warp's first row
+        if (!p.causal || behind + kKeys - 1 <= 0) {
 #pragma unroll 8
-        for (int key = 0; key < kKeys; ++key) step<2>(out, pw + key * T::kPPitch + ty * 4, vb + key * T::kVPitch, 32);
+            for (int key = 0; key < kKeys; ++key) step<2>(out, pw + key * T::kPPitch + ty * 4, vb + key * T::kVPitch, 32);
+        } else {
+            const int seen = 32 - behind < kKeys ? 32 - behind : kKeys;  // by the warp's last row
+#pragma unroll 2
+            for (int key = 0; key < seen; ++key)
+                step<2, true>(out, pw + key * T::kPPitch + ty * 4, vb + key * T::kVPitch, 32, behind + key - ty * 4);
+        }
         __syncthreads();  // every warp is done with V (and with its probabilities)
         if (j + p.splits < n_blocks) load_rows<kKeys, T::kDim, T::kVPitch, NT>(av, v, p.vs[2], (j + p.splits) * kKeys, p.seq_k, p.head_dim, p.v_vec);
         cp_commit();

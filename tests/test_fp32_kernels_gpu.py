@@ -95,3 +95,21 @@ def test_attention_hands_nans_on(causal, dt, b, h, sq, sk, d):
     bad[0, 0, :64] = math.nan  # every key of the first blocks: all rows see key 0
     got = cuda_mod().attention(q.cuda(), bad.cuda(), v.cuda(), scale, causal=causal).cpu()
     assert bool(torch.isnan(got[0, 0]).all()) and torch.equal(got.flatten(0, 1)[1:], clean.flatten(0, 1)[1:])
+
+
+# rows of several warps and CTAs, keys shared by a cluster, two warps per row group, more keys than queries and fewer
+@pytest.mark.parametrize("b,h,sq,sk,d", [(1, 1, 300, 300, 64), (1, 1, 300, 1030, 64), (3, 50, 129, 257, 64), (2, 40, 130, 96, 40), (1, 3, 190, 190, 128),
+                                         (3, 50, 128, 129, 100)])
+def test_attention_rows_do_not_touch_values_behind_the_causal_limit(b, h, sq, sk, d):
+    g = torch.Generator().manual_seed(sq + d)
+    q, k, v = (torch.randn(b, h, s, d, generator=g) for s in (sq, sk, sk))
+    scale = 1 / math.sqrt(d)
+    want = oracle.attention(q, k, v, scale, causal=True)
+    magnitude = oracle.attention(q, k, v.abs(), scale, causal=True)
+    for limit in (1, 37, 64, min(sq, sk) - 1):
+        for bad in (math.inf, math.nan):
+            k2, v2 = k.clone(), v.clone()
+            k2[:, :, limit:], v2[:, :, limit:] = bad, bad
+            got = to_np(cuda_mod().attention(q.cuda(), k2.cuda(), v2.cuda(), scale, causal=True))
+            assert_close(got[:, :, :limit], want[:, :, :limit], 1e-5, f"{limit} {bad}", magnitude=magnitude[:, :, :limit])
+            assert np.isnan(got[:, :, limit:]).all()

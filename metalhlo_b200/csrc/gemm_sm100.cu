@@ -886,28 +886,43 @@ static int launch_cluster(const GemmProblem& pr, int splits, cudaStream_t stream
     return MHLO_CUDA_OK;
 }
 
-// Whether K is split over a cluster, and how: the cheaper of the configurations by a model of measured times (us, kernels
-// behind one another in a graph). One CTA per 128-column tile: 4.5 + 0.27 per 64-deep step of K. A cluster: 4.2, 0.25 or 0.275
-// per step of a 64- or 128-column tile, 0.5 to 0.7 for the exchange; steps cost half as much again once the CTAs outnumber the
-// SMs (two then share a port to L2), and clusters of four and eight do not pack the GPCs completely from about 112 CTAs on.
-// A saving below one microsecond leaves the sum over K in one piece.
-// Measured, [rows, K] . [K, N]: 201 x 768 x 768 8.6 -> 4.8, 201 x 3072 x 768 18.8 -> 7.7, 201 x 768 x 2304 8.4 -> 5.8,
-// 201 x 768 x 3072 9.3 -> 7.2, 1024 x 3072 x 768 19.1 -> 13.1, 256 x 8192 x 256 41.3 -> 8.1; 512 x 768 x 3072 stays with whole tiles.
+// Whether K is split over a cluster, and how: the cheapest configuration by a model of measured times (us, the kernel behind itself
+// in a graph, f16, 429 shapes with 1 to 1024 rows, 64 to 4096 columns, K 128 to 16384). One CTA per tile of 128 columns: 3.7 +
+// 0.285 per 64-deep step of K. A cluster: a fixed cost for launch and exchange and a cost per step of the longest share, both of
+// which grow once the CTAs pass half of the SMs (they share ports to L2, and clusters of four and eight do not pack the GPCs
+// completely), and again beyond one CTA per SM. A saving below one microsecond leaves the sum over K in one piece: no shape of
+// the 429 was slower than that, the choice is 2.6 % behind the best on average.
+// Measured, whole -> split, [rows, K] . [K, N]: 201 x 768 x 768 7.2 -> 5.2, 201 x 3072 x 768 17.4 -> 7.5, 201 x 768 x 2304
+// 7.4 -> 6.0 (a cluster of eight on 288 CTAs: 14.5), 1024 x 3072 x 768 17.9 -> 12.4, 1 x 8192 x 256 38.8 -> 8.4;
+// 201 x 768 x 3072 (7.4) stays whole.
 // Returns the CTAs per cluster, 0 = no split.
 static int cluster_plan(const GemmProblem& p, int* bn) {
     if (p.n_copies > 0 || p.residual != nullptr || p.c_col0 != 0 || (p.ldc != 0 && p.ldc != p.n)) return 0;
     const int64_t rows = (p.m + BM - 1) / BM * p.batch0 * p.batch1, steps = (p.k + BK - 1) / BK;
     const int64_t whole = rows * ((p.n + 127) / 128);
     if (whole > kNumSMs || steps < 2) return 0;
-    double best = 4.5 + 0.27 * static_cast<double>(steps) - 1.0;
+    struct Cost { double fixed, crowded, full, beyond; };  // at few CTAs, + per SM's worth above half, one per SM passed, + per SM's worth
+    static const Cost kCost[2][3] = {{{3.85, 0.5, 4.9, 1.0}, {4.0, 2.4, 5.5, 1.5}, {4.1, 3.0, 6.4, 1.5}},    // 64 columns, clusters of 2, 4, 8
+                                     {{4.55, 1.2, 6.0, 0.8}, {4.9, 2.2, 7.4, 2.6}, {5.1, 5.5, 8.4, 2.0}}};  // 128 columns
+    double best = 3.7 + 0.285 * static_cast<double>(steps) - 1.0;
     int splits = 0;
-    for (const int width : {64, 128})
-        for (const int s : {2, 4, 8}) {
-            const int64_t ctas = rows * ((p.n + width - 1) / width) * s;
+    for (const int wide : {0, 1})
+        for (int i = 0, s = 2; s <= 8; ++i, s *= 2) {
+            const int64_t ctas = rows * ((p.n + (wide ? 127 : 63)) / (wide ? 128 : 64)) * s;
             if (steps < s || ctas > 2 * kNumSMs) continue;
-            const double load = ctas <= (s == 2 ? kNumSMs : 112) ? 1.0 : ctas <= kNumSMs ? 1.3 : 1.5;
-            const double t = 4.2 + load * static_cast<double>((steps + s - 1) / s) * (width == 64 ? 0.25 : 0.275) + (s == 8 ? 0.7 : s == 4 ? 0.5 : 0.6);
-            if (t < best) { best = t; splits = s; *bn = width; }
+            const Cost& c = kCost[wide][i];
+            const double fill = static_cast<double>(ctas) / kNumSMs, longest = static_cast<double>((steps + s - 1) / s);
+            double t, step;
+            if (fill <= 1.0) {
+                const double over = std::max(0.0, fill - 0.5);
+                t = c.fixed + c.crowded * over;
+                step = (wide ? 0.296 : 0.252) * (1.0 + 0.45 * over);
+            } else {
+                t = c.full + c.beyond * (fill - 1.0);
+                step = !wide ? 0.31 + 0.13 * (fill - 1.0) : s == 2 ? 0.39 + 0.07 * (fill - 1.0) : 0.40 + 0.2 * (fill - 1.0);
+            }
+            t += step * longest;
+            if (t < best) { best = t; splits = s; *bn = wide ? 128 : 64; }
         }
     return splits;
 }

@@ -42,10 +42,12 @@ inline OperandMajor a_major(const GemmProblem& p) {
 inline OperandMajor b_major(const GemmProblem& p) {
     return contiguous_along(p.bs[2], p.k, p.bs[3], p.n) ? kMajorK : contiguous_along(p.bs[3], p.n, p.bs[2], p.k) ? kMajorMN : kNoMajor;
 }
-// Base and batch strides of an operand on the grid.
+// Base and batch strides of an operand on the grid. A batch stride of 0 (one matrix for every entry) is: the tensor map then has
+// extent 1 in that dimension and every entry reads coordinate 0.
 inline bool operand_on_grid(const GemmProblem& p, const void* base, const int64_t* st) {
-    return aligned16(base) && (p.batch0 == 1 || tma_stride(st[0])) && (p.batch1 == 1 || tma_stride(st[1]));
+    return aligned16(base) && (p.batch0 == 1 || st[0] == 0 || tma_stride(st[0])) && (p.batch1 == 1 || st[1] == 0 || tma_stride(st[1]));
 }
+inline int64_t operand_batch(int64_t extent, int64_t stride) { return stride == 0 ? 1 : extent; }
 
 // A 2-D convolution of dense NHWC input with dense HWIO filters into dense NHWC output, stride 1, one feature group: the
 // form the tensor-core kernel reads without a patch matrix.

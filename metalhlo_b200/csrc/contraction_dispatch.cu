@@ -173,8 +173,12 @@ int mhlo_cuda_gemm(int32_t in_dtype, int32_t out_dtype, const void* a_dev, const
 namespace {
 // Whether the tensor-core epilogue takes the CUDA library's tanhf and expf rather than the hardware's approximations (2^-11
 // relative). The approximations are for products whose epilogue has to keep up with the MMAs: at least 64 x 64 results, K
-// above 1, operands read in place. Everything else (and every packed product) is bound elsewhere and keeps fp32 precision.
-bool exact_activation(const GemmProblem& p) { return p.m * p.n < 64 * 64 || p.k == 1; }
+// above 1, operands read in place, one matrix each per batch entry. Everything else (and every packed product) is bound elsewhere
+// and keeps fp32 precision.
+bool exact_activation(const GemmProblem& p) {
+    const bool shared = (p.batch0 > 1 && (p.as[0] == 0 || p.bs[0] == 0)) || (p.batch1 > 1 && (p.as[1] == 0 || p.bs[1] == 0));
+    return p.m * p.n < 64 * 64 || p.k == 1 || shared;
+}
 }  // namespace
 
 int mhlo_cuda_gemm_tuned(int32_t in_dtype, int32_t out_dtype, const void* a_dev, const int64_t a_strides[4],

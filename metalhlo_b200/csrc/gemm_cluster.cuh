@@ -84,6 +84,7 @@ __global__ void __launch_bounds__(kClusterThreads, 1) gemm_cluster_kernel(const 
     if (warp == 0) {
         if (lane == 0) {
             const int b0 = bz / static_cast<int>(p.batch1), b1 = bz % static_cast<int>(p.batch1);
+            const int a0 = b0 * p.a_batch[0], a1 = b1 * p.a_batch[1], w0 = b0 * p.b_batch[0], w1 = b1 * p.b_batch[1];
             int stage = 0;
             uint32_t phase = 0;
             for (int kb = kb_begin; kb < kb_end; ++kb) {
@@ -92,16 +93,16 @@ __global__ void __launch_bounds__(kClusterThreads, 1) gemm_cluster_kernel(const 
                 uint8_t* sb = sa + L::kABytes;
                 mbar_expect_tx(&full_bar[stage], L::kStageBytes);
                 if (!p.a_mn_major) {
-                    tma_load_4d(sa, &map_a, &full_bar[stage], kb * BK, tm * BM, b1, b0);
+                    tma_load_4d(sa, &map_a, &full_bar[stage], kb * BK, tm * BM, a1, a0);
                 } else {
 #pragma unroll
-                    for (int j = 0; j < BM / 64; ++j) tma_load_4d(sa + j * 64 * BK * 2, &map_a, &full_bar[stage], tm * BM + j * 64, kb * BK, b1, b0);
+                    for (int j = 0; j < BM / 64; ++j) tma_load_4d(sa + j * 64 * BK * 2, &map_a, &full_bar[stage], tm * BM + j * 64, kb * BK, a1, a0);
                 }
                 if (!p.b_mn_major) {
-                    tma_load_4d(sb, &map_b, &full_bar[stage], kb * BK, tn * BN, b1, b0);
+                    tma_load_4d(sb, &map_b, &full_bar[stage], kb * BK, tn * BN, w1, w0);
                 } else {
 #pragma unroll
-                    for (int j = 0; j < BN / 64; ++j) tma_load_4d(sb + j * 64 * BK * 2, &map_b, &full_bar[stage], tn * BN + j * 64, kb * BK, b1, b0);
+                    for (int j = 0; j < BN / 64; ++j) tma_load_4d(sb + j * 64 * BK * 2, &map_b, &full_bar[stage], tn * BN + j * 64, kb * BK, w1, w0);
                 }
                 if (++stage == kClusterStages) { stage = 0; phase ^= 1; }
             }

@@ -92,6 +92,7 @@ struct GemmParams {
     int32_t tiles_m, tiles_n;
     int64_t num_tiles;
     int32_t a_mn_major, b_mn_major;  // 0 = K-major, 1 = M/N-major
+    int32_t a_batch[2], b_batch[2];  // 0: the operand is the same for every entry of that batch dimension
     int32_t in_bf16;                 // operand format: 1 = bf16, 0 = f16
     int32_t out_dtype;               // MHLO_DT_BF16 / F16 / F32
     int32_t epilogue;
@@ -219,6 +220,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
                 int bz, tm, tn;
                 tile_coords(tile, p, &bz, &tm, &tn);
                 const int b0 = bz / static_cast<int>(p.batch1), b1 = bz % static_cast<int>(p.batch1);
+                const int za[2] = {b0 * p.a_batch[0], b1 * p.a_batch[1]}, zb[2] = {b0 * p.b_batch[0], b1 * p.b_batch[1]};
                 const int row_a = (tm * CTAS + static_cast<int>(cta_rank)) * BM;    // first row of A this CTA stages
                 const int row_b = tn * BN + static_cast<int>(cta_rank) * BNL;       // first row of B (column of the tile)
                 for (int kb = 0; kb < k_blocks; ++kb) {
@@ -234,10 +236,10 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
                     } else {
                         mbar_expect_tx(&full_bar[stage], L::kStageBytes);
                     }
-                    auto load = [&](uint8_t* dst, const CUtensorMap* map, int c0, int c1) {
-                        if constexpr (kPair) tma_load_4d_pair(dst, map, full_addr, c0, c1, b1, b0);
+                    auto load = [&](uint8_t* dst, const CUtensorMap* map, int c0, int c1, const int* batch) {
+                        if constexpr (kPair) tma_load_4d_pair(dst, map, full_addr, c0, c1, batch[1], batch[0]);
                         else if constexpr (MODE == 3) tma_load_4d(dst, map, &full_bar[stage], c0, c1, 0, 0);  // the filter matrix has no batch
-                        else tma_load_4d(dst, map, &full_bar[stage], c0, c1, b1, b0);
+                        else tma_load_4d(dst, map, &full_bar[stage], c0, c1, batch[1], batch[0]);
                     };
                     if constexpr (MODE == 3) {
                         const int ty = tm / p.conv_tiles_x, tx = tm - ty * p.conv_tiles_x;
@@ -248,16 +250,16 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
                         tma_load_4d(sa, &map_a, &full_bar[stage], cb * 64, tx * 16 * p.conv_stride_w + dx * p.conv_dil_w - p.conv_pad_w,
                                     ty * 8 * p.conv_stride_h + dy * p.conv_dil_h - p.conv_pad_h, bz);
                     } else if (!p.a_mn_major) {
-                        load(sa, &map_a, kb * BK, row_a);
+                        load(sa, &map_a, kb * BK, row_a, za);
                     } else {
 #pragma unroll
-                        for (int j = 0; j < BM / 64; ++j) load(sa + j * 64 * BK * 2, &map_a, row_a + j * 64, kb * BK);
+                        for (int j = 0; j < BM / 64; ++j) load(sa + j * 64 * BK * 2, &map_a, row_a + j * 64, kb * BK, za);
                     }
                     if (!p.b_mn_major) {
-                        load(sb, &map_b, kb * BK, row_b);
+                        load(sb, &map_b, kb * BK, row_b, zb);
                     } else {
 #pragma unroll
-                        for (int j = 0; j < BNL / 64; ++j) load(sb + j * 64 * BK * 2, &map_b, row_b + j * 64, kb * BK);
+                        for (int j = 0; j < BNL / 64; ++j) load(sb + j * 64 * BK * 2, &map_b, row_b + j * 64, kb * BK, zb);
                     }
                     if (++stage == p.stages) { stage = 0; phase ^= 1; }
                 }
@@ -717,11 +719,11 @@ static int launch_gemm_act(const GemmProblem& pr, cudaStream_t stream) {
     CUtensorMap map_a, map_b;
     std::string why;
     bool ok;
-    if (a_k) ok = operand_map(&map_a, pr.a, pr.k, pr.m, pr.as[2], pr.batch1, pr.as[1], pr.batch0, pr.as[0], BK, BM, &why);
-    else ok = operand_map(&map_a, pr.a, pr.m, pr.k, pr.as[3], pr.batch1, pr.as[1], pr.batch0, pr.as[0], 64, BK, &why);
+    if (a_k) ok = operand_map(&map_a, pr.a, pr.k, pr.m, pr.as[2], operand_batch(pr.batch1, pr.as[1]), pr.as[1], operand_batch(pr.batch0, pr.as[0]), pr.as[0], BK, BM, &why);
+    else ok = operand_map(&map_a, pr.a, pr.m, pr.k, pr.as[3], operand_batch(pr.batch1, pr.as[1]), pr.as[1], operand_batch(pr.batch0, pr.as[0]), pr.as[0], 64, BK, &why);
     if (!ok) return fail(MHLO_CUDA_EXECUTION_FAILED, "gemm: tensor map for A: %s", why.c_str());
-    if (b_k) ok = operand_map(&map_b, pr.b, pr.k, pr.n, pr.bs[3], pr.batch1, pr.bs[1], pr.batch0, pr.bs[0], BK, BN / CTAS, &why);
-    else ok = operand_map(&map_b, pr.b, pr.n, pr.k, pr.bs[2], pr.batch1, pr.bs[1], pr.batch0, pr.bs[0], 64, BK, &why);
+    if (b_k) ok = operand_map(&map_b, pr.b, pr.k, pr.n, pr.bs[3], operand_batch(pr.batch1, pr.bs[1]), pr.bs[1], operand_batch(pr.batch0, pr.bs[0]), pr.bs[0], BK, BN / CTAS, &why);
+    else ok = operand_map(&map_b, pr.b, pr.n, pr.k, pr.bs[2], operand_batch(pr.batch1, pr.bs[1]), pr.bs[1], operand_batch(pr.batch0, pr.bs[0]), pr.bs[0], 64, BK, &why);
     if (!ok) return fail(MHLO_CUDA_EXECUTION_FAILED, "gemm: tensor map for B: %s", why.c_str());
 
     GemmParams p;
@@ -736,6 +738,7 @@ static int launch_gemm_act(const GemmProblem& pr, cudaStream_t stream) {
     p.num_tiles = static_cast<int64_t>(p.tiles_m) * p.tiles_n * pr.batch0 * pr.batch1;
     p.a_mn_major = a_k ? 0 : 1;
     p.b_mn_major = b_k ? 0 : 1;
+    for (int i = 0; i < 2; ++i) { p.a_batch[i] = pr.as[i] != 0; p.b_batch[i] = pr.bs[i] != 0; }
     p.in_bf16 = pr.in_dtype == MHLO_DT_BF16;
     p.out_dtype = pr.out_dtype;
     p.epilogue = pr.epilogue;
@@ -850,11 +853,11 @@ static int launch_cluster(const GemmProblem& pr, int splits, cudaStream_t stream
     CUtensorMap map_a, map_b;
     std::string why;
     bool ok;
-    if (a_k) ok = operand_map(&map_a, pr.a, pr.k, pr.m, pr.as[2], pr.batch1, pr.as[1], pr.batch0, pr.as[0], BK, BM, &why);
-    else ok = operand_map(&map_a, pr.a, pr.m, pr.k, pr.as[3], pr.batch1, pr.as[1], pr.batch0, pr.as[0], 64, BK, &why);
+    if (a_k) ok = operand_map(&map_a, pr.a, pr.k, pr.m, pr.as[2], operand_batch(pr.batch1, pr.as[1]), pr.as[1], operand_batch(pr.batch0, pr.as[0]), pr.as[0], BK, BM, &why);
+    else ok = operand_map(&map_a, pr.a, pr.m, pr.k, pr.as[3], operand_batch(pr.batch1, pr.as[1]), pr.as[1], operand_batch(pr.batch0, pr.as[0]), pr.as[0], 64, BK, &why);
     if (!ok) return fail(MHLO_CUDA_EXECUTION_FAILED, "gemm: tensor map for A: %s", why.c_str());
-    if (b_k) ok = operand_map(&map_b, pr.b, pr.k, pr.n, pr.bs[3], pr.batch1, pr.bs[1], pr.batch0, pr.bs[0], BK, BN, &why);
-    else ok = operand_map(&map_b, pr.b, pr.n, pr.k, pr.bs[2], pr.batch1, pr.bs[1], pr.batch0, pr.bs[0], 64, BK, &why);
+    if (b_k) ok = operand_map(&map_b, pr.b, pr.k, pr.n, pr.bs[3], operand_batch(pr.batch1, pr.bs[1]), pr.bs[1], operand_batch(pr.batch0, pr.bs[0]), pr.bs[0], BK, BN, &why);
+    else ok = operand_map(&map_b, pr.b, pr.n, pr.k, pr.bs[2], operand_batch(pr.batch1, pr.bs[1]), pr.bs[1], operand_batch(pr.batch0, pr.bs[0]), pr.bs[0], 64, BK, &why);
     if (!ok) return fail(MHLO_CUDA_EXECUTION_FAILED, "gemm: tensor map for B: %s", why.c_str());
     GemmParams p;
     memset(&p, 0, sizeof p);
@@ -867,6 +870,7 @@ static int launch_cluster(const GemmProblem& pr, int splits, cudaStream_t stream
     p.num_tiles = static_cast<int64_t>(p.tiles_m) * p.tiles_n * pr.batch0 * pr.batch1;
     p.a_mn_major = a_k ? 0 : 1;
     p.b_mn_major = b_k ? 0 : 1;
+    for (int i = 0; i < 2; ++i) { p.a_batch[i] = pr.as[i] != 0; p.b_batch[i] = pr.bs[i] != 0; }
     p.in_bf16 = pr.in_dtype == MHLO_DT_BF16;
     p.out_dtype = pr.out_dtype;
     p.epilogue = pr.epilogue | (pr.exact_act ? kExactAct : 0);

@@ -35,9 +35,12 @@ __global__ void __launch_bounds__(256) pack_operands_kernel(const __grid_constan
     for (int64_t c = lane; c < j.cols; c += 32) d[c] = s[c * j.s_col];
 }
 
-// Packs along whichever dimension is contiguous (the columns if neither is) and rewrites the operand's strides.
+// Packs along whichever dimension is contiguous (if neither is, the columns; a single column as one row) and rewrites the
+// operand's strides. A matrix that every entry of a batch dimension shares is packed once.
 void plan(PackJob* j, const void* p, int64_t* st, int64_t batch0, int64_t batch1, int64_t rows, int64_t cols) {
-    const bool along_rows = st[3] != 1 && st[2] == 1;
+    const bool along_rows = cols == 1 || (st[3] != 1 && st[2] == 1 && rows > 1);
+    batch0 = operand_batch(batch0, st[0]);
+    batch1 = operand_batch(batch1, st[1]);
     j->src = static_cast<const uint16_t*>(p);
     j->s_batch0 = st[0]; j->s_batch1 = st[1];
     j->s_row = along_rows ? st[3] : st[2];
@@ -48,8 +51,8 @@ void plan(PackJob* j, const void* p, int64_t* st, int64_t batch0, int64_t batch1
     j->pitch = (j->cols + 7) / 8 * 8;
     j->all_rows = batch0 * batch1 * j->rows;
     const int64_t matrix = j->rows * j->pitch;
-    st[0] = batch1 * matrix;
-    st[1] = matrix;
+    if (st[0] != 0) st[0] = batch1 * matrix;
+    if (st[1] != 0) st[1] = matrix;
     st[2] = along_rows ? 1 : j->pitch;
     st[3] = along_rows ? j->pitch : 1;
 }

@@ -131,3 +131,20 @@ def test_activations_in_fp32(m, n, k, split, epilogue, dt, out_dtype):
     bound = UNIT[out_dtype] * ACT[epilogue](x).abs() + 1.13 * (k + 2) * u * (magnitude + bias.double().abs()) + 12 * u * (x.abs() + 1)
     worst = ((got.double() - ACT[epilogue](x)).abs() / bound).max().item()
     assert worst <= 1.0, worst
+
+
+# one matrix for every batch entry (stride 0) on either side and in either batch dimension, rows on the grid and off it, K split or not
+@pytest.mark.parametrize("split", [0, 1])
+@pytest.mark.parametrize("m,n,k", [(130, 200, 64), (65, 131, 300), (64, 64, 2048), (1, 1000, 129)])
+@pytest.mark.parametrize("shared", ["a", "b", "a0", "b1", "ab"])
+def test_matrices_shared_by_a_batch(m, n, k, shared, split):
+    b0, b1 = 3, 2
+    g = torch.Generator().manual_seed(m + k)
+    na = (1 if shared in ("a", "ab", "a0") else b0, 1 if shared in ("a", "ab") else b1)
+    nb = (1 if shared in ("b", "ab") else b0, 1 if shared in ("b", "ab", "b1") else b1)
+    a = torch.randn(*na, m, k, generator=g).half().cuda()
+    b = (torch.randn(*nb, k, n, generator=g) / math.sqrt(k)).half().cuda()
+    strides = [tuple(0 if e == 1 else s for e, s in zip(x.shape[:2], x.stride()[:2])) for x in (a, b)]
+    got = raw_gemm(a, b, torch.float16, b0, b1, *strides, tuning=(0, 0, 0, split))
+    shape = (b0, b1, m, n)
+    close(got, (a.double() @ b.double()).expand(shape), k, (a.double().abs() @ b.double().abs()).expand(shape))

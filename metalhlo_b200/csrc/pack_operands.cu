@@ -60,7 +60,7 @@ void plan(PackJob* j, const void* p, int64_t* st, int64_t batch0, int64_t batch1
 }  // namespace
 
 bool gemm_pack_launch(GemmProblem p, cudaStream_t stream, int* status) {
-    if (p.in_dtype != MHLO_DT_F16 && p.in_dtype != MHLO_DT_BF16) return false;
+    if ((p.in_dtype != MHLO_DT_F16 && p.in_dtype != MHLO_DT_BF16) || p.out_dtype != p.in_dtype) return false;  // fp32 results: fp32 sums
     if (p.a == nullptr || p.b == nullptr || p.n_copies > 0 || p.m <= 0 || p.n <= 0 || p.k <= 0 || p.batch0 <= 0 || p.batch1 <= 0) return false;
     if (p.m > 0x7fffffff || p.n > 0x7fffffff || p.k > 0x7fffffff || p.batch0 * p.batch1 > 0x7fffffff) return false;
     // the copy and the product's fixed cost are about 6 us: the general kernel is quicker for a few panels of one tile

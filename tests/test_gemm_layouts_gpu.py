@@ -148,3 +148,15 @@ def test_matrices_shared_by_a_batch(m, n, k, shared, split):
     got = raw_gemm(a, b, torch.float16, b0, b1, *strides, tuning=(0, 0, 0, split))
     shape = (b0, b1, m, n)
     close(got, (a.double() @ b.double()).expand(shape), k, (a.double().abs() @ b.double().abs()).expand(shape))
+
+
+# fp32 results of 16-bit operands: packed, few results, K of 1, a shared matrix
+@pytest.mark.parametrize("m,n,k,shared", [(65, 67, 1069, False), (16, 128, 4096, False), (8, 10, 4096, False), (512, 512, 1, False), (130, 200, 2048, True)])
+@pytest.mark.parametrize("split", [0, 1])
+def test_fp32_results_of_other_products_have_fp32_sums(m, n, k, shared, split):
+    g = torch.Generator().manual_seed(k)
+    a, b = torch.randn(2 if shared else 1, m, k, generator=g).half().cuda(), (torch.randn(k, n, generator=g) / math.sqrt(k)).half().cuda()
+    got = raw_gemm(a, b, torch.float16, 1, 2 if shared else 1, (0, m * k), tuning=(0, 0, 0, split), out_dtype=torch.float32)[0]
+    want = a.double() @ b.double()
+    # a running fp32 sum of k independent terms errs by about sqrt(k) / 2 roundings of the result's size; the tensor cores by 3e-6 at 4096
+    assert float((got.double() - want).norm() / want.norm()) <= 2.0 ** -24 * (1 + math.sqrt(k) / 2)

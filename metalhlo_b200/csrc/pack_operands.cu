@@ -14,25 +14,31 @@ struct PackJob {
     int64_t s_batch0, s_batch1, s_row, s_col;  // element strides of the source
     int64_t batch1, rows, cols, pitch;         // destination: [batch0][batch1][rows][pitch]
     int64_t all_rows;                          // batch0 * batch1 * rows
+    int64_t pieces;                            // of kPackColumns columns per row
 };
 struct PackJobs {
     PackJob job[2];
     int64_t blocks0;  // blocks of the first job
 };
 
-// A warp per row, consecutive lanes on consecutive columns (64 bytes per load and store instruction).
+// A warp per row, or per 512 columns of a longer row, consecutive lanes on consecutive columns (64 bytes per load and store
+// instruction). 512 columns are 16 trips of a warp: with whole rows, an operand of few long rows kept few warps busy
+// ([768, 50257], the weights of a product of one row: 543 us with it, 92 in pieces).
+constexpr int kPackColumns = 512;
+
 __global__ void __launch_bounds__(256) pack_operands_kernel(const __grid_constant__ PackJobs jobs) {
     const bool second = blockIdx.x >= jobs.blocks0;
     const PackJob& j = jobs.job[second];
     const int64_t block = blockIdx.x - (second ? jobs.blocks0 : 0);
     const int lane = threadIdx.x & 31;
-    const int64_t row = block * 8 + (threadIdx.x >> 5);
+    const int64_t unit = block * 8 + (threadIdx.x >> 5), row = unit / j.pieces;
     if (row >= j.all_rows) return;
+    const int64_t c0 = unit % j.pieces * kPackColumns, c1 = c0 + kPackColumns < j.cols ? c0 + kPackColumns : j.cols;
     const int64_t b = row / j.rows, r = row % j.rows;
     const uint16_t* s = j.src + b / j.batch1 * j.s_batch0 + b % j.batch1 * j.s_batch1 + r * j.s_row;
     uint16_t* d = j.dst + row * j.pitch;
 #pragma unroll 8
-    for (int64_t c = lane; c < j.cols; c += 32) d[c] = s[c * j.s_col];
+    for (int64_t c = c0 + lane; c < c1; c += 32) d[c] = s[c * j.s_col];
 }
 
 // Packs along whichever dimension is contiguous (if neither is, the columns; a single column as one row) and rewrites the
@@ -50,6 +56,7 @@ void plan(PackJob* j, const void* p, int64_t* st, int64_t batch0, int64_t batch1
     j->cols = along_rows ? rows : cols;
     j->pitch = (j->cols + 7) / 8 * 8;
     j->all_rows = batch0 * batch1 * j->rows;
+    j->pieces = (j->cols + kPackColumns - 1) / kPackColumns;
     const int64_t matrix = j->rows * j->pitch;
     if (st[0] != 0) st[0] = batch1 * matrix;
     if (st[1] != 0) st[1] = matrix;
@@ -63,8 +70,10 @@ bool gemm_pack_launch(GemmProblem p, cudaStream_t stream, int* status) {
     if ((p.in_dtype != MHLO_DT_F16 && p.in_dtype != MHLO_DT_BF16) || p.out_dtype != p.in_dtype) return false;  // fp32 results: fp32 sums
     if (p.a == nullptr || p.b == nullptr || p.n_copies > 0 || p.m <= 0 || p.n <= 0 || p.k <= 0 || p.batch0 <= 0 || p.batch1 <= 0) return false;
     if (p.m > 0x7fffffff || p.n > 0x7fffffff || p.k > 0x7fffffff || p.batch0 * p.batch1 > 0x7fffffff) return false;
-    // the copy and the product's fixed cost are about 6 us: the general kernel is quicker for a few panels of one tile
-    if (p.m * p.n * p.k < 64 * 1024) return false;
+    // Copy and product cost 10 to 14 us before the first panel; the general kernel does 32 steps of K in 10, whatever the number of
+    // results up to about eight million ([33,31] . [31,4001] 14 us packed, 10 there; with K = 63 14 and 15; [301,15] . [15,50257]
+    // 37 and 46).
+    if (p.m * p.n * p.k < 64 * 1024 || (p.k <= 32 && p.m * p.n * p.batch0 * p.batch1 < int64_t{1} << 23)) return false;
     PackJobs jobs;
     memset(&jobs, 0, sizeof jobs);
     int n = 0;
@@ -81,7 +90,7 @@ bool gemm_pack_launch(GemmProblem p, cudaStream_t stream, int* status) {
         bytes += static_cast<size_t>(jobs.job[n].all_rows * jobs.job[n].pitch * 2 + 255) / 256 * 256;
         ++n;
     }
-    const int64_t blocks[2] = {(jobs.job[0].all_rows + 7) / 8, (jobs.job[1].all_rows + 7) / 8};
+    const int64_t blocks[2] = {(jobs.job[0].all_rows * jobs.job[0].pieces + 7) / 8, (jobs.job[1].all_rows * jobs.job[1].pieces + 7) / 8};
     p.exact_act = 1;
     if (n == 0 || !gemm_tc_supported(p) || blocks[0] + blocks[1] > 0x7fffffff) return false;
     void* scratch = nullptr;

@@ -351,6 +351,7 @@ int launch_split(Fp32Gemm p, int64_t batches, cudaStream_t stream) {
 }  // namespace
 
 bool gemm_fp32_supported(const GemmProblem& g) {
+    if (g.batch0 <= 0 || g.batch1 <= 0 || g.m <= 0 || g.n <= 0) return false;
     return g.in_dtype == MHLO_DT_F32 && g.out_dtype == MHLO_DT_F32 && g.residual == nullptr && g.n_copies == 0 && (g.ldc == 0 || g.ldc == g.n) &&
            g.c_col0 == 0 && g.batch0 * g.batch1 <= 65535 && g.m * g.n > 0 && g.k > 0 && g.m < (int64_t{1} << 31) && g.n < (int64_t{1} << 31);
 }

@@ -113,3 +113,21 @@ def test_attention_rows_do_not_touch_values_behind_the_causal_limit(b, h, sq, sk
             got = to_np(cuda_mod().attention(q.cuda(), k2.cuda(), v2.cuda(), scale, causal=True))
             assert_close(got[:, :, :limit], want[:, :, :limit], 1e-5, f"{limit} {bad}", magnitude=magnitude[:, :, :limit])
             assert np.isnan(got[:, :, limit:]).all()
+
+
+def test_gemm_fp32_empty_and_refused_extents():
+    import ctypes as C
+
+    cuda = cuda_mod()
+    bias = torch.zeros(6).cuda()
+    for shape_a, shape_b in (((0, 4, 5), (0, 5, 6)), ((2, 0, 4, 5), (2, 0, 5, 6)), ((3, 0, 5), (3, 5, 6))):
+        got = cuda.gemm(torch.zeros(shape_a).cuda(), torch.zeros(shape_b).cuda(), bias=bias, epilogue="relu")
+        assert got.shape == (*shape_a[:-1], 6) and got.numel() == 0
+    x = torch.ones(64).cuda()
+    for b0, b1, m, n, k in ((-1, -1, 4, 4, 4), (1, 1, -4, -4, 4), (1, 1, 4, 4, -4)):
+        status = cuda.lib.mhlo_cuda_gemm(cuda.F32, cuda.F32, x.data_ptr(), cuda._i64s([0, 0, 4, 1]), x.data_ptr(), cuda._i64s([0, 0, 4, 1]),
+                                         x.data_ptr(), b0, b1, m, n, k, None, 0, None)
+        assert status == 10, (b0, b1, m, n, k)
+    torch.cuda.synchronize()
+    assert bool((x == 1).all())
+

@@ -11,7 +11,7 @@
 //
 // Three shapes of the same CTA:  128 x 128, one group of threads;  64 x 64, four groups that take a quarter of every K
 // panel each;  16 x 64, sixteen groups. Smaller tiles trade operand reuse for CTAs: the dispatch takes the largest whose
-// tiles fill the 148 SMs. When even 64 x 64 (or 16 x 64) tiles are too few, K is split over a cluster of 2, 4 or 8 CTAs
+// tiles fill the 148 SMs and are mostly filled themselves. When even 64 x 64 (or 16 x 64) tiles are too few, K is split over a cluster of 2, 4 or 8 CTAs
 // whose partial tiles meet through distributed shared memory - no workspace, no atomics, the same sum on every run.
 #include <cooperative_groups.h>
 
@@ -350,8 +350,16 @@ int launch_split(Fp32Gemm p, int64_t batches, cudaStream_t stream) {
 
 }  // namespace
 
+// Few steps of K in many tiles: a CTA's prologue (addresses, the ring's first two panels) is then most of its work and the general
+// kernel is quicker: 4096 products of [64,4] . [4,4] 41 us there, 67 here; [262144,8] . [8,32] 42 and 68. At K = 32 the second takes
+// 69 and 70, at K = 64 120 and 80; with two tiles per SM or fewer this kernel leads at any K.
+static bool short_sums(const GemmProblem& g) {
+    const int64_t tiles = (g.m <= 16 ? 1 : (g.m + 63) / 64) * ((g.n + 63) / 64) * g.batch0 * g.batch1;
+    return g.k <= 16 && tiles > 2 * kNumSMs;
+}
+
 bool gemm_fp32_supported(const GemmProblem& g) {
-    if (g.batch0 <= 0 || g.batch1 <= 0 || g.m <= 0 || g.n <= 0) return false;
+    if (g.batch0 <= 0 || g.batch1 <= 0 || g.m <= 0 || g.n <= 0 || short_sums(g)) return false;
     return g.in_dtype == MHLO_DT_F32 && g.out_dtype == MHLO_DT_F32 && g.residual == nullptr && g.n_copies == 0 && (g.ldc == 0 || g.ldc == g.n) &&
            g.c_col0 == 0 && g.batch0 * g.batch1 <= 65535 && g.m * g.n > 0 && g.k > 0 && g.m < (int64_t{1} << 31) && g.n < (int64_t{1} << 31);
 }
@@ -374,7 +382,10 @@ int gemm_fp32_launch(const GemmProblem& g, cudaStream_t stream) {
     p.tiles_n = static_cast<int32_t>((p.n + 127) / 128);
     const int64_t large = (p.m + 127) / 128 * p.tiles_n;
     if (large > 0x7fffffff) return fail(MHLO_CUDA_UNSUPPORTED, "gemm: more than 2^31 tiles");
-    if (large * batches >= kFill) return launch<128, 128, 16, 1, false>(p, large, batches, 1, stream);
+    // Large tiles only where at least 0.6 of them is results (a row or column block of 64 of the 128 takes no less time than a
+    // whole one: [65536,64] . [64,32] 47 us, 24 in tiles of 64 x 64) and K is more than two panels of the small tile.
+    const bool filled = 5 * p.m * p.n >= 3 * large * 128 * 128;
+    if (large * batches >= kFill && filled && p.k > 64) return launch<128, 128, 16, 1, false>(p, large, batches, 1, stream);
     return launch_split<64, 64, 32, 4>(p, batches, stream);
 }
 

@@ -131,3 +131,15 @@ def test_gemm_fp32_empty_and_refused_extents():
     torch.cuda.synchronize()
     assert bool((x == 1).all())
 
+
+
+# either side of the lines of the dispatch: K of 16 and 17 with 296 tiles and more; 128 x 128 tiles filled to 0.6 or not, K of 64 and 65
+@pytest.mark.parametrize("b,m,n,k", [(296, 16, 64, 16), (297, 16, 64, 16), (297, 1, 3, 4), (297, 16, 64, 17), (296, 17, 64, 16), (297, 17, 64, 16), (297, 64, 33, 17),
+                                     (1, 19000, 5, 16), (1, 30208, 77, 65), (1, 30208, 76, 65), (1, 77, 30208, 65), (1, 30208, 128, 64), (60, 129, 200, 70),
+                                     (1, 40000, 1, 100)])
+def test_gemm_fp32_lines_of_the_dispatch(b, m, n, k):
+    g = torch.Generator().manual_seed(b + m + n + k)
+    x, y = torch.randn(b, m, k, generator=g), torch.randn(b, k, n, generator=g)
+    got = cuda_mod().gemm(x.cuda(), y.cuda()).double().cpu()
+    bound = (k + 2) * 2.0 ** -24 * (x.double().abs() @ y.double().abs())
+    assert bool(((got - x.double() @ y.double()).abs() <= bound).all())

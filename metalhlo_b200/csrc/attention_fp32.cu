@@ -376,7 +376,32 @@ int launch(Fp32Attention p, int64_t batch_heads, cudaStream_t stream) {
 
 }  // namespace
 
+// Whether the tiles are quicker than the general kernel's warp per query row. A tile costs the same whether 1 or 32 of its rows exist:
+// one query against many keys of many heads (a decoding step), or a handful of keys, is the general kernel's. The times (us) are
+// fits to 508 measured shapes (1 to 4096 heads, 1 to 32 queries, 1 to 512 keys, head dimensions 4 to 128); none of them is sent to
+// the tiles to take longer there. 4096 heads of one query and 128 keys of 64: 236 us there, 411 here; 8 queries: 1319 and 420.
+static bool tiles_pay(const AttnShape& s) {
+    const int64_t heads = s.batch * s.heads, rows = heads * s.seq_q, keys = s.causal && s.seq_q < s.seq_k ? s.seq_q : s.seq_k;
+    const double dim = static_cast<double>(s.head_dim), seen = s.causal ? 0.5 * static_cast<double>(keys + 1) : static_cast<double>(keys);
+    const double one_row = 3.0 + static_cast<double>(keys) * (0.13 + 0.0045 * dim);              // a warp's chain over its keys
+    const double all_rows = static_cast<double>(rows) * (0.45 + seen * (0.034 + 0.0036 * dim)) * 1e-3;  // the machine full of warps
+    const int64_t tiles = heads * ((s.seq_q + 31) / 32), per = s.head_dim <= 64 ? 32 : 64, blocks = (keys + per - 1) / per;
+    int64_t splits = 1;
+    while (splits < 8 && tiles * splits * 2 <= 2 * kNumSMs && blocks >= splits * 2) splits *= 2;
+    const double longest = static_cast<double>((blocks + splits - 1) / splits), exchange = splits > 1 ? 4.0 : 0.0;
+    double one_tile, all_tiles;
+    if (s.head_dim <= 64) {
+        one_tile = 3.5 + 5.2 * longest + exchange;
+        all_tiles = static_cast<double>(tiles) * (3.5 + 24.5 * static_cast<double>(blocks)) * 1e-3;
+    } else {  // one CTA to an SM
+        one_tile = 2.0 + 10.3 * longest + exchange;
+        all_tiles = tiles > kNumSMs ? (2.0 + 13.5 * static_cast<double>(blocks)) * static_cast<double>((tiles + kNumSMs - 1) / kNumSMs) : 0.0;
+    }
+    return (one_tile > all_tiles ? one_tile : all_tiles) <= (one_row > all_rows ? one_row : all_rows);
+}
+
 bool attention_fp32_supported(int dtype, const AttnShape& s) {
+    if (!tiles_pay(s)) return false;
     return dtype == MHLO_DT_F32 && s.head_dim <= 128 && s.batch * s.heads < (int64_t{1} << 27) && s.seq_q <= 32 * int64_t{65535} &&
            s.seq_k < (int64_t{1} << 30);
 }

@@ -143,3 +143,19 @@ def test_gemm_fp32_lines_of_the_dispatch(b, m, n, k):
     got = cuda_mod().gemm(x.cuda(), y.cuda()).double().cpu()
     bound = (k + 2) * 2.0 ** -24 * (x.double().abs() @ y.double().abs())
     assert bool(((got - x.double() @ y.double()).abs() <= bound).all())
+
+
+# shapes either side of the choice between tiles and a warp per query row: a decoding step of few and of many heads, few keys, few queries
+@pytest.mark.parametrize("causal", [False, True])
+@pytest.mark.parametrize("b,h,sq,sk,d", [(1, 1, 1, 300, 64), (40, 50, 1, 100, 64), (40, 50, 3, 100, 64), (40, 50, 8, 100, 64), (1, 1, 32, 8, 64), (1, 1, 32, 40, 64),
+                                         (30, 10, 1, 200, 128), (30, 10, 9, 200, 128), (2, 2, 5, 64, 4), (2, 2, 5, 300, 4), (3, 1, 700, 3, 20)])
+def test_attention_fp32_few_rows_or_keys(causal, b, h, sq, sk, d):
+    g = torch.Generator().manual_seed(sq + sk + d)
+    q, k, v = (torch.randn(b, h, s, d, generator=g) for s in (sq, sk, sk))
+    scale = 1 / math.sqrt(d)
+    s = q.double() @ k.double().transpose(-1, -2) * scale
+    if causal:
+        s = s.masked_fill(torch.ones(sq, sk, dtype=torch.bool).triu(1), -math.inf)
+    p = torch.softmax(s, -1)
+    got = cuda_mod().attention(q.cuda(), k.cuda(), v.cuda(), scale, causal=causal)
+    assert_close(to_np(got), (p @ v.double()).numpy(), 1e-5, f"{sq}x{sk} d{d}", magnitude=(p @ v.double().abs()).numpy())

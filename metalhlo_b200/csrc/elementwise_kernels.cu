@@ -4,7 +4,8 @@
 //
 // A thread works on V consecutive elements of the innermost dimension (16 bytes of a 16-bit or 32-bit operand), so that the
 // opcode switch, the coordinate arithmetic (multiply-high divisions by the extents) and the type switch of a load are paid
-// once per V elements and dense operands move in 16-byte accesses. Rows whose length is no multiple of V end in a partial
+// once per V elements and dense operands move in 16-byte accesses. Where the elements are too few to fill the machine a thread
+// takes one (kFewElements): its chain of work is then what a call lasts. Rows whose length is no multiple of V end in a partial
 // vector. A program of one instruction keeps its operands in registers; a longer one keeps the values that more than the
 // next instruction reads in shared-memory slots, one private column of 16-byte words per thread (no conflicts, no
 // barriers), assigned by liveness on the host.
@@ -176,6 +177,9 @@ __device__ __noinline__ int64_t ew_int_outlined(int op, int64_t a, int64_t b, in
     return ew_int_op(op, a, b, c, imm, uns, boolean, bits);
 }
 
+// (powf from a call of its own: behind the switch of ew_outlined it took 7 % longer, 16.8 M elements 77 us against 72)
+__device__ __noinline__ float ew_pow(float a, float b) { return powf(a, b); }
+
 // ---- launch parameters -------------------------------------------------------------------------------------------------
 
 enum EwAccess : int32_t { kSplat = 0, kVector = 1, kStrided = 2 };  // the operand along the innermost dimension
@@ -233,7 +237,7 @@ __device__ __forceinline__ void load_operand(const EwOperand& o, int64_t at, int
         for (int e = 0; e < V; ++e) x[e] = v;
         return;
     }
-    if constexpr (std::is_same<C, float>::value) {
+    if constexpr (std::is_same<C, float>::value && V >= 4) {
         if (o.access == kVector && count == V) {
             if (o.dtype == MHLO_DT_F32) {
 #pragma unroll
@@ -263,7 +267,7 @@ __device__ __forceinline__ void load_operand(const EwOperand& o, int64_t at, int
         case MHLO_DT_I16: return load_strided<int16_t, C, V>(o.base, at, o.inner, count, x);
         case MHLO_DT_UI16: return load_strided<uint16_t, C, V>(o.base, at, o.inner, count, x);
         case MHLO_DT_I32:
-            if constexpr (std::is_same<C, int64_t>::value) {
+            if constexpr (std::is_same<C, int64_t>::value && V == 4) {
                 if (o.access == kVector && count == V) {
                     const int4 f = *reinterpret_cast<const int4*>(static_cast<const int32_t*>(o.base) + at);
                     x[0] = f.x; x[1] = f.y; x[2] = f.z; x[3] = f.w;
@@ -279,7 +283,7 @@ __device__ __forceinline__ void load_operand(const EwOperand& o, int64_t at, int
 
 template <typename C, int V>
 __device__ __forceinline__ void store_result(const EwOperand& o, int64_t at, int count, const C* x) {
-    if constexpr (std::is_same<C, float>::value) {
+    if constexpr (std::is_same<C, float>::value && V >= 4) {
         if (o.access == kVector && count == V) {
             if (o.dtype == MHLO_DT_F32) {
 #pragma unroll
@@ -299,7 +303,7 @@ __device__ __forceinline__ void store_result(const EwOperand& o, int64_t at, int
             }
         }
     }
-    if constexpr (std::is_same<C, int64_t>::value) {
+    if constexpr (std::is_same<C, int64_t>::value && V == 4) {
         if (o.access == kVector && count == V && o.dtype == MHLO_DT_I32) {
             *reinterpret_cast<int4*>(static_cast<int32_t*>(o.base) + at) =
                 make_int4(static_cast<int>(x[0]), static_cast<int>(x[1]), static_cast<int>(x[2]), static_cast<int>(x[3]));
@@ -355,6 +359,7 @@ __device__ __forceinline__ void ew_apply(const EwParams& p, int op, double imm, 
         }
         if constexpr (std::is_same<C, float>::value) {
             switch (op) {
+                case MHLO_EW_POW: MHLO_EW_EACH(ew_pow(x, y))
                 case MHLO_EW_EXP: MHLO_EW_EACH(expf(x))
                 case MHLO_EW_TANH: MHLO_EW_EACH(tanhf(x))
                 case MHLO_EW_LOGISTIC: MHLO_EW_EACH(1.f / (1.f + expf(-x)))
@@ -477,23 +482,24 @@ constexpr int kProgramThreads = 128;
 
 template <typename C, int V>
 __global__ void __launch_bounds__(kProgramThreads) ew_program_kernel(const __grid_constant__ EwParams p) {
-    // slot s of a thread: V elements as V * sizeof(C) / 16 words of 16 bytes, word q at [s][q][thread]
+    // slot s of a thread: V elements as words of 16 bytes (or the one element), word q at [s][q][thread]
     extern __shared__ __align__(16) unsigned char slots[];
-    constexpr int W = V * static_cast<int>(sizeof(C)) / 16;
-    uint4* const mine = reinterpret_cast<uint4*>(slots) + threadIdx.x;
+    using Word = typename std::conditional<V == 1, C, uint4>::type;
+    constexpr int W = V * static_cast<int>(sizeof(C)) / static_cast<int>(sizeof(Word));
+    Word* const mine = reinterpret_cast<Word*>(slots) + threadIdx.x;
     auto put = [&](int s, const C* x) {
 #pragma unroll
         for (int q = 0; q < W; ++q) {
-            uint4 u;
-            memcpy(&u, x + q * (V / W), 16);
+            Word u;
+            memcpy(&u, x + q * (V / W), sizeof u);
             mine[(s * W + q) * kProgramThreads] = u;
         }
     };
     auto get = [&](int s, C* x) {
 #pragma unroll
         for (int q = 0; q < W; ++q) {
-            const uint4 u = mine[(s * W + q) * kProgramThreads];
-            memcpy(x + q * (V / W), &u, 16);
+            const Word u = mine[(s * W + q) * kProgramThreads];
+            memcpy(x + q * (V / W), &u, sizeof u);
         }
     };
     const int64_t step = static_cast<int64_t>(gridDim.x) * kProgramThreads;
@@ -603,7 +609,7 @@ void fill_operand(EwOperand* o, void* base, int dtype, const EwShape& s, int k, 
     o->dtype = dtype;
     o->inner = s.stride[k][inner];
     // a 16-byte access needs a dense innermost dimension and every row on the grid of V elements
-    bool on_grid = o->inner == 1 && (reinterpret_cast<uintptr_t>(base) % static_cast<uintptr_t>(vec * es < 16 ? vec * es : 16)) == 0;
+    bool on_grid = vec > 1 && o->inner == 1 && (reinterpret_cast<uintptr_t>(base) % static_cast<uintptr_t>(vec * es < 16 ? vec * es : 16)) == 0;
     for (int d = 0; d < inner; ++d) {
         o->outer[d] = s.stride[k][d];
         on_grid = on_grid && s.stride[k][d] % vec == 0;
@@ -659,6 +665,22 @@ int assign_slots(const mhlo_cuda_ew_inst* prog, int n_inputs, int n_insts, EwIns
         }
     }
     return high;
+}
+
+// Up to this many elements (two CTAs of 256 threads per SM) a thread takes one element of anything but a short program of cheap
+// float operators over dense operands, whose 16-byte accesses are worth more. 10000 elements, V elements a thread -> one: bf16 power
+// 5.1 -> 3.2 us, f64 exponential 3.6 -> 2.6, i32 divide 3.6 -> 3.0, f32 compare 3.4 -> 2.6, sixteen bf16 instructions 12.5 -> 9.0;
+// f32 add 2.1 -> 2.6. At 320000 the vectors lead everywhere.
+constexpr int64_t kFewElements = kNumSMs * 512;
+
+// Float operators that ew_apply has inline: a few instructions each.
+bool inlined_op(int op) {
+    switch (op) {
+        case MHLO_EW_COPY: case MHLO_EW_IMM: case MHLO_EW_ADD: case MHLO_EW_SUB: case MHLO_EW_MUL: case MHLO_EW_DIV: case MHLO_EW_MAX: case MHLO_EW_MIN:
+        case MHLO_EW_NEG: case MHLO_EW_ABS: case MHLO_EW_SQRT: case MHLO_EW_RSQRT: case MHLO_EW_SELECT: case MHLO_EW_RELU: case MHLO_EW_EXP:
+        case MHLO_EW_TANH: case MHLO_EW_LOGISTIC: case MHLO_EW_SILU: case MHLO_EW_GELU_TANH: case MHLO_EW_ROUND_TO: return true;
+        default: return false;
+    }
 }
 
 template <typename C, int V>
@@ -756,11 +778,28 @@ static int elementwise_impl(const mhlo_cuda_view* inputs, int32_t n_inputs, cons
             else insts[k].imm = d;
         }
     // eight elements per thread where a 16-bit (or narrower) tensor takes part, four otherwise: 16 bytes of the narrower type
-    const int vec = !any_f64 && any_float && narrow ? 8 : 4;
+    int vec = !any_f64 && any_float && narrow ? 8 : 4;
     EwParams p;
     memset(&p, 0, sizeof p);
-    for (int k = 0; k < n_inputs; ++k) fill_operand(&p.in[k], const_cast<void*>(inputs[k].base), inputs[k].dtype, shape, k, vec);
-    fill_operand(&p.out, out_dev, out_dtype, shape, n_inputs, vec);
+    auto lay_out = [&] {
+        auto wide = [](const EwOperand& o) { return o.access == kVector && is_float_dt(o.dtype); };
+        bool all = true;  // operands move in 16-byte accesses
+        for (int k = 0; k < n_inputs; ++k) {
+            fill_operand(&p.in[k], const_cast<void*>(inputs[k].base), inputs[k].dtype, shape, k, vec);
+            all = all && (p.in[k].access == kSplat || wide(p.in[k]));
+        }
+        fill_operand(&p.out, out_dev, out_dtype, shape, n_inputs, vec);
+        return all && wide(p.out);
+    };
+    const bool in_vectors = lay_out();
+    if (n <= kFewElements) {
+        bool cheap = in_vectors && !any_f64 && (vec == 4 || n_insts == 1);
+        for (int k = 0; k < n_insts; ++k) cheap = cheap && inlined_op(insts[k].op);
+        if (!cheap) {
+            vec = 1;
+            lay_out();
+        }
+    }
     if (p.out.access == kSplat) p.out.access = kStrided;  // one innermost element
     p.n_outer = shape.rank - 1;
     p.per_row = (shape.extent[p.n_outer] + vec - 1) / vec;
@@ -787,11 +826,14 @@ static int elementwise_impl(const mhlo_cuda_view* inputs, int32_t n_inputs, cons
     if (n_insts == 1 && n_inputs <= 3 && in_order) {
         p.prog[0].op = static_cast<int16_t>(first.op);
         p.prog[0].imm = first.imm;
+        if (vec == 1) return any_f64 ? launch_single<double, 1>(p, s) : !any_float ? launch_single<int64_t, 1>(p, s) : launch_single<float, 1>(p, s);
         if (any_f64) return launch_single<double, 4>(p, s);
         if (!any_float) return launch_single<int64_t, 4>(p, s);
         return vec == 8 ? launch_single<float, 8>(p, s) : launch_single<float, 4>(p, s);
     }
     const int slots = assign_slots(insts, n_inputs, n_insts, p.prog);
+    if (vec == 1)
+        return any_f64 ? launch_program<double, 1>(p, slots, s) : !any_float ? launch_program<int64_t, 1>(p, slots, s) : launch_program<float, 1>(p, slots, s);
     if (any_f64) return launch_program<double, 4>(p, slots, s);
     if (!any_float) return launch_program<int64_t, 4>(p, slots, s);
     return vec == 8 ? launch_program<float, 8>(p, slots, s) : launch_program<float, 4>(p, slots, s);

@@ -54,3 +54,40 @@ def test_operands_may_share_registers(n_inputs, dt):
             assert torch.equal(out, w), (name, a, b, c)
             run(x, [(OP["NEG"], 0, 0, 0, 0.0), (OP[name], a, b, c, 0.0)], out)
             assert torch.equal(out, w), (name, a, b, c, "second instruction")
+
+
+# one element per thread up to 75776 elements, 4 or 8 beyond; short programs of cheap float operators keep their vectors
+@pytest.mark.parametrize("dt", [torch.float32, torch.bfloat16, torch.float64, torch.int32, torch.int8, torch.int64])
+@pytest.mark.parametrize("shape,view", [((1,), None), ((7,), None), ((1001,), "shift"), ((75776,), None), ((75777,), None), ((37, 2049), "columns"),
+                                        ((300, 257), "transpose"), ((5, 1, 7, 9), None), ((1000, 3), "row")])
+def test_elements_per_thread(shape, view, dt):
+    g = torch.Generator().manual_seed(len(shape))
+    n = 1
+    for e in shape:
+        n *= e
+
+    def tensor(k):
+        x = torch.randint(-9, 10, (n + 1,), generator=g).to(dt).cuda()
+        if view == "shift":
+            return x[1:].view(shape)
+        if view == "columns":
+            return torch.cat([x, x])[:2 * n].view(shape[0], 2 * shape[1])[:, ::2]
+        if view == "transpose":
+            return x[:n].view(shape[::-1]).t()
+        if view == "row" and k == 1:
+            return x[:shape[-1]].expand(shape)
+        return x[:n].view(shape)
+
+    x, y = tensor(0), tensor(1)
+    out = torch.empty(shape, dtype=dt, device="cuda")
+    flags = torch.empty(shape, dtype=torch.bool, device="cuda")
+    run([x, y], [(OP["SUB"], 0, 1, 0, 0.0)], out)
+    assert torch.equal(out, x - y)
+    run([x, y], [(OP["CMP_LT"], 0, 1, 0, 0.0)], flags)
+    assert torch.equal(flags, x < y)
+    # a value kept for the last instruction, one used at once, and a coordinate
+    prog = [(OP["MUL"], 0, 1, 0, 0.0), (OP["NEG"], 2, 2, 2, 0.0), (OP["IOTA"], 0, 0, 0, float(len(shape) - 1)), (OP["ADD"], 3, 0, 0, 0.0), (OP["MAX"], 5, 2, 0, 0.0)]
+    run([x, y], prog, out)
+    prod = (x * y) if dt not in (torch.bfloat16, torch.int8) else (x.to(torch.int32) * y.to(torch.int32)).to(torch.float64)
+    want = torch.maximum(-prod + x.to(prod.dtype), prod)
+    assert torch.equal(out, want.to(dt) if dt != torch.int8 else want.to(torch.int64).to(torch.int8))

@@ -12,6 +12,8 @@
 // One element per iteration with 64-bit divisions and a dynamically indexed register file in local memory, the former
 // shape of this kernel, ran a seven-instruction chain over 4.2 M bf16 elements in 75 us and a scalar multiply over
 // 134 M bf16 elements in 208 us (HBM time: 4 us and 82 us).
+#include <atomic>
+
 #include "common.cuh"
 #include "element_access.cuh"
 
@@ -700,9 +702,19 @@ int launch_single(const EwParams& p, cudaStream_t s) {
 template <typename C, int V>
 int launch_program(const EwParams& p, int n_slots, cudaStream_t s) {
     const size_t smem = static_cast<size_t>(n_slots) * V * sizeof(C) * kProgramThreads;  // at most 40 slots x 4 KB
-    if (smem > 48 * 1024)
-        MHLO_CUDA_TRY(cudaFuncSetAttribute(ew_program_kernel<C, V>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)),
-                      MHLO_CUDA_EXECUTION_FAILED);
+    if (smem > 48 * 1024) {
+        // The limit belongs to the kernel and not to a launch: once per device, for the largest program there is, so that one
+        // thread's setting is never too small for what another is about to launch.
+        constexpr int kMost = (MHLO_CUDA_EW_MAX_INPUTS + MHLO_CUDA_EW_MAX_INSTS) * V * static_cast<int>(sizeof(C)) * kProgramThreads;
+        static std::atomic<uint64_t> configured{0};
+        int dev = 0;
+        MHLO_CUDA_TRY(cudaGetDevice(&dev), MHLO_CUDA_NO_DEVICE);
+        const uint64_t bit = uint64_t{1} << (dev & 63);
+        if (!(configured.load(std::memory_order_acquire) & bit)) {
+            MHLO_CUDA_TRY(cudaFuncSetAttribute(ew_program_kernel<C, V>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMost), MHLO_CUDA_EXECUTION_FAILED);
+            configured.fetch_or(bit, std::memory_order_release);
+        }
+    }
     const int64_t blocks = (p.n_vec + kProgramThreads - 1) / kProgramThreads;
     const int grid = static_cast<int>(blocks < kNumSMs * 64 ? blocks : kNumSMs * 64);
     ew_program_kernel<C, V><<<grid, kProgramThreads, smem, s>>>(p);

@@ -91,3 +91,46 @@ def test_elements_per_thread(shape, view, dt):
     prod = (x * y) if dt not in (torch.bfloat16, torch.int8) else (x.to(torch.int32) * y.to(torch.int32)).to(torch.float64)
     want = torch.maximum(-prod + x.to(prod.dtype), prod)
     assert torch.equal(out, want.to(dt) if dt != torch.int8 else want.to(torch.int64).to(torch.int8))
+
+
+def test_large_programs_from_several_threads():
+    """Programs that keep 15, 20 and 22 values (60, 80 and 88 KB of shared memory a CTA), launched by three threads at the same time."""
+    import threading
+
+    n, failures = 80000, []
+
+    def kept(count):
+        """count results of x * x chained by sums, all of them read again at the end."""
+        prog = [(OP["MUL"], 0, 0, 0, 0.0)] + [(OP["ADD"], k, 0, 0, 0.0) for k in range(1, count)]
+        total = count
+        for k in range(1, 32 - count + 1):
+            prog.append((OP["ADD"], total, k, 0, 0.0))
+            total = count + k
+        return prog
+
+    def expected(x, prog):
+        regs = [x]
+        for op, a, b, _c, _imm in prog:
+            regs.append(regs[a] * regs[b] if op == OP["MUL"] else regs[a] + regs[b])
+        return regs[-1]
+
+    def work(count, extra):
+        try:
+            with torch.cuda.stream(torch.cuda.Stream()):
+                x = torch.full((n,), 0.5, device="cuda")
+                y = torch.zeros(n, dtype=torch.bfloat16, device="cuda")
+                inputs, prog = [x] + [y] * extra, [(op, a + (extra if a else 0), b + (extra if b else 0), 0, imm) for op, a, b, _c, imm in kept(count)]
+                out = torch.empty(n, device="cuda")
+                for _ in range(1500):
+                    run(inputs, prog, out)
+                torch.cuda.current_stream().synchronize()
+                assert torch.equal(out, expected(x, kept(count)))
+        except Exception as e:  # noqa: BLE001 - reported below, from the main thread
+            failures.append(e)
+
+    threads = [threading.Thread(target=work, args=a) for a in ((16, 3), (18, 7), (12, 2))]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not failures, failures[0]

@@ -46,9 +46,14 @@ cudaMemPool_t scratch_pool(bool create) {
         props.location.type = cudaMemLocationTypeDevice;
         props.location.id = dev;
         cudaMemPool_t pool = nullptr;
-        if (cudaMemPoolCreate(&pool, &props) != cudaSuccess) { cudaGetLastError(); return nullptr; }
+        // The first request may come inside a stream capture, which creating a pool would otherwise invalidate.
+        cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+        cudaThreadExchangeStreamCaptureMode(&mode);
+        const bool made = cudaMemPoolCreate(&pool, &props) == cudaSuccess;
         uint64_t kept = kScratchKept;
-        cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &kept);
+        if (made) cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &kept);
+        cudaThreadExchangeStreamCaptureMode(&mode);
+        if (!made) { cudaGetLastError(); return nullptr; }
         g_scratch_pool[dev] = pool;
     }
     return g_scratch_pool[dev];

@@ -23,7 +23,7 @@ struct PackJobs {
 
 // A warp per row, or per 512 columns of a longer row, consecutive lanes on consecutive columns (64 bytes per load and store
 // instruction). 512 columns are 16 trips of a warp: with whole rows, an operand of few long rows kept few warps busy
-// ([768, 50257], the weights of a product of one row: 543 us with it, 92 in pieces).
+// ([768, 50257], the weights of a product of one row: 543 us with it, 89 in pieces).
 constexpr int kPackColumns = 512;
 
 __global__ void __launch_bounds__(256) pack_operands_kernel(const __grid_constant__ PackJobs jobs) {

@@ -229,7 +229,7 @@ int32_t mhlo_b200_executable_output_is_complex(MHLOExecutableRef executable, int
 MHLOStatusCode mhlo_b200_buffer_to_host_async(MHLOBufferRef buffer, void* out_data, size_t data_size, void (*done)(void*), void* user);
 /* Enqueues the program on `stream` (a cudaStream_t) reading/writing caller-owned dense device tensors of the
  * executable's declared types. Does not synchronise; the only device allocations are stream-ordered scratch of split
- * reductions. On a non-default stream, repeated calls with the same addresses replay a recorded CUDA graph. */
+ * reductions and of products whose 16-bit operands lie off the 16-byte grid. On a non-default stream, repeated calls with the same addresses replay a recorded CUDA graph. */
 MHLOStatusCode mhlo_b200_execute_on_device(MHLOExecutableRef executable, const void* const* input_ptrs,
                                            void* const* output_ptrs, void* stream);
 

@@ -551,8 +551,10 @@ enum {
  *   C[b0,b1,m,n] = act( sum_k A(b0,b1,m,k) * B(b0,b1,k,n) + bias[n] ),  C dense row-major, fp32 accumulation.
  * a_strides / b_strides = {batch0, batch1, row, col} element strides, so transposed and batch-interleaved
  * operands need no copy. bias_dev ([n], dtype = out_dtype) may be NULL. BF16/F16 operands whose rows or columns
- * are contiguous and 16-byte aligned run on the tcgen05 tensor-core kernel (TMA-fed, TMEM accumulators);
- * everything else takes the general-layout kernel behind mhlo_cuda_dot_strided. Replaces kernel_matmul (MPP and
+ * are contiguous and 16-byte aligned run on the tcgen05 tensor-core kernel (TMA-fed, TMEM accumulators); BF16/F16
+ * operands that are not are first copied onto that grid where it pays, into stream-ordered scratch of the library's own
+ * memory pool (inside a stream capture: nodes of the graph). F32 runs on packed FMAs. Everything else, and a product whose
+ * scratch cannot be had, takes the general-layout kernel behind mhlo_cuda_dot_strided, which never allocates. Replaces kernel_matmul (MPP and
  * simdgroup variants, Sources/MetalHLOCore/Compiler/CodeGenerator.swift:3463-3886), kernel_matmul_bias_act
  * (:4797-4850) and the semantics of FusedMatMulBiasActivationHandler
  * (Sources/MetalHLOCore/Compiler/CustomCallHandlers.swift:927-1073).
@@ -666,8 +668,8 @@ int mhlo_cuda_device_error_take(int32_t* out_code);
  * exactly as the contraction kernels record an expired wait.
  */
 int mhlo_cuda_debug_store_device_error(int32_t which, int32_t code);
-/* Test hook of the allocator's failure path: the next `count` mhlo_cuda_alloc calls return MHLO_CUDA_BUFFER_FAILED
- * without reaching the driver (0 switches it off). */
+/* Test hook of the allocator's failure path: the next `count` requests for device memory (mhlo_cuda_alloc, the scratch
+ * of a call) fail with MHLO_CUDA_BUFFER_FAILED without reaching the driver (0 switches it off). */
 int mhlo_cuda_debug_refuse_allocs(int32_t count);
 int mhlo_cuda_debug_wait_expiry_probe(uint64_t limit_ns, mhlo_cuda_stream_t stream);
 

@@ -95,9 +95,9 @@ bool gemm_pack_launch(GemmProblem p, cudaStream_t stream, int* status) {
     if (n == 0 || !gemm_tc_supported(p) || blocks[0] + blocks[1] > 0x7fffffff) return false;
     void* scratch = nullptr;
     int st = scratch_alloc(&scratch, bytes, stream);
-    if (st != MHLO_CUDA_OK) {
-        *status = st;
-        return true;
+    if (st != MHLO_CUDA_OK) {  // no memory to pack into: the general kernel reads the operands where they are
+        clear_error();
+        return false;
     }
     for (int i = 0; i < n; ++i) {
         jobs.job[i].dst = reinterpret_cast<uint16_t*>(static_cast<char*>(scratch) + offset[i]);

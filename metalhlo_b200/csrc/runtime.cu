@@ -60,12 +60,25 @@ cudaMemPool_t scratch_pool(bool create) {
 }
 }  // namespace
 
+// Test hook: the next requests for device memory are refused before they reach the driver.
+static std::atomic<int> g_refuse_allocs{0};
+
+static bool refused() {
+    int left = g_refuse_allocs.load();
+    while (left > 0 && !g_refuse_allocs.compare_exchange_weak(left, left - 1)) {}
+    return left > 0;
+}
+
 int scratch_alloc(void** out, size_t bytes, cudaStream_t stream) {
     *out = nullptr;
+    if (refused()) return fail(MHLO_CUDA_BUFFER_FAILED, "scratch of %zu bytes refused (test hook)", bytes);
     cudaMemPool_t pool = scratch_pool(true);
     if (pool == nullptr) return fail(MHLO_CUDA_BUFFER_FAILED, "scratch of %zu bytes: no memory pool", bytes);
-    MHLO_CUDA_TRY(cudaMallocFromPoolAsync(out, bytes, pool, stream), MHLO_CUDA_BUFFER_FAILED);
-    return MHLO_CUDA_OK;
+    const cudaError_t e = cudaMallocFromPoolAsync(out, bytes, pool, stream);
+    if (e == cudaSuccess) return MHLO_CUDA_OK;
+    cudaGetLastError();  // a caller that goes on without scratch must not find it behind its own launch
+    *out = nullptr;
+    return fail(MHLO_CUDA_BUFFER_FAILED, "scratch of %zu bytes: %s", bytes, cudaGetErrorString(e));
 }
 
 int scratch_free(void* p, cudaStream_t stream) {
@@ -214,11 +227,8 @@ int mhlo_cuda_stream_sync(mhlo_cuda_stream_t stream) {
     return MHLO_CUDA_OK;
 }
 
-// Test hook: the next `count` device allocations are refused before they reach the driver.
-static std::atomic<int> g_refuse_allocs{0};
-
 int mhlo_cuda_debug_refuse_allocs(int32_t count) {
-    g_refuse_allocs.store(count < 0 ? 0 : count);
+    mhlo::g_refuse_allocs.store(count < 0 ? 0 : count);
     return MHLO_CUDA_OK;
 }
 
@@ -226,14 +236,14 @@ int mhlo_cuda_alloc(size_t bytes, void** out_dev) {
     if (!out_dev) return fail(MHLO_CUDA_INVALID_ARGUMENT, "alloc: null output");
     *out_dev = nullptr;
     if (bytes == 0) return MHLO_CUDA_OK;
-    int left = g_refuse_allocs.load();
-    while (left > 0 && !g_refuse_allocs.compare_exchange_weak(left, left - 1)) {}
-    if (left > 0) return fail(MHLO_CUDA_BUFFER_FAILED, "alloc of %zu bytes refused (test hook)", bytes);
+    if (mhlo::refused()) return fail(MHLO_CUDA_BUFFER_FAILED, "alloc of %zu bytes refused (test hook)", bytes);
     if (cudaMalloc(out_dev, bytes) == cudaSuccess) return MHLO_CUDA_OK;
     cudaGetLastError();
     mhlo::scratch_trim();  // what the scratch pool keeps goes back to the driver before the second try
-    MHLO_CUDA_TRY(cudaMalloc(out_dev, bytes), MHLO_CUDA_BUFFER_FAILED);
-    return MHLO_CUDA_OK;
+    const cudaError_t e = cudaMalloc(out_dev, bytes);
+    if (e == cudaSuccess) return MHLO_CUDA_OK;
+    cudaGetLastError();
+    return fail(MHLO_CUDA_BUFFER_FAILED, "alloc of %zu bytes: %s", bytes, cudaGetErrorString(e));
 }
 
 int mhlo_cuda_free(void* dev) {

@@ -160,3 +160,28 @@ def test_fp32_results_of_other_products_have_fp32_sums(m, n, k, shared, split):
     want = a.double() @ b.double()
     # a running fp32 sum of k independent terms errs by about sqrt(k) / 2 roundings of the result's size; the tensor cores by 3e-6 at 4096
     assert float((got.double() - want).norm() / want.norm()) <= 2.0 ** -24 * (1 + math.sqrt(k) / 2)
+
+
+def test_product_without_scratch():
+    """Off the grid with no memory to pack into: the general kernel takes it, and nothing of the refusal stays behind."""
+    from metalhlo_b200 import cuda
+
+    g = torch.Generator().manual_seed(11)
+    a, b = torch.randn(130, 333, generator=g).half().cuda(), (torch.randn(333, 201, generator=g) / 18).half().cuda()
+    bias = torch.randn(201, generator=g).half().cuda()
+    want, magnitude = product(a, b, "f16")
+    for _ in range(2):
+        try:
+            assert cuda.lib.mhlo_cuda_debug_refuse_allocs(1) == 0
+            close(cuda.gemm(a, b), want, 333, magnitude)
+            assert cuda.last_error() == ""
+        finally:
+            cuda.lib.mhlo_cuda_debug_refuse_allocs(0)
+    cuda.lib.mhlo_cuda_debug_refuse_allocs(1)
+    try:
+        got = cuda.gemm(a, b, bias=bias, epilogue="relu")
+    finally:
+        cuda.lib.mhlo_cuda_debug_refuse_allocs(0)
+    # the product is rounded before the bias there
+    assert float((got.double() - torch.relu(want + bias.double())).abs().max()) <= 2 * 2.0 ** -11 * float(want.abs().max() + bias.abs().max())
+    close(cuda.gemm(a, b), want, 333, magnitude)

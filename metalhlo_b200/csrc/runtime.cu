@@ -88,6 +88,9 @@ int scratch_free(void* p, cudaStream_t stream) {
 
 void scratch_trim() {
     if (cudaMemPool_t pool = scratch_pool(false)) cudaMemPoolTrimTo(pool, 0);
+    int dev = 0;  // and what the device keeps for graphs that have been destroyed
+    if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGraphMemTrim(dev);
+    cudaGetLastError();
 }
 
 }  // namespace mhlo

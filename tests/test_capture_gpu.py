@@ -50,3 +50,30 @@ def test_first_scratch_of_a_process_under_capture(program):
     root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
     r = subprocess.run([sys.executable, "-c", program], cwd=root, capture_output=True, text=True, timeout=300)
     assert r.returncode == 0 and "replayed" in r.stdout, r.stderr[-2000:]
+
+
+def test_scratch_of_destroyed_graphs_goes_back_when_memory_runs_short():
+    import ctypes as C
+    import gc
+
+    import torch
+
+    from metalhlo_b200 import cuda
+
+    a, b = torch.zeros(8192, 20001, dtype=torch.float16, device="cuda"), torch.zeros(20001, 8191, dtype=torch.float16, device="cuda")
+    out = torch.empty(8192, 8191, dtype=torch.float16, device="cuda")
+    graph, stream = torch.cuda.CUDAGraph(), torch.cuda.Stream()
+    stream.wait_stream(torch.cuda.current_stream())
+    before = torch.cuda.mem_get_info()[0]
+    with torch.cuda.graph(graph, stream=stream):
+        cuda.gemm(a, b, out=out)  # about 650 MB of packed operands, owned by the graph
+    graph.replay()
+    torch.cuda.synchronize()
+    del graph
+    gc.collect()
+    p = C.c_void_p()
+    assert cuda.lib.mhlo_cuda_alloc(1 << 50, C.byref(p)) == 6 and not p.value  # more than there is
+    assert torch.cuda.mem_get_info()[0] >= before - (64 << 20)
+    small = torch.zeros(4, device="cuda")
+    cuda.check(cuda.lib.mhlo_cuda_memset(small.data_ptr(), 1, 16, torch.cuda.current_stream().cuda_stream))  # nothing of the refusal is left
+    torch.cuda.synchronize()

@@ -788,7 +788,8 @@ typedef void* mhlo_cuda_plan_t;
  * FusedOp.fusedOpTypeFromCustomCall (Compiler/IntegrationTypes.swift:471-600) on the CUDA side. MHLO_CUDA_UNSUPPORTED
  * when the library has no such kernel for the dtype. */
 int mhlo_cuda_kernel_lookup(const char* fused_op_kind, int32_t dtype, int32_t* out_kernel);
-/* Validates the ops, allocates the arena and uploads the constant pool (either may be empty). The caller owns the plan. */
+/* Validates the ops, allocates the arena and the scratch of products whose 16-bit operands lie off the 16-byte grid (without
+ * that scratch they run on the general kernel), and uploads the constant pool. Each may be empty. The caller owns the plan. */
 int mhlo_cuda_plan_create(const mhlo_cuda_plan_op* ops, int32_t n_ops, int32_t n_inputs, int32_t n_outputs, int64_t arena_bytes,
                           const void* constants_host, int64_t constant_bytes, mhlo_cuda_plan_t* out_plan);
 /* Enqueues every op in order on `stream`; inputs / outputs are device pointers. No allocation, no synchronisation. */

@@ -76,7 +76,17 @@ bool gemm_tc_supported(const GemmProblem& p);
 int gemm_tc_launch(const GemmProblem& p, cudaStream_t stream);
 // 16-bit operands that have to be copied onto the 16-byte grid first. False: not a product this applies to, nothing was queued and
 // the general kernel takes it; true: *status is the result of the launches.
-bool gemm_pack_launch(GemmProblem p, cudaStream_t stream, int* status);
+// scratch: the caller's own memory (256-byte aligned; too little: false), null: from the library's pool.
+struct PackScratch {
+    void* base;
+    size_t bytes;
+};
+bool gemm_pack_launch(GemmProblem p, const PackScratch* scratch, cudaStream_t stream, int* status);
+size_t gemm_pack_bytes(GemmProblem p);  // what that takes when both operands start on the grid; 0: nothing is packed
+// mhlo_cuda_gemm_tuned with the scratch of packed operands from the caller.
+int gemm_entry(int32_t in_dtype, int32_t out_dtype, const void* a, const int64_t* a_strides, const void* b, const int64_t* b_strides, void* c,
+               int64_t batch0, int64_t batch1, int64_t m, int64_t n, int64_t k, const void* bias, int32_t epilogue,
+               const mhlo_cuda_gemm_tuning* tuning, const PackScratch* scratch, cudaStream_t stream);
 // fp32 operands and results on the FMA units, any strides.
 bool gemm_fp32_supported(const GemmProblem& p);
 int gemm_fp32_launch(const GemmProblem& p, cudaStream_t stream);

@@ -96,6 +96,65 @@ int launch_attention_rows(const void* q, const void* k, const void* v, const voi
 }  // namespace
 }  // namespace mhlo
 
+namespace mhlo {
+namespace {
+// Whether the tensor-core epilogue takes the CUDA library's tanhf and expf rather than the hardware's approximations (2^-11
+// relative). The approximations are for products whose epilogue has to keep up with the MMAs: at least 64 x 64 results, K
+// above 1, operands read in place, one matrix each per batch entry. Everything else (and every packed product) is bound elsewhere
+// and keeps fp32 precision.
+bool exact_activation(const GemmProblem& p) {
+    const bool shared = (p.batch0 > 1 && (p.as[0] == 0 || p.bs[0] == 0)) || (p.batch1 > 1 && (p.as[1] == 0 || p.bs[1] == 0));
+    return p.m * p.n < 64 * 64 || p.k == 1 || shared;
+}
+}  // namespace
+
+int gemm_entry(int32_t in_dtype, int32_t out_dtype, const void* a_dev, const int64_t* a_strides, const void* b_dev, const int64_t* b_strides,
+               void* c_dev, int64_t batch0, int64_t batch1, int64_t m, int64_t n, int64_t k, const void* bias_dev, int32_t epilogue,
+               const mhlo_cuda_gemm_tuning* tuning, const PackScratch* scratch, cudaStream_t stream) {
+    if (tuning) {
+        if ((tuning->tile_n != 0 && tuning->tile_n != 128 && tuning->tile_n != 256) || tuning->stages < 0 || tuning->stages > 8 ||
+            tuning->stages == 1 || tuning->cta_group < 0 || tuning->cta_group > 2 || (tuning->cta_group == 2 && tuning->tile_n == 128))
+            return fail(MHLO_CUDA_INVALID_ARGUMENT, "gemm: tuning {tile_n %d, stages %d, cta_group %d} is not a configuration of the kernel",
+                        tuning->tile_n, tuning->stages, tuning->cta_group);
+    }
+    if (epilogue < MHLO_EPILOGUE_NONE || epilogue > MHLO_EPILOGUE_SIGMOID)
+        return fail(MHLO_CUDA_INVALID_ARGUMENT, "gemm: unknown epilogue %d", epilogue);
+    if (!a_strides || !b_strides) return fail(MHLO_CUDA_INVALID_ARGUMENT, "gemm: null strides");
+    GemmProblem p;
+    p.a = a_dev; p.b = b_dev; p.c = c_dev; p.bias = bias_dev;
+    for (int i = 0; i < 4; ++i) { p.as[i] = a_strides[i]; p.bs[i] = b_strides[i]; }
+    p.batch0 = batch0; p.batch1 = batch1; p.m = m; p.n = n; p.k = k;
+    p.in_dtype = in_dtype; p.out_dtype = out_dtype; p.epilogue = epilogue;
+    if (tuning) { p.tile_n = tuning->tile_n; p.stages = tuning->stages; p.cta_group = tuning->cta_group; p.split_k = tuning->split_k; }
+    p.exact_act = exact_activation(p);
+    // Those products keep fp32 sums too where the result is fp32: the tensor cores add more coarsely than FMAs (error against fp64 of
+    // [1021,1111] . [1111,3001] f16 -> f32 1.0e-6 and 4.4e-7, of K = 4096 3.5e-6 and 8.8e-7), which a 16-bit result does not show.
+    const bool fp32_sums = p.exact_act && out_dtype == MHLO_DT_F32;
+    if (!fp32_sums && gemm_tc_supported(p)) return gemm_tc_launch(p, stream);
+    if (gemm_fp32_supported(p)) return gemm_fp32_launch(p, stream);
+    int st = MHLO_CUDA_OK;
+    if (gemm_pack_launch(p, scratch, stream, &st)) return st;
+    st = mhlo_cuda_dot_strided(in_dtype, out_dtype, a_dev, a_strides, b_dev, b_strides, c_dev, batch0, batch1, m, n, k, stream);
+    if (st != MHLO_CUDA_OK || (bias_dev == nullptr && epilogue == MHLO_EPILOGUE_NONE)) return st;
+    // bias / activation as an in-place elementwise pass over C
+    mhlo_cuda_view in[2];
+    memset(in, 0, sizeof in);
+    const int64_t rows = batch0 * batch1 * m;
+    in[0].base = c_dev; in[0].dtype = out_dtype; in[0].rank = 2;
+    in[0].shape[0] = rows; in[0].shape[1] = n; in[0].stride[0] = n; in[0].stride[1] = 1;
+    in[1] = in[0];
+    in[1].base = bias_dev; in[1].stride[0] = 0;
+    mhlo_cuda_ew_inst prog[2];
+    int ni = 0, n_in = 1, cur = 0;
+    if (bias_dev != nullptr) { n_in = 2; prog[ni++] = {MHLO_EW_ADD, 0, 1, 0, 0.0}; cur = n_in; }
+    static const int act_op[] = {MHLO_EW_COPY, MHLO_EW_RELU, MHLO_EW_GELU_TANH, MHLO_EW_GELU_ERF, MHLO_EW_SILU, MHLO_EW_TANH, MHLO_EW_LOGISTIC};
+    if (epilogue != MHLO_EPILOGUE_NONE) { prog[ni] = {act_op[epilogue], cur, cur, cur, 0.0}; ++ni; }
+    const int64_t shape[2] = {rows, n};
+    return mhlo_cuda_elementwise(in, n_in, prog, ni, c_dev, out_dtype, shape, 2, stream);
+}
+
+}  // namespace mhlo
+
 using namespace mhlo;
 
 extern "C" {
@@ -170,61 +229,12 @@ int mhlo_cuda_gemm(int32_t in_dtype, int32_t out_dtype, const void* a_dev, const
                                 nullptr, stream);
 }
 
-namespace {
-// Whether the tensor-core epilogue takes the CUDA library's tanhf and expf rather than the hardware's approximations (2^-11
-// relative). The approximations are for products whose epilogue has to keep up with the MMAs: at least 64 x 64 results, K
-// above 1, operands read in place, one matrix each per batch entry. Everything else (and every packed product) is bound elsewhere
-// and keeps fp32 precision.
-bool exact_activation(const GemmProblem& p) {
-    const bool shared = (p.batch0 > 1 && (p.as[0] == 0 || p.bs[0] == 0)) || (p.batch1 > 1 && (p.as[1] == 0 || p.bs[1] == 0));
-    return p.m * p.n < 64 * 64 || p.k == 1 || shared;
-}
-}  // namespace
-
 int mhlo_cuda_gemm_tuned(int32_t in_dtype, int32_t out_dtype, const void* a_dev, const int64_t a_strides[4],
                          const void* b_dev, const int64_t b_strides[4], void* c_dev, int64_t batch0, int64_t batch1,
                          int64_t m, int64_t n, int64_t k, const void* bias_dev, int32_t epilogue,
                          const mhlo_cuda_gemm_tuning* tuning, mhlo_cuda_stream_t stream) {
-    if (tuning) {
-        if ((tuning->tile_n != 0 && tuning->tile_n != 128 && tuning->tile_n != 256) || tuning->stages < 0 || tuning->stages > 8 ||
-            tuning->stages == 1 || tuning->cta_group < 0 || tuning->cta_group > 2 || (tuning->cta_group == 2 && tuning->tile_n == 128))
-            return fail(MHLO_CUDA_INVALID_ARGUMENT, "gemm: tuning {tile_n %d, stages %d, cta_group %d} is not a configuration of the kernel",
-                        tuning->tile_n, tuning->stages, tuning->cta_group);
-    }
-    if (epilogue < MHLO_EPILOGUE_NONE || epilogue > MHLO_EPILOGUE_SIGMOID)
-        return fail(MHLO_CUDA_INVALID_ARGUMENT, "gemm: unknown epilogue %d", epilogue);
-    if (!a_strides || !b_strides) return fail(MHLO_CUDA_INVALID_ARGUMENT, "gemm: null strides");
-    GemmProblem p;
-    p.a = a_dev; p.b = b_dev; p.c = c_dev; p.bias = bias_dev;
-    for (int i = 0; i < 4; ++i) { p.as[i] = a_strides[i]; p.bs[i] = b_strides[i]; }
-    p.batch0 = batch0; p.batch1 = batch1; p.m = m; p.n = n; p.k = k;
-    p.in_dtype = in_dtype; p.out_dtype = out_dtype; p.epilogue = epilogue;
-    if (tuning) { p.tile_n = tuning->tile_n; p.stages = tuning->stages; p.cta_group = tuning->cta_group; p.split_k = tuning->split_k; }
-    p.exact_act = exact_activation(p);
-    // Those products keep fp32 sums too where the result is fp32: the tensor cores add more coarsely than FMAs (error against fp64 of
-    // [1021,1111] . [1111,3001] f16 -> f32 1.0e-6 and 4.4e-7, of K = 4096 3.5e-6 and 8.8e-7), which a 16-bit result does not show.
-    const bool fp32_sums = p.exact_act && out_dtype == MHLO_DT_F32;
-    if (!fp32_sums && gemm_tc_supported(p)) return gemm_tc_launch(p, static_cast<cudaStream_t>(stream));
-    if (gemm_fp32_supported(p)) return gemm_fp32_launch(p, static_cast<cudaStream_t>(stream));
-    int st = MHLO_CUDA_OK;
-    if (gemm_pack_launch(p, static_cast<cudaStream_t>(stream), &st)) return st;
-    st = mhlo_cuda_dot_strided(in_dtype, out_dtype, a_dev, a_strides, b_dev, b_strides, c_dev, batch0, batch1, m, n, k, stream);
-    if (st != MHLO_CUDA_OK || (bias_dev == nullptr && epilogue == MHLO_EPILOGUE_NONE)) return st;
-    // bias / activation as an in-place elementwise pass over C
-    mhlo_cuda_view in[2];
-    memset(in, 0, sizeof in);
-    const int64_t rows = batch0 * batch1 * m;
-    in[0].base = c_dev; in[0].dtype = out_dtype; in[0].rank = 2;
-    in[0].shape[0] = rows; in[0].shape[1] = n; in[0].stride[0] = n; in[0].stride[1] = 1;
-    in[1] = in[0];
-    in[1].base = bias_dev; in[1].stride[0] = 0;
-    mhlo_cuda_ew_inst prog[2];
-    int ni = 0, n_in = 1, cur = 0;
-    if (bias_dev != nullptr) { n_in = 2; prog[ni++] = {MHLO_EW_ADD, 0, 1, 0, 0.0}; cur = n_in; }
-    static const int act_op[] = {MHLO_EW_COPY, MHLO_EW_RELU, MHLO_EW_GELU_TANH, MHLO_EW_GELU_ERF, MHLO_EW_SILU, MHLO_EW_TANH, MHLO_EW_LOGISTIC};
-    if (epilogue != MHLO_EPILOGUE_NONE) { prog[ni] = {act_op[epilogue], cur, cur, cur, 0.0}; ++ni; }
-    const int64_t shape[2] = {rows, n};
-    return mhlo_cuda_elementwise(in, n_in, prog, ni, c_dev, out_dtype, shape, 2, stream);
+    return gemm_entry(in_dtype, out_dtype, a_dev, a_strides, b_dev, b_strides, c_dev, batch0, batch1, m, n, k, bias_dev, epilogue, tuning, nullptr,
+                      static_cast<cudaStream_t>(stream));
 }
 
 int mhlo_cuda_conv2d_nhwc(int32_t dtype, int32_t out_dtype, const void* x_dev, const void* filter_dev, void* out_dev, int64_t images,

@@ -64,51 +64,71 @@ void plan(PackJob* j, const void* p, int64_t* st, int64_t batch0, int64_t batch1
     st[3] = along_rows ? j->pitch : 1;
 }
 
-}  // namespace
+struct PackWork {
+    PackJobs jobs;
+    int count;
+    int packed[2];  // 0 = A, 1 = B
+    size_t bytes, offset[2];
+    int64_t blocks[2];
+};
 
-bool gemm_pack_launch(GemmProblem p, cudaStream_t stream, int* status) {
-    if ((p.in_dtype != MHLO_DT_F16 && p.in_dtype != MHLO_DT_BF16) || p.out_dtype != p.in_dtype) return false;  // fp32 results: fp32 sums
-    if (p.a == nullptr || p.b == nullptr || p.n_copies > 0 || p.m <= 0 || p.n <= 0 || p.k <= 0 || p.batch0 <= 0 || p.batch1 <= 0) return false;
-    if (p.m > 0x7fffffff || p.n > 0x7fffffff || p.k > 0x7fffffff || p.batch0 * p.batch1 > 0x7fffffff) return false;
+// Whether *p has operands to pack, and how; rewrites their strides and leaves their addresses null.
+bool lay_out(GemmProblem* p, PackWork* w) {
+    memset(w, 0, sizeof *w);
+    int n = 0;
+    if ((p->in_dtype != MHLO_DT_F16 && p->in_dtype != MHLO_DT_BF16) || p->out_dtype != p->in_dtype) return false;  // fp32 results: fp32 sums
+    if (p->a == nullptr || p->b == nullptr || p->n_copies > 0 || p->m <= 0 || p->n <= 0 || p->k <= 0 || p->batch0 <= 0 || p->batch1 <= 0) return false;
+    if (p->m > 0x7fffffff || p->n > 0x7fffffff || p->k > 0x7fffffff || p->batch0 * p->batch1 > 0x7fffffff) return false;
     // Copy and product cost 10 to 14 us before the first panel; the general kernel does 32 steps of K in 10, whatever the number of
     // results up to about eight million ([33,31] . [31,4001] 14 us packed, 10 there; with K = 63 14 and 15; [301,15] . [15,50257]
     // 37 and 46).
-    if (p.m * p.n * p.k < 64 * 1024 || (p.k <= 32 && p.m * p.n * p.batch0 * p.batch1 < int64_t{1} << 23)) return false;
-    PackJobs jobs;
-    memset(&jobs, 0, sizeof jobs);
-    int n = 0;
-    size_t bytes = 0, offset[2] = {0, 0};
-    const void** packed[2] = {nullptr, nullptr};
+    if (p->m * p->n * p->k < 64 * 1024 || (p->k <= 32 && p->m * p->n * p->batch0 * p->batch1 < int64_t{1} << 23)) return false;
     for (const bool is_a : {true, false}) {
-        const void** base = is_a ? &p.a : &p.b;
-        int64_t* st = is_a ? p.as : p.bs;
-        if (operand_on_grid(p, *base, st) && (is_a ? a_major(p) : b_major(p)) != kNoMajor) continue;
-        plan(&jobs.job[n], *base, st, p.batch0, p.batch1, is_a ? p.m : p.k, is_a ? p.k : p.n);
-        offset[n] = bytes;
-        packed[n] = base;
+        const void** base = is_a ? &p->a : &p->b;
+        int64_t* st = is_a ? p->as : p->bs;
+        if (operand_on_grid(*p, *base, st) && (is_a ? a_major(*p) : b_major(*p)) != kNoMajor) continue;
+        plan(&w->jobs.job[n], *base, st, p->batch0, p->batch1, is_a ? p->m : p->k, is_a ? p->k : p->n);
+        w->offset[n] = w->bytes;
+        w->packed[n] = is_a ? 0 : 1;
         *base = nullptr;  // on the grid; its address comes with the scratch
-        bytes += static_cast<size_t>(jobs.job[n].all_rows * jobs.job[n].pitch * 2 + 255) / 256 * 256;
+        w->bytes += static_cast<size_t>(w->jobs.job[n].all_rows * w->jobs.job[n].pitch * 2 + 255) / 256 * 256;
         ++n;
     }
-    const int64_t blocks[2] = {(jobs.job[0].all_rows * jobs.job[0].pieces + 7) / 8, (jobs.job[1].all_rows * jobs.job[1].pieces + 7) / 8};
-    p.exact_act = 1;
-    if (n == 0 || !gemm_tc_supported(p) || blocks[0] + blocks[1] > 0x7fffffff) return false;
-    void* scratch = nullptr;
-    int st = scratch_alloc(&scratch, bytes, stream);
+    for (int i = 0; i < 2; ++i) w->blocks[i] = (w->jobs.job[i].all_rows * w->jobs.job[i].pieces + 7) / 8;
+    w->count = n;
+    p->exact_act = 1;
+    if (n == 0 || !gemm_tc_supported(*p) || w->blocks[0] + w->blocks[1] > 0x7fffffff) return false;
+    return true;
+}
+
+}  // namespace
+
+size_t gemm_pack_bytes(GemmProblem p) {
+    PackWork w;
+    p.a = p.b = reinterpret_cast<const void*>(uintptr_t{256});  // any address on the grid
+    return lay_out(&p, &w) ? w.bytes : 0;
+}
+
+bool gemm_pack_launch(GemmProblem p, const PackScratch* own, cudaStream_t stream, int* status) {
+    PackWork w;
+    if (!lay_out(&p, &w)) return false;
+    void* scratch = own != nullptr ? own->base : nullptr;
+    if (own != nullptr && own->bytes < w.bytes) return false;
+    int st = own != nullptr ? MHLO_CUDA_OK : scratch_alloc(&scratch, w.bytes, stream);
     if (st != MHLO_CUDA_OK) {  // no memory to pack into: the general kernel reads the operands where they are
         clear_error();
         return false;
     }
-    for (int i = 0; i < n; ++i) {
-        jobs.job[i].dst = reinterpret_cast<uint16_t*>(static_cast<char*>(scratch) + offset[i]);
-        *packed[i] = jobs.job[i].dst;
+    for (int i = 0; i < w.count; ++i) {
+        w.jobs.job[i].dst = reinterpret_cast<uint16_t*>(static_cast<char*>(scratch) + w.offset[i]);
+        (w.packed[i] == 0 ? p.a : p.b) = w.jobs.job[i].dst;
     }
-    jobs.blocks0 = blocks[0];
-    pack_operands_kernel<<<static_cast<unsigned>(blocks[0] + blocks[1]), 256, 0, stream>>>(jobs);
+    w.jobs.blocks0 = w.blocks[0];
+    pack_operands_kernel<<<static_cast<unsigned>(w.blocks[0] + w.blocks[1]), 256, 0, stream>>>(w.jobs);
     const cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) st = fail(MHLO_CUDA_EXECUTION_FAILED, "launch of pack_operands failed: %s", cudaGetErrorString(e));
     if (st == MHLO_CUDA_OK) st = gemm_tc_launch(p, stream);
-    const int freed = scratch_free(scratch, stream);
+    const int freed = own != nullptr ? MHLO_CUDA_OK : scratch_free(scratch, stream);
     *status = st != MHLO_CUDA_OK ? st : freed;
     return true;
 }

@@ -14,7 +14,7 @@
 #include <string>
 #include <vector>
 
-#include "common.cuh"
+#include "contraction.cuh"
 
 namespace mhlo {
 namespace {
@@ -23,6 +23,8 @@ struct Plan {
     std::vector<mhlo_cuda_plan_op> ops;
     void* arena = nullptr;
     void* constants = nullptr;
+    void* scratch = nullptr;  // for the operands that a product packs; one product at a time, as the ops run in stream order
+    size_t scratch_bytes = 0;
     int64_t arena_bytes = 0, constant_bytes = 0;
     int32_t n_inputs = 0, n_outputs = 0;
     int device = 0;
@@ -56,6 +58,17 @@ const void* resolve(const Plan& p, const mhlo_cuda_binding& b, const void* const
     }
 }
 
+// Scratch that a product of the plan packs its operands into, as far as the strides say (the addresses come with the call).
+size_t pack_bytes(const mhlo_cuda_plan_op& op) {
+    GemmProblem g;
+    g.a = g.b = g.c = nullptr;
+    g.bias = nullptr;
+    for (int i = 0; i < 4; ++i) { g.as[i] = op.strides[i]; g.bs[i] = op.strides[4 + i]; }
+    g.batch0 = op.dims[0]; g.batch1 = op.dims[1]; g.m = op.dims[2]; g.n = op.dims[3]; g.k = op.dims[4];
+    g.in_dtype = op.dtype; g.out_dtype = op.out_dtype; g.epilogue = op.flags[0];
+    return gemm_pack_bytes(g);
+}
+
 int run_op(const Plan& p, const mhlo_cuda_plan_op& op, const void* const* inputs, void* const* outputs, mhlo_cuda_stream_t stream) {
     const void* a[6] = {nullptr, nullptr, nullptr, nullptr, nullptr, nullptr};
     for (int i = 0; i < 6; ++i) a[i] = resolve(p, op.args[i], inputs, outputs);
@@ -72,8 +85,9 @@ int run_op(const Plan& p, const mhlo_cuda_plan_op& op, const void* const* inputs
         case MHLO_CUDA_KERNEL_GEMM: {
             mhlo_cuda_gemm_tuning t{op.tuning[0], op.tuning[1], op.tuning[2], 0};
             const bool tuned = op.tuning[0] || op.tuning[1] || op.tuning[2];
-            return mhlo_cuda_gemm_tuned(op.dtype, op.out_dtype, a[0], op.strides, a[1], op.strides + 4, out(3), op.dims[0], op.dims[1], op.dims[2],
-                                        op.dims[3], op.dims[4], a[2], op.flags[0], tuned ? &t : nullptr, stream);
+            const PackScratch scratch{p.scratch, p.scratch_bytes};
+            return gemm_entry(op.dtype, op.out_dtype, a[0], op.strides, a[1], op.strides + 4, out(3), op.dims[0], op.dims[1], op.dims[2], op.dims[3],
+                              op.dims[4], a[2], op.flags[0], tuned ? &t : nullptr, &scratch, static_cast<cudaStream_t>(stream));
         }
         case MHLO_CUDA_KERNEL_ATTENTION: {
             mhlo_cuda_attention_tuning t{op.tuning[0], {0, 0, 0}};
@@ -161,6 +175,12 @@ int mhlo_cuda_plan_create(const mhlo_cuda_plan_op* ops, int32_t n_ops, int32_t n
     if (st == MHLO_CUDA_OK && constant_bytes > 0) st = mhlo_cuda_alloc(static_cast<size_t>(constant_bytes), &p->constants);
     if (st == MHLO_CUDA_OK && constant_bytes > 0) st = mhlo_cuda_upload(p->constants, constants_host, static_cast<size_t>(constant_bytes), nullptr);
     if (st == MHLO_CUDA_OK && constant_bytes > 0) st = mhlo_cuda_stream_sync(nullptr);
+    for (const mhlo_cuda_plan_op& op : p->ops)
+        if (op.kernel == MHLO_CUDA_KERNEL_GEMM) p->scratch_bytes = std::max(p->scratch_bytes, pack_bytes(op));
+    if (st == MHLO_CUDA_OK && p->scratch_bytes > 0 && mhlo_cuda_alloc(p->scratch_bytes, &p->scratch) != MHLO_CUDA_OK) {
+        p->scratch_bytes = 0;  // without it those products run on the general kernel
+        clear_error();
+    }
     if (st != MHLO_CUDA_OK) {
         mhlo_cuda_free(p->arena);
         mhlo_cuda_free(p->constants);
@@ -176,6 +196,7 @@ int mhlo_cuda_plan_destroy(mhlo_cuda_plan_t plan) {
     if (!p) return MHLO_CUDA_OK;
     mhlo_cuda_free(p->arena);
     mhlo_cuda_free(p->constants);
+    mhlo_cuda_free(p->scratch);
     delete p;
     return MHLO_CUDA_OK;
 }

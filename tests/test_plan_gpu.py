@@ -160,3 +160,26 @@ def test_communicator_on_the_visible_devices():
     assert cuda.lib.mhlo_cuda_all_gather(comm, ptrs, 24) == 10  # shards are whole 16-byte words
     assert cuda.lib.mhlo_cuda_comm_destroy(comm) == 0
     torch.cuda.set_device(0)
+
+
+@pytest.mark.gpu
+def test_products_off_the_grid_allocate_nothing_when_a_plan_runs():
+    """[65,77] . [77,131] in f16 is packed onto the 16-byte grid: into scratch of the plan, made with it."""
+    cuda = cuda_mod()
+    g = torch.Generator().manual_seed(9)
+    a, b = torch.randn(65, 77, generator=g).half().cuda(), torch.randn(77, 131, generator=g).half().cuda()
+    want = cuda.gemm(a, b)
+    op = cuda.plan_op("dot_general", cuda.F16, [(cuda.SRC_INPUT, 0, 0), (cuda.SRC_INPUT, 1, 0), (cuda.SRC_NONE, 0, 0), (cuda.SRC_OUTPUT, 0, 0)],
+                      [1, 1, 65, 131, 77], strides=[0, 0, 77, 1, 0, 0, 131, 1])
+    plan, out = cuda.Plan([op], 2, 1), torch.zeros_like(want)
+    try:
+        cuda.lib.mhlo_cuda_debug_refuse_allocs(1000)
+        plan.execute([a, b], [out])
+        torch.cuda.synchronize()
+        assert torch.equal(out, want)
+        poor = cuda.Plan([op], 2, 1)  # no memory for the scratch: the general kernel
+        out.zero_()
+        poor.execute([a, b], [out])
+    finally:
+        cuda.lib.mhlo_cuda_debug_refuse_allocs(0)
+    assert float((out.double() - a.double() @ b.double()).abs().max()) <= 2.0 ** -10 * float(want.abs().max())

@@ -401,7 +401,8 @@ static bool tiles_pay(const AttnShape& s) {
 }
 
 bool attention_fp32_supported(int dtype, const AttnShape& s) {
-    if (!tiles_pay(s)) return false;
+    const bool general = s.batch * s.heads * s.seq_q <= int64_t{4} * 0x7fffffff;  // rows the general kernel's grid holds
+    if (general && !tiles_pay(s)) return false;
     return dtype == MHLO_DT_F32 && s.head_dim <= 128 && s.batch * s.heads < (int64_t{1} << 27) && s.seq_q <= 32 * int64_t{65535} &&
            s.seq_k < (int64_t{1} << 30);
 }

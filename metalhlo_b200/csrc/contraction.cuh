@@ -27,6 +27,9 @@ struct GemmProblem {
     int32_t exact_act = 0;  // 1: the activation in fp32 with the CUDA library's functions, as the elementwise programs have it
 };
 
+// The limits of mhlo_cuda_dot_strided: a product beyond them is no one else's to hand over.
+inline bool general_kernel_takes(const GemmProblem& p) { return p.batch0 * p.batch1 <= 65535 && (p.m + 63) / 64 <= 65535; }
+
 // How the tensor-core kernels read a 16-bit operand [rows, cols] with element strides {batch0, batch1, row, col} in place: which
 // dimension its tensor map has as the contiguous one, kNoMajor if neither can be (TMA wants every other stride to be a positive
 // multiple of 16 bytes). A dimension of extent 1 is contiguous and on every grid, whatever its stride says. K comes first where

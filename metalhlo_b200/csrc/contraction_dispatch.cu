@@ -129,7 +129,7 @@ int gemm_entry(int32_t in_dtype, int32_t out_dtype, const void* a_dev, const int
     p.exact_act = exact_activation(p);
     // Those products keep fp32 sums too where the result is fp32: the tensor cores add more coarsely than FMAs (error against fp64 of
     // [1021,1111] . [1111,3001] f16 -> f32 1.0e-6 and 4.4e-7, of K = 4096 3.5e-6 and 8.8e-7), which a 16-bit result does not show.
-    const bool fp32_sums = p.exact_act && out_dtype == MHLO_DT_F32;
+    const bool fp32_sums = p.exact_act && out_dtype == MHLO_DT_F32 && general_kernel_takes(p);
     if (!fp32_sums && gemm_tc_supported(p)) return gemm_tc_launch(p, stream);
     if (gemm_fp32_supported(p)) return gemm_fp32_launch(p, stream);
     int st = MHLO_CUDA_OK;

@@ -355,7 +355,7 @@ int launch_split(Fp32Gemm p, int64_t batches, cudaStream_t stream) {
 // 69 and 70, at K = 64 120 and 80; with two tiles per SM or fewer this kernel leads at any K.
 static bool short_sums(const GemmProblem& g) {
     const int64_t tiles = (g.m <= 16 ? 1 : (g.m + 63) / 64) * ((g.n + 63) / 64) * g.batch0 * g.batch1;
-    return g.k <= 16 && tiles > 2 * kNumSMs;
+    return g.k <= 16 && tiles > 2 * kNumSMs && general_kernel_takes(g);
 }
 
 bool gemm_fp32_supported(const GemmProblem& g) {

@@ -76,13 +76,16 @@ struct PackWork {
 bool lay_out(GemmProblem* p, PackWork* w) {
     memset(w, 0, sizeof *w);
     int n = 0;
-    if ((p->in_dtype != MHLO_DT_F16 && p->in_dtype != MHLO_DT_BF16) || p->out_dtype != p->in_dtype) return false;  // fp32 results: fp32 sums
+    if (p->in_dtype != MHLO_DT_F16 && p->in_dtype != MHLO_DT_BF16) return false;
+    const bool elsewhere = general_kernel_takes(*p);
+    if (p->out_dtype != p->in_dtype && (elsewhere || p->out_dtype != MHLO_DT_F32)) return false;  // fp32 results: fp32 sums
     if (p->a == nullptr || p->b == nullptr || p->n_copies > 0 || p->m <= 0 || p->n <= 0 || p->k <= 0 || p->batch0 <= 0 || p->batch1 <= 0) return false;
     if (p->m > 0x7fffffff || p->n > 0x7fffffff || p->k > 0x7fffffff || p->batch0 * p->batch1 > 0x7fffffff) return false;
     // Copy and product cost 10 to 14 us before the first panel; the general kernel does 32 steps of K in 10, whatever the number of
     // results up to about eight million ([33,31] . [31,4001] 14 us packed, 10 there; with K = 63 14 and 15; [301,15] . [15,50257]
     // 37 and 46).
-    if (p->m * p->n * p->k < 64 * 1024 || (p->k <= 32 && p->m * p->n * p->batch0 * p->batch1 < int64_t{1} << 23)) return false;
+    if (p->m * p->n * p->k < 64 * 1024 || (p->k <= 32 && elsewhere && p->m * p->n * p->batch0 * p->batch1 < int64_t{1} << 23))
+        return false;
     for (const bool is_a : {true, false}) {
         const void** base = is_a ? &p->a : &p->b;
         int64_t* st = is_a ? p->as : p->bs;

@@ -185,3 +185,16 @@ def test_product_without_scratch():
     # the product is rounded before the bias there
     assert float((got.double() - torch.relu(want + bias.double())).abs().max()) <= 2 * 2.0 ** -11 * float(want.abs().max() + bias.abs().max())
     close(cuda.gemm(a, b), want, 333, magnitude)
+
+
+# more batch entries, or more rows, than the general kernel takes: nothing that the other kernels take is handed to it
+@pytest.mark.parametrize("dt,out_dtype,b,m,n,k", [(torch.float16, torch.float16, 66000, 64, 65, 17), (torch.float16, torch.float32, 66000, 16, 32, 72),
+                                                  (torch.float16, torch.float32, 66000, 40, 45, 41), (torch.float32, torch.float32, 1, 4194304 + 65, 4, 8)])
+def test_products_beyond_the_general_kernel(dt, out_dtype, b, m, n, k):
+    g = torch.Generator(device="cuda").manual_seed(k)
+    x, y = (torch.randn(s, generator=g, device="cuda", dtype=torch.float32).to(dt) for s in ((b, m, k), (b, k, n)))
+    got = raw_gemm(x, y, dt, 1, b, (0, m * k), (0, k * n), out_dtype=out_dtype)[0]
+    some = slice(0, None, 997) if b > 1 else slice(None)
+    rows = slice(None) if b > 1 else slice(0, None, 1009)
+    xs, ys = x[some, rows].double(), y[some].double()
+    close(got[some, rows], xs @ ys, k, xs.abs() @ ys.abs())

@@ -179,7 +179,7 @@ __device__ __noinline__ int64_t ew_int_outlined(int op, int64_t a, int64_t b, in
     return ew_int_op(op, a, b, c, imm, uns, boolean, bits);
 }
 
-// (powf from a call of its own: behind the switch of ew_outlined it took 7 % longer, 16.8 M elements 77 us against 72)
+// (powf from a call of its own: behind the switch of ew_outlined 16.8 M elements took 77 us, so 68)
 __device__ __noinline__ float ew_pow(float a, float b) { return powf(a, b); }
 
 // ---- launch parameters -------------------------------------------------------------------------------------------------

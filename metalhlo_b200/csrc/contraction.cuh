@@ -85,6 +85,7 @@ struct PackScratch {
     size_t bytes;
 };
 bool gemm_pack_launch(GemmProblem p, const PackScratch* scratch, cudaStream_t stream, int* status);
+bool gemm_fp32_sums(const GemmProblem& p);  // whether a 16-bit product read in place is kept from the tensor cores' sums
 size_t gemm_pack_bytes(GemmProblem p);  // what that takes when both operands start on the grid; 0: nothing is packed
 // mhlo_cuda_gemm_tuned with the scratch of packed operands from the caller.
 int gemm_entry(int32_t in_dtype, int32_t out_dtype, const void* a, const int64_t* a_strides, const void* b, const int64_t* b_strides, void* c,

@@ -108,6 +108,10 @@ bool exact_activation(const GemmProblem& p) {
 }
 }  // namespace
 
+// Those products keep fp32 sums too where the result is fp32: the tensor cores add more coarsely than FMAs (error against fp64 of
+// [1021,1111] . [1111,3001] f16 -> f32 1.0e-6 and 4.4e-7, of K = 4096 3.5e-6 and 8.8e-7), which a 16-bit result does not show.
+bool gemm_fp32_sums(const GemmProblem& p) { return exact_activation(p) && p.out_dtype == MHLO_DT_F32 && general_kernel_takes(p); }
+
 int gemm_entry(int32_t in_dtype, int32_t out_dtype, const void* a_dev, const int64_t* a_strides, const void* b_dev, const int64_t* b_strides,
                void* c_dev, int64_t batch0, int64_t batch1, int64_t m, int64_t n, int64_t k, const void* bias_dev, int32_t epilogue,
                const mhlo_cuda_gemm_tuning* tuning, const PackScratch* scratch, cudaStream_t stream) {
@@ -127,10 +131,7 @@ int gemm_entry(int32_t in_dtype, int32_t out_dtype, const void* a_dev, const int
     p.in_dtype = in_dtype; p.out_dtype = out_dtype; p.epilogue = epilogue;
     if (tuning) { p.tile_n = tuning->tile_n; p.stages = tuning->stages; p.cta_group = tuning->cta_group; p.split_k = tuning->split_k; }
     p.exact_act = exact_activation(p);
-    // Those products keep fp32 sums too where the result is fp32: the tensor cores add more coarsely than FMAs (error against fp64 of
-    // [1021,1111] . [1111,3001] f16 -> f32 1.0e-6 and 4.4e-7, of K = 4096 3.5e-6 and 8.8e-7), which a 16-bit result does not show.
-    const bool fp32_sums = p.exact_act && out_dtype == MHLO_DT_F32 && general_kernel_takes(p);
-    if (!fp32_sums && gemm_tc_supported(p)) return gemm_tc_launch(p, stream);
+    if (!gemm_fp32_sums(p) && gemm_tc_supported(p)) return gemm_tc_launch(p, stream);
     if (gemm_fp32_supported(p)) return gemm_fp32_launch(p, stream);
     int st = MHLO_CUDA_OK;
     if (gemm_pack_launch(p, scratch, stream, &st)) return st;

@@ -198,3 +198,22 @@ def test_products_beyond_the_general_kernel(dt, out_dtype, b, m, n, k):
     rows = slice(None) if b > 1 else slice(0, None, 1009)
     xs, ys = x[some, rows].double(), y[some].double()
     close(got[some, rows], xs @ ys, k, xs.abs() @ ys.abs())
+
+
+# fp32 results through widened operands: either type, every layout, a matrix shared by a batch, bias and activation
+@pytest.mark.parametrize("dt", ["f16", "bf16"])
+@pytest.mark.parametrize("m,n,k", [(300, 257, 65), (33, 61, 600), (1, 3000, 40), (3000, 1, 40)])
+@pytest.mark.parametrize("la,lb", [(("row", 0, 0), ("row", 1, 0)), (("row", 0, 1), ("col", 5, 2)), (("col", 3, 0), ("both", 0, 0)), (("both", 0, 0), ("row", 0, 0))])
+def test_fp32_results_of_views(m, n, k, la, lb, dt):
+    g = torch.Generator().manual_seed(m + k)
+    a, b = torch.randn(m, k, generator=g).to(DT[dt]).cuda(), (torch.randn(k, n, generator=g) / math.sqrt(k)).to(DT[dt]).cuda()
+    a[0, 0], b[k - 1, n - 1] = 6e-8, -1e-40  # an f16 subnormal and a bf16 one
+    views = []
+    for x, (order, extra, offset) in ((a, la), (b, lb)):
+        inner = x.shape[0] if order == "col" else x.shape[1]
+        views.append(strided(x, order, (inner + 7) // 8 * 8 + extra, offset))
+    bias = torch.randn(n, generator=g).cuda()
+    want, magnitude = product(a, b, dt)
+    close(raw_gemm(*views, DT[dt], out_dtype=torch.float32)[0, 0], want, k, magnitude)
+    got = raw_gemm(*views, DT[dt], 1, 3, (0, 0), (0, 0), bias=bias, epilogue="relu", out_dtype=torch.float32)[0]
+    close(got, torch.relu(want + bias.double()).expand(3, m, n), k + 1, (magnitude + bias.double().abs()).expand(3, m, n))

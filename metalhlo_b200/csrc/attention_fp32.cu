@@ -11,7 +11,7 @@
 // K is transposed on the way in (4-byte cp.async, 8 elements x 4 keys per warp instruction), V arrives in 16-byte copies;
 // the next K is in flight during the softmax and the product with V, the next V during the next scores.
 // 32 keys and at most 168 registers let three CTAs of four warps share an SM: [8,12,512,64] is one wave of 384 CTAs and runs
-// in 188 us (34 TFLOP/s); with 64 keys, two CTAs and two waves it took 210 us. Tiles too few for the machine share their
+// in 174 us (37 TFLOP/s); with 64 keys, two CTAs and two waves it took 210 us against 188. Tiles too few for the machine share their
 // keys among a cluster of up to 8 CTAs, whose sums, maxima and partial O meet through distributed shared memory: one head of
 // 1024 causal rows 198 us without, 31 us with it. One warp per query row with scalar loads, the former kernel, took 6.94 ms
 // and 571 us.
@@ -119,7 +119,7 @@ __device__ __forceinline__ void step(float2 (*acc)[2 * C], const float* a, const
     }
 }
 
-template <int RG, int HALVES, int kKeys>
+template <int RG, int HALVES, int kKeys, bool CAUSAL>
 __global__ void __launch_bounds__((Fp32AttentionTile<RG, HALVES, kKeys>::kThreads), (Fp32AttentionTile<RG, HALVES, kKeys>::kMinCtas))
 attention_fp32_kernel(const __grid_constant__ Fp32Attention p) {
     using T = Fp32AttentionTile<RG, HALVES, kKeys>;
@@ -134,7 +134,7 @@ attention_fp32_kernel(const __grid_constant__ Fp32Attention p) {
     const int ty = lane / 8, tx = lane % 8;
     const int rank = static_cast<int>(blockIdx.x) % p.splits, head = static_cast<int>(blockIdx.x) / p.splits;
     // the tiles that see most keys under a causal mask first, those of all heads before the next: every SM gets some of each
-    const int tile = p.causal ? static_cast<int>(gridDim.y) - 1 - static_cast<int>(blockIdx.y) : static_cast<int>(blockIdx.y);
+    const int tile = CAUSAL ? static_cast<int>(gridDim.y) - 1 - static_cast<int>(blockIdx.y) : static_cast<int>(blockIdx.y);
     const int q0 = tile * T::kRows;
     const int64_t b = head / p.heads, h = head % p.heads;
     const float* q = p.q + b * p.qs[0] + h * p.qs[1];
@@ -144,7 +144,7 @@ attention_fp32_kernel(const __grid_constant__ Fp32Attention p) {
     const uint32_t aq = static_cast<uint32_t>(__cvta_generic_to_shared(sq)), ak = static_cast<uint32_t>(__cvta_generic_to_shared(sk)),
                    av = static_cast<uint32_t>(__cvta_generic_to_shared(sv));
     int limit = p.seq_k;  // keys any row of this tile sees
-    if (p.causal && q0 + T::kRows < limit) limit = q0 + T::kRows;
+    if (CAUSAL && q0 + T::kRows < limit) limit = q0 + T::kRows;
     const int n_blocks = (limit + kKeys - 1) / kKeys;
     // the two warps of a row group
     auto pair_sync = [&]() {
@@ -191,7 +191,7 @@ attention_fp32_kernel(const __grid_constant__ Fp32Attention p) {
         cp_commit();
 
         const int key0 = j * kKeys + half * 32 + tx * 4;  // this thread's keys: key0 + {0..3} (+ 32)
-        const bool ragged = (j + 1) * kKeys > p.seq_k || (p.causal && (j + 1) * kKeys - 1 > q0 + group * 32);
+        const bool ragged = (j + 1) * kKeys > p.seq_k || (CAUSAL && (j + 1) * kKeys - 1 > q0 + group * 32);
         float* sf = reinterpret_cast<float*>(s);
 #pragma unroll
         for (int r = 0; r < 8; ++r)
@@ -203,7 +203,7 @@ attention_fp32_kernel(const __grid_constant__ Fp32Attention p) {
                     const int row = row_of(r);
                     if (row < p.seq_q && key < p.seq_k) x += p.mask[static_cast<int64_t>(row) * p.seq_k + key];
                 }
-                if (ragged && (key >= p.seq_k || (p.causal && key > row_of(r)))) x = -INFINITY;
+                if (ragged && (key >= p.seq_k || (CAUSAL && key > row_of(r)))) x = -INFINITY;
                 sf[r * 4 * C + e] = x;
             }
         float top[8];
@@ -252,12 +252,12 @@ attention_fp32_kernel(const __grid_constant__ Fp32Attention p) {
         __syncthreads();
         // keys of this block that some of the warp's rows do not see: those rows leave the key's V alone, which need not be finite
         const int behind = j * kKeys - (q0 + group * 32);  // key - row of the block's first key and the warp's first row
-        if (!p.causal || behind + kKeys - 1 <= 0) {
+        if (!CAUSAL || behind + kKeys - 1 <= 0) {
 #pragma unroll 8
             for (int key = 0; key < kKeys; ++key) step<2>(out, pw + key * T::kPPitch + ty * 4, vb + key * T::kVPitch, 32);
         } else {
             const int seen = 32 - behind < kKeys ? 32 - behind : kKeys;  // by the warp's last row
-#pragma unroll 2
+#pragma unroll 8
             for (int key = 0; key < seen; ++key)
                 step<2, true>(out, pw + key * T::kPPitch + ty * 4, vb + key * T::kVPitch, 32, behind + key - ty * 4);
         }
@@ -345,13 +345,17 @@ attention_fp32_kernel(const __grid_constant__ Fp32Attention p) {
 template <int RG, int HALVES, int KEYS>
 int launch(Fp32Attention p, int64_t batch_heads, cudaStream_t stream) {
     using T = Fp32AttentionTile<RG, HALVES, KEYS>;
-    static std::atomic<uint64_t> configured{0};  // devices whose copy of the kernel may use this much shared memory
+    // A kernel of its own for causal masks: as a run-time condition their rows' limits cost the others 3 to 6 % (without them and with
+    // the mask known at compile time [8,12,512,64] 174 us, one query against 1024 keys of 12 heads 26). Under a mask the limits cost
+    // nothing up to head dimension 64 and 4 to 6 % above.
+    auto kernel = p.causal ? attention_fp32_kernel<RG, HALVES, KEYS, true> : attention_fp32_kernel<RG, HALVES, KEYS, false>;
+    static std::atomic<uint64_t> configured{0};  // devices whose copies of the kernels may use this much shared memory
     int dev = 0;
     MHLO_CUDA_TRY(cudaGetDevice(&dev), MHLO_CUDA_NO_DEVICE);
     const uint64_t bit = uint64_t{1} << (dev & 63);
     if (!(configured.load(std::memory_order_relaxed) & bit)) {
-        MHLO_CUDA_TRY(cudaFuncSetAttribute(attention_fp32_kernel<RG, HALVES, KEYS>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(T::kShared)),
-                      MHLO_CUDA_EXECUTION_FAILED);
+        for (auto each : {attention_fp32_kernel<RG, HALVES, KEYS, true>, attention_fp32_kernel<RG, HALVES, KEYS, false>})
+            MHLO_CUDA_TRY(cudaFuncSetAttribute(each, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(T::kShared)), MHLO_CUDA_EXECUTION_FAILED);
         configured.fetch_or(bit, std::memory_order_relaxed);
     }
     const int64_t tiles = (p.seq_q + T::kRows - 1) / T::kRows;
@@ -370,7 +374,7 @@ int launch(Fp32Attention p, int64_t batch_heads, cudaStream_t stream) {
     attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
     cfg.attrs = attr;
     cfg.numAttrs = p.splits > 1 ? 1 : 0;
-    MHLO_CUDA_TRY(cudaLaunchKernelEx(&cfg, attention_fp32_kernel<RG, HALVES, KEYS>, p), MHLO_CUDA_EXECUTION_FAILED);
+    MHLO_CUDA_TRY(cudaLaunchKernelEx(&cfg, kernel, p), MHLO_CUDA_EXECUTION_FAILED);
     return MHLO_CUDA_OK;
 }
 

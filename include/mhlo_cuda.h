@@ -553,11 +553,12 @@ enum {
  * operands need no copy. bias_dev ([n], dtype = out_dtype) may be NULL. BF16/F16 operands whose rows or columns
  * are contiguous and 16-byte aligned run on the tcgen05 tensor-core kernel (TMA-fed, TMEM accumulators); BF16/F16
  * operands that are not are first copied onto that grid where it pays, into stream-ordered scratch of the library's own
- * memory pool (inside a stream capture: nodes of the graph). F32 runs on packed FMAs. Everything else, and a product whose
- * scratch cannot be had, takes the general-layout kernel behind mhlo_cuda_dot_strided, which never allocates. Replaces kernel_matmul (MPP and
- * simdgroup variants, Sources/MetalHLOCore/Compiler/CodeGenerator.swift:3463-3886), kernel_matmul_bias_act
- * (:4797-4850) and the semantics of FusedMatMulBiasActivationHandler
- * (Sources/MetalHLOCore/Compiler/CustomCallHandlers.swift:927-1073).
+ * memory pool (inside a stream capture: nodes of the graph). F32 runs on packed FMAs, and so do, widened on the way, the
+ * operands of an F32 result that would be packed or has fewer than 64 x 64 elements (the tensor cores add more coarsely).
+ * Everything else, and a product whose scratch cannot be had, takes the general-layout kernel behind
+ * mhlo_cuda_dot_strided, which never allocates. Replaces kernel_matmul (MPP and simdgroup variants,
+ * Sources/MetalHLOCore/Compiler/CodeGenerator.swift:3463-3886), kernel_matmul_bias_act (:4797-4850) and the semantics of
+ * FusedMatMulBiasActivationHandler (Sources/MetalHLOCore/Compiler/CustomCallHandlers.swift:927-1073).
  */
 int mhlo_cuda_gemm(int32_t in_dtype, int32_t out_dtype, const void* a_dev, const int64_t a_strides[4],
                    const void* b_dev, const int64_t b_strides[4], void* c_dev, int64_t batch0, int64_t batch1,
@@ -788,8 +789,8 @@ typedef void* mhlo_cuda_plan_t;
  * FusedOp.fusedOpTypeFromCustomCall (Compiler/IntegrationTypes.swift:471-600) on the CUDA side. MHLO_CUDA_UNSUPPORTED
  * when the library has no such kernel for the dtype. */
 int mhlo_cuda_kernel_lookup(const char* fused_op_kind, int32_t dtype, int32_t* out_kernel);
-/* Validates the ops, allocates the arena and the scratch of products whose 16-bit operands lie off the 16-byte grid (without
- * that scratch they run on the general kernel), and uploads the constant pool. Each may be empty. The caller owns the plan. */
+/* Validates the ops, allocates the arena and the scratch of products whose 16-bit operands are copied first (without that
+ * scratch they run on the general kernel), and uploads the constant pool. Each may be empty. The caller owns the plan. */
 int mhlo_cuda_plan_create(const mhlo_cuda_plan_op* ops, int32_t n_ops, int32_t n_inputs, int32_t n_outputs, int64_t arena_bytes,
                           const void* constants_host, int64_t constant_bytes, mhlo_cuda_plan_t* out_plan);
 /* Enqueues every op in order on `stream`; inputs / outputs are device pointers. No allocation, no synchronisation. */

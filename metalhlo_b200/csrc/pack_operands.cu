@@ -96,7 +96,7 @@ bool lay_out(GemmProblem* p, PackWork* w) {
     // Copy and product cost 10 to 14 us before the first panel; the general kernel does 32 steps of K in 10, whatever the number of
     // results up to about eight million ([33,31] . [31,4001] 14 us packed, 10 there; with K = 63 14 and 15; [301,15] . [15,50257]
     // 37 and 46).
-    if (p->m * p->n * p->k < (w->widen ? 32 : 64) * 1024 || (p->k <= 32 && elsewhere && p->m * p->n * p->batch0 * p->batch1 < int64_t{1} << 23))
+    if (p->m * p->n * p->k < 32 * 1024 || (p->k <= 32 && elsewhere && p->m * p->n * p->batch0 * p->batch1 < int64_t{1} << 23))
         return false;
     for (const bool is_a : {true, false}) {
         const void** base = is_a ? &p->a : &p->b;

@@ -93,11 +93,6 @@ int launch_attention_rows(const void* q, const void* k, const void* v, const voi
     return MHLO_CUDA_OK;
 }
 
-}  // namespace
-}  // namespace mhlo
-
-namespace mhlo {
-namespace {
 // Whether the tensor-core epilogue takes the CUDA library's tanhf and expf rather than the hardware's approximations (2^-11
 // relative). The approximations are for products whose epilogue has to keep up with the MMAs: at least 64 x 64 results, K
 // above 1, operands read in place, one matrix each per batch entry. Everything else (and every packed product) is bound elsewhere
@@ -106,6 +101,7 @@ bool exact_activation(const GemmProblem& p) {
     const bool shared = (p.batch0 > 1 && (p.as[0] == 0 || p.bs[0] == 0)) || (p.batch1 > 1 && (p.as[1] == 0 || p.bs[1] == 0));
     return p.m * p.n < 64 * 64 || p.k == 1 || shared;
 }
+
 }  // namespace
 
 // Those products keep fp32 sums too where the result is fp32: the tensor cores add more coarsely than FMAs (error against fp64 of
